@@ -25,14 +25,22 @@
 // searches it in registers by shuffles, a longer one by a per-lane binary
 // search inside the window.
 //
-// Work stealing: warps that run out of input wait for work.  A busy warp
-// checks every 64 steps whether idle warps outnumber the queued records; if
-// so it hands its shallowest pending depth (buffered candidates and the
-// remaining driver range) to the queue as task records and carries on with
-// the rest.  Waiting is bounded: a warp that waits too long simply leaves,
-// which never loses work -- records still queued when the pass ends are the
-// next pass's input.  Every value that steers a warp's control flow is read
-// by lane 0 and broadcast.
+// Work stealing: a warp that runs out of input takes a ticket, one atomicAdd
+// on the queue's head, and waits for the record of that number, polling the
+// record's own ready word.  A busy warp checks every 64 steps whether more
+// tickets than records are out; if so it hands its shallowest pending depth
+// (buffered candidates and the remaining driver range) to the queue as task
+// records and carries on with the rest.  One counter holds the warps at work
+// plus the records not taken yet; the pass is over when it reaches zero.
+// (Tickets replaced a compare-and-swap on the head by every idle warp for
+// every record: up to 2048 warps retrying on one word served a record in
+// 0.4-1.0 us whatever the work in it, which bounded every batch but the
+// largest.  One 4-vertex query on a 10k-vertex graph 3.8 -> 0.37 ms, 100 of
+// them 37 -> 2.5 ms, 37 refined queries on 2^26 edges 78 -> 29 ms, a
+// 512-query batch there 390 -> 305 ms.)  Waiting is bounded: a warp that waits too long leaves, which
+// never loses work -- the records nobody took are the next pass's input.
+// Every value that steers a warp's control flow is read by lane 0 and
+// broadcast.
 #pragma once
 
 namespace fsig {
@@ -57,14 +65,16 @@ struct EnumArgs {
   uint32_t t_end;  // pass-0 tasks [initial ctr[0], t_end) (a range of the task space)
   // explicit input tasks (passes >= 1)
   const TaskRec* __restrict__ in_tasks;
+  const uint32_t* __restrict__ in_index;  // [in_count] records of in_tasks
   uint32_t in_count;
   // work queue
   TaskRec* out_tasks;
   uint32_t* out_ready;
-  uint32_t out_cap;
-  uint32_t tag;
-  uint32_t* ctr;  // counters, kCtrStride apart: [0] input grab, [1] queue tail (reserved),
-                  // [2] queue head, [3] error bits, [4] idle warps, [5] active warps
+  uint32_t out_cap;  // a power of two
+  uint32_t* ctr;  // counters, kCtrStride apart: [0] input grab, [1] queue tail (records reserved) and,
+                  // in the next word, tickets taken, [2] warps at work + records not taken yet,
+                  // [3] error bits, [4] fault injection's one-shot, [5] once a waiting warp has left,
+                  // the record number from which on no more are reserved
   uint32_t chunk;
   long long budget;  // cycles on a task before it may be split while warps are idle
   QueryResult* res;
@@ -103,7 +113,13 @@ constexpr int kGroup = 2;
 
 constexpr uint32_t kErrTimeout = 1u;
 constexpr uint32_t kCtrStride = 32;        // one 128-byte line per counter
-constexpr uint32_t kMaxWaiters = 2048;     // warps beyond this many idle ones leave instead of waiting
+// The queue is a ring: record number t lies in slot t mod out_cap, use
+// g = t / out_cap of that slot.  The slot's ready word is 2g while it is free
+// for that use, 2g + 1 from the record's publication until its ticket holder
+// has read it, then 2g + 2 (= free for use g + 1).  Records are reserved only
+// while warps wait, so at most (warps) x (records of one hand-off) numbers lie
+// between the tickets and the tail, far below the ring's 2^20 slots: a
+// reserved slot's previous record always has a ticket holder.
 
 __device__ __forceinline__ unsigned long long global_ns() {
   unsigned long long t;
@@ -448,22 +464,36 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
     const uint32_t total = __shfl_sync(kFull, mine, l);
     uint32_t base = 0;
     if (lane == 0) {
-      base = kInvalid;
-      uint32_t r = *(volatile uint32_t*)&A.ctr[1 * kCtrStride];
-      while (r + total <= A.out_cap) {
-        const uint32_t prev = atomicCAS(&A.ctr[1 * kCtrStride], r, r + total);
-        if (prev == r) { base = r; break; }
-        r = prev;
+      const uint32_t limit = *(volatile uint32_t*)&A.ctr[5 * kCtrStride];
+      if (limit && *(volatile uint32_t*)&A.ctr[1 * kCtrStride] + total > limit) {
+        base = kInvalid;
+      } else {
+        base = atomicAdd(&A.ctr[1 * kCtrStride], total);
+        atomicAdd(&A.ctr[2 * kCtrStride], total);
       }
     }
     base = __shfl_sync(kFull, base, 0);
     if (base == kInvalid) return false;
+    // the slots' previous records are read by now, or about to be (see above)
+    {
+      const uint32_t mask = A.out_cap - 1, shift = 31 - __clz(A.out_cap);
+      const unsigned long long t0 = global_ns();
+      for (uint32_t k = base + lane; k < base + total; k += 32) {
+        while (*(volatile uint32_t*)&A.out_ready[k & mask] != 2 * (k >> shift)) {
+          if (global_ns() - t0 > A.ready_wait_ns) {
+            atomicOr(&A.ctr[3 * kCtrStride], kErrTimeout);
+            break;
+          }
+        }
+      }
+      __syncwarp();
+    }
     uint32_t slot = base;
     const uint32_t c_l = __shfl_sync(kFull, cnt, l), i_l = __shfl_sync(kFull, it, l);
     const uint32_t p_l = __shfl_sync(kFull, dpos, l), e_l = __shfl_sync(kFull, dend, l);
     if (l + 1 < n) {
       for (uint32_t k = i_l; k < c_l; k++) {
-        TaskRec* r = A.out_tasks + slot++;
+        TaskRec* r = A.out_tasks + (slot++ & (A.out_cap - 1));
         const uint32_t cv = ws.cand[l][k];
         if (lane < l) r->f[lane] = f;
         if (lane == l) r->f[lane] = cv;
@@ -471,7 +501,7 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
       }
     }
     for (uint32_t p = p_l; p < e_l; p += hand) {
-      TaskRec* r = A.out_tasks + slot++;
+      TaskRec* r = A.out_tasks + (slot++ & (A.out_cap - 1));
       if (lane < l) r->f[lane] = f;
       if (lane == 0) { r->q = cur_q; r->d = l; r->lo = p; r->hi = min(p + hand, e_l); }
     }
@@ -482,24 +512,23 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
     __threadfence();
     __syncwarp();
     int hold = 0;  // test hook: keep the pass's first handed-off record unpublished
-    if (A.unpublished && lane == 0) hold = atomicCAS(&A.ctr[6 * kCtrStride], 0u, 1u) == 0u;
+    if (A.unpublished && lane == 0) hold = atomicCAS(&A.ctr[4 * kCtrStride], 0u, 1u) == 0u;
     hold = __shfl_sync(kFull, hold, 0);
-    for (uint32_t s = base + lane; s < base + total; s += 32)
-      if (!(hold && s == base)) atomicExch(&A.out_ready[s], A.tag);
+    for (uint32_t k = base + lane; k < base + total; k += 32)
+      if (!(hold && k == base))
+        atomicExch(&A.out_ready[k & (A.out_cap - 1)], 2 * (k >> (31 - __clz(A.out_cap))) + 1);
     if (lane == 0) { n_handoffs++; n_recs += total; }
     return true;
   };
 
-  // Whether idle warps are waiting for more work than the queue holds.
-  // Decided by lane 0 alone and broadcast.
+  // Whether warps wait for records that nobody has reserved: more tickets
+  // than records.  Decided by lane 0 alone and broadcast.
   auto should_split = [&](uint32_t t_start) -> bool {
     int w = 0;
     if (lane == 0 && A.out_cap) {
-      const uint32_t idle = *(volatile uint32_t*)&A.ctr[4 * kCtrStride];
-      if (idle) {
-        const uint32_t tail = *(volatile uint32_t*)&A.ctr[1 * kCtrStride], head = *(volatile uint32_t*)&A.ctr[2 * kCtrStride];
-        w = (tail - min(head, tail) < idle) && (long long)(uint32_t(clock()) - t_start) > A.budget;
-      }
+      uint32_t tail, tickets;
+      asm volatile("ld.volatile.global.v2.u32 {%0, %1}, [%2];" : "=r"(tail), "=r"(tickets) : "l"(A.ctr + kCtrStride));
+      w = int32_t(tickets - tail) > 0 && (long long)(uint32_t(clock()) - t_start) > A.budget;
     }
     return __shfl_sync(kFull, w, 0) != 0;
   };
@@ -716,7 +745,7 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
   // The header is read by lane 0 and broadcast, like every other value that
   // steers the warp's control flow; records popped in this launch were
   // written by another SM, so they are read through L2 (ld.cg).
-  auto run_record = [&](const TaskRec* r) {
+  auto run_record = [&](const TaskRec* r, uint32_t* ready, uint32_t free_word) {
     uint32_t q = 0, d = 0, lo = 0, hi = 0;
     if (lane == 0) {
       q = __ldcg(&r->q);
@@ -728,8 +757,13 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
     d = __shfl_sync(kFull, d, 0);
     lo = __shfl_sync(kFull, lo, 0);
     hi = __shfl_sync(kFull, hi, 0);
-    use_query(q);
     if (lane < d) f = __ldcg(&r->f[lane]);
+    if (ready) {  // the record is read: its slot is free again
+      __threadfence();
+      __syncwarp();
+      if (lane == 0) *(volatile uint32_t*)ready = free_word;
+    }
+    use_query(q);
     run(d, lo, hi);
   };
 
@@ -742,7 +776,7 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
       const uint32_t t1 = min(t0 + A.chunk, T_in);
       for (uint32_t t = t0; t < t1; t++) {
         if (A.in_tasks) {
-          run_record(A.in_tasks + t);
+          run_record(A.in_tasks + A.in_index[t], nullptr, 0);
         } else {
           // implicit: root i, chunk c of its depth-1 driver range
           uint32_t lo = 0, hi = nroots;  // last i with chunk_off[i] <= t
@@ -767,53 +801,48 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
       }
       continue;
     }
-    // 2. input exhausted: take queued records, waiting while others work
+    // 2. input exhausted: take a ticket and wait for its record while others work
     uint32_t slot = kInvalid;
     if (lane == 0) {
-      atomicSub(&A.ctr[5 * kCtrStride], 1u);
-      const uint32_t waiting = atomicAdd(&A.ctr[4 * kCtrStride], 1u);
-      uint32_t sleep_ns = 256;
-      // enough warps already wait: leave at once (queued work is never lost)
+      const uint32_t t = atomicAdd(&A.ctr[1 * kCtrStride + 1], 1u);
+      atomicSub(&A.ctr[2 * kCtrStride], 1u);
       const unsigned long long t_idle = global_ns();
-      const unsigned long long idle_ns = waiting >= kMaxWaiters ? 0ull : A.idle_wait_ns;
+      unsigned long long t_reserved = 0;  // when the record of this ticket was first seen reserved
+      uint32_t sleep_ns = 32;
+      volatile uint32_t* ready = A.out_ready + (t & (A.out_cap - 1));
+      const uint32_t published = 2 * (t >> (31 - __clz(A.out_cap))) + 1;
       for (;;) {
-        const uint32_t tail = min(*(volatile uint32_t*)&A.ctr[1 * kCtrStride], A.out_cap);
-        uint32_t h = *(volatile uint32_t*)&A.ctr[2 * kCtrStride];
-        bool got = false;
-        while (h < tail) {
-          const uint32_t prev = atomicCAS(&A.ctr[2 * kCtrStride], h, h + 1);
-          if (prev == h) { slot = h; got = true; break; }
-          h = prev;
-        }
-        if (got) break;
-        // finished when nobody works and nothing is queued (active read first)
-        if (*(volatile uint32_t*)&A.ctr[5 * kCtrStride] == 0 &&
-            *(volatile uint32_t*)&A.ctr[2 * kCtrStride] >= min(*(volatile uint32_t*)&A.ctr[1 * kCtrStride], A.out_cap))
+        if (*ready == published) {
+          slot = t;
           break;
-        if (global_ns() - t_idle >= idle_ns || *(volatile uint32_t*)&A.ctr[3 * kCtrStride]) break;
-        __nanosleep(sleep_ns);
-        if (sleep_ns < 8192) sleep_ns <<= 1;
-      }
-      atomicSub(&A.ctr[4 * kCtrStride], 1u);
-      if (slot != kInvalid) {
-        atomicAdd(&A.ctr[5 * kCtrStride], 1u);
-        const unsigned long long t_ready = global_ns();
-        while (*(volatile uint32_t*)&A.out_ready[slot] != A.tag) {
-          if (global_ns() - t_ready > A.ready_wait_ns) {
+        }
+        // finished when nobody works and every record is taken
+        if (*(volatile uint32_t*)&A.ctr[2 * kCtrStride] == 0 || *(volatile uint32_t*)&A.ctr[3 * kCtrStride]) break;
+        const unsigned long long now = global_ns();
+        const uint32_t tail = *(volatile uint32_t*)&A.ctr[1 * kCtrStride];
+        if (int32_t(tail - t) > 0) {
+          if (!t_reserved) {
+            t_reserved = now;
+          } else if (now - t_reserved > A.ready_wait_ns) {
             atomicOr(&A.ctr[3 * kCtrStride], kErrTimeout);
-            slot = kInvalid - 1;
             break;
           }
-          __nanosleep(64);
+        } else if (now - t_idle >= A.idle_wait_ns) {
+          // leave: this ticket's record, if it comes, waits for the next pass,
+          // so no slot from here on may be used again
+          atomicCAS(&A.ctr[5 * kCtrStride], 0u, max(tail + A.out_cap / 2, 1u));
+          break;
         }
-        if (slot == kInvalid - 1) atomicSub(&A.ctr[5 * kCtrStride], 1u);
+        __nanosleep(sleep_ns);
+        if (sleep_ns < 1024) sleep_ns <<= 1;
       }
     }
     slot = __shfl_sync(kFull, slot, 0);
-    if (slot >= kInvalid - 1) break;
+    if (slot == kInvalid) break;
     __threadfence();
     if (lane == 0) n_pops++;
-    run_record(A.out_tasks + slot);
+    run_record(A.out_tasks + (slot & (A.out_cap - 1)), A.out_ready + (slot & (A.out_cap - 1)),
+               2 * (slot >> (31 - __clz(A.out_cap))) + 2);
   }
   if (cur_q != kInvalid) over_limit();
   flush();

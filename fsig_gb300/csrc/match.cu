@@ -684,7 +684,7 @@ int filter_stage(Engine& e, const BatchLayout& b, uint32_t mode, int refine_iter
 }  // namespace
 
 namespace {
-constexpr uint32_t kOverflowCap = 1u << 20;  // task records per overflow queue
+constexpr uint32_t kOverflowCap = 1u << 20;  // slots of a pass's record ring (a power of two)
 
 // Records ev on s.  Inside a stream capture an ordinary record only orders
 // the capture; the external form makes it a node of the graph.
@@ -738,12 +738,30 @@ __global__ void given_scores_kernel(const uint32_t* __restrict__ qoff, uint32_t 
 
 __global__ void ctr_init_kernel(uint32_t* ctr, uint32_t first_task, uint32_t active) {
   for (uint32_t i = threadIdx.x; i < 8 * kCtrStride; i += blockDim.x)
-    ctr[i] = i == 0 ? first_task : (i == 5 * kCtrStride ? active : 0u);
+    ctr[i] = i == 0 ? first_task : (i == 2 * kCtrStride ? active : 0u);
+}
+
+// Records of a finished pass that no warp took (waiting warps left before
+// they were published): the ready words become the list of their slots, in
+// place (one block; a write never passes a read), their number goes to *count.
+__global__ void __launch_bounds__(256) untaken_kernel(uint32_t* ready, uint32_t slots, uint32_t* count) {
+  __shared__ uint32_t sw[33];
+  uint32_t found = 0;
+  for (uint32_t b = 0; b < slots; b += blockDim.x) {
+    const uint32_t i = b + threadIdx.x;
+    const bool left = i < slots && (ready[i] & 1u);  // published, not read
+    uint32_t total;
+    const uint32_t k = found + block_exclusive_scan<uint32_t>(left ? 1u : 0u, sw, total);
+    if (left) ready[k] = i;
+    found += total;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) *count = found;
 }
 
 // The enumeration passes of one batch: pass 0 over the implicit root tasks,
-// then passes over the records each pass leaves in its overflow queue, until
-// none are left.  Launching a pass is stream-ordered work only (capturable);
+// then passes over the records that each pass leaves untaken in its queue,
+// until none are left.  Launching a pass is stream-ordered work only (capturable);
 // deciding whether another pass is needed reads the counters the pass copied
 // to pinned host memory, after the stream has reached them.
 struct EnumRun {
@@ -792,8 +810,6 @@ int enum_prepare(Engine& e, const BatchOptions& opt, const GraphView& gv, const 
   R.d_ev = e.arena.take<unsigned long long>(8);
   if (!qa || !qb || !ra || !rb || !R.ctr || !R.d_ev)
     return fail(FSIG_EADMISSION, "work queues do not fit the device arena");
-  FSIG_CUDA_TRY(cudaMemsetAsync(ra, 0, sizeof(uint32_t) * kOverflowCap, s));
-  FSIG_CUDA_TRY(cudaMemsetAsync(rb, 0, sizeof(uint32_t) * kOverflowCap, s));
   FSIG_CUDA_TRY(cudaMemsetAsync(R.d_ev, 0, 64, s));
   FSIG_CUDA_TRY(cudaMemsetAsync(d_misc + 1, 0, sizeof(unsigned long long), s));
   const uint32_t wpb = std::max<uint32_t>(1, std::min<uint32_t>(opt.warps_per_block, kEnumWarps));
@@ -820,6 +836,7 @@ int enum_prepare(Engine& e, const BatchOptions& opt, const GraphView& gv, const 
   A.emit_cap = d_emit ? opt.emit_cap : 0;
   A.emit_ctr = d_emit_ctr;
   A.in_tasks = nullptr;
+  A.in_index = nullptr;
   A.in_count = 0;
   A.out_cap = kOverflowCap;
   A.ctr = R.ctr;
@@ -845,7 +862,7 @@ int enum_launch(Engine& e, EnumRun& R) {
   cudaStream_t s = e.stream;
   R.A.out_tasks = R.out;
   R.A.out_ready = R.ready;
-  R.A.tag = R.pass + 1;
+  FSIG_CUDA_TRY(cudaMemsetAsync(R.ready, 0, sizeof(uint32_t) * kOverflowCap, s));
   ctr_init_kernel<<<1, 256, 0, s>>>(R.ctr, R.pass == 0 ? R.first_task : 0u, R.active);
   FSIG_CUDA_TRY(cudaGetLastError());
   FSIG_CUDA_TRY(record(e.ev_enum[0], s));
@@ -866,12 +883,18 @@ int enum_after(Engine& e, EnumRun& R, bool& more, float& ms_enum, uint64_t& d2h)
   d2h += sizeof(uint32_t) * 4 * kCtrStride;
   const uint32_t* hc = R.h_ctr;
   if (hc[3 * kCtrStride] & kErrTimeout) return fail(FSIG_ETIMEOUT, "a work-queue record was not published in time");
-  const uint32_t head = hc[2 * kCtrStride], tail = std::min(hc[1 * kCtrStride], kOverflowCap);
-  more = head < tail;
+  more = hc[2 * kCtrStride] != 0;
   if (!more) return FSIG_OK;
-  // unconsumed records become the next pass's input
-  R.A.in_tasks = R.out + head;
-  R.A.in_count = tail - head;
+  // the records nobody took become the next pass's input
+  uint32_t* count = R.ctr + 7 * kCtrStride;
+  untaken_kernel<<<1, 256, 0, e.stream>>>(R.ready, kOverflowCap, count);
+  FSIG_CUDA_TRY(cudaGetLastError());
+  FSIG_CUDA_TRY(cudaMemcpyAsync(R.h_ctr, count, sizeof(uint32_t), cudaMemcpyDeviceToHost, e.stream));
+  FSIG_CUDA_TRY(cudaStreamSynchronize(e.stream));
+  if (R.h_ctr[0] != hc[2 * kCtrStride]) return fail(FSIG_EOVERFLOW, "task records were lost");
+  R.A.in_tasks = R.out;
+  R.A.in_index = R.ready;
+  R.A.in_count = R.h_ctr[0];
   std::swap(R.out, R.other);
   std::swap(R.ready, R.other_ready);
   if (++R.pass > 4096) return fail(FSIG_EOVERFLOW, "enumeration did not converge");

@@ -93,3 +93,29 @@ def test_queue_wait_arguments_are_checked():
         assert ei.value.status == F.EINVAL
         with pytest.raises(F.FsigError):
             e._check(e._L.fsig_set_queue_waits(e._h, 0, 0, 2), "set_queue_waits")
+
+
+@pytest.mark.parametrize("name", ["house", "c5"])
+@pytest.mark.parametrize("idle_wait_ns", [1, 20_000, 0])
+def test_untaken_records_run_in_a_later_pass(name, idle_wait_ns):
+    """Warps that run out of input leave almost at once (1 ns), after a while
+    or never: the records handed off to warps that left are the next pass's
+    input, and count, hash and per-depth counts are the oracle's and the same
+    whatever the waits."""
+    g = F.gen_rmat(1 << 8, 1 << 11, 0.57, 0.19, 0.19, seed=3)
+    off, adj = g.csr()
+    q = pattern(name)
+    c, h, _ = O.match(g.labels, off, adj, q.labels, q.edges)
+    with F.Engine(0, arena_bytes=2 << 30) as e:
+        e.load_graph(g)
+        e.set_queue_waits(idle_wait_ns=idle_wait_ns)
+        passes, levels = [], set()
+        for use_graph in (False, True):
+            r, = e.match_batch([q], algo=F.ALGO_FUSED, split_cycles=1000, split_len=32, use_graph=use_graph)
+            assert (r.status, r.count, r.hash) == (0, c, h)
+            levels.add(tuple(r.level_counts))
+            passes.append(e.last_stats()["enum_passes"])
+        e.set_queue_waits()
+        levels.add(tuple(e.match(q, F.ALGO_FUSED).level_counts))
+    assert len(levels) == 1
+    assert min(passes) > 1 if idle_wait_ns == 1 else min(passes) >= 1
