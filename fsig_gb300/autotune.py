@@ -10,12 +10,9 @@ The enumeration kernel's behaviour on a workload depends on five knobs of
   hand-offs, and so of load balance);
 * ``split_cycles`` - SM cycles a task runs before its unexplored frontier may
   be handed to idle warps;
-* ``isect`` - the set-intersection strategy of the membership tests: 0
-  every lane binary-searches the segment alone, 1 warp-cooperative 32-ary
-  window search (galloping-like), 2 adaptive (the 32 entries after a
-  segment's cursor first, merge-like, then the window search), 3 the tile
-  search for segments whose rest fits 32 entries and per-lane binary search
-  for longer ones.
+* ``isect`` - the set-intersection strategy of the membership tests, 0..3:
+  the enumeration has one strategy by now, so the values time alike; the
+  knob stays for callers that set it.
 
 When the batch refines candidates (``refine_iters`` > 0) one more joins:
 

@@ -430,7 +430,6 @@ int fsig_match_batch(fsig_engine* h, uint32_t nq, const fsig_query* qs, const fs
   if (bo.split_cycles) o.budget_cycles = (long long)bo.split_cycles;
   o.max_work = bo.max_work;
   if (bo.isect > 3) return finish(h, fsig::fail(FSIG_EINVAL, "unknown intersection strategy"));
-  o.isect = bo.isect;
   if (bo.refine_coop) o.refine_coop = bo.refine_coop;
   fsig::BatchOutput out_b;
   rc = fsig::run_batch(h->e, hq, o, out_b);

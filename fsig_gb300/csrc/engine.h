@@ -50,9 +50,10 @@ struct Engine {
   // pinned host staging for batches
   void* pinned = nullptr;
   uint64_t pinned_bytes = 0;
-  // enumeration kernel: resident blocks per SM (0 until first queried)
-  int enum_per_sm[9] = {0};       // resident blocks per SM at 1..8 warps per block (0 until queried)
-  int enum_per_sm_rows[9] = {0};  // the same for a graph store without a segment table
+  // enumeration kernel: resident blocks per SM at 1..8 warps per block and 1..31
+  // depths with a buffer (0 until queried), with and without a segment table
+  int enum_per_sm[9][32] = {};
+  int enum_per_sm_rows[9][32] = {};
   int seg_index = 0;              // segment index of the next graph build (FSIG_SEGMENTS_*)
   // timing events
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};

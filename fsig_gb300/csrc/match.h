@@ -86,7 +86,8 @@ struct QueryResult {
 constexpr uint32_t kRefineCoopDefault = 32;
 
 // Enumeration launch shape: at most kEnumWarps warps per block, compiled for
-// kEnumMinBlocks resident blocks per SM (which caps registers per thread).
+// kEnumMinBlocks resident blocks per SM (which caps registers per thread);
+// batches with queries of more than about 20 vertices have room for 3 blocks.
 constexpr uint32_t kEnumWarps = 8;
 constexpr uint32_t kEnumMinBlocks = 4;
 
@@ -116,9 +117,7 @@ struct BatchOptions {
   // Single-query batches: report the size of the pass-0 task space in
   // BatchOutput::tasks_total (ordinary launches, not a CUDA graph).
   bool want_tasks = false;
-  // Set-intersection strategy of the enumeration (kIsect* in enumerate.cuh)
-  // and the refinement's lane/warp split (kRefineCoopDefault).
-  uint32_t isect = 0;
+  // The refinement's lane/warp split (kRefineCoopDefault).
   uint32_t refine_coop = kRefineCoopDefault;
   // Run the batch as one CUDA graph (uploads, filter, order, roots, first
   // enumeration pass, results back) when orders are chosen on the device.

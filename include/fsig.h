@@ -108,15 +108,11 @@ typedef struct {
   uint32_t no_classes;      /* 1: filter and refine every query vertex on its own,
                                with every neighbour count one; 0 (default):
                                refinement classes (see fsig_refine_classes)      */
-  uint32_t isect;           /* set-intersection strategy of the enumeration:
-                               0 (default) every lane binary-searches the
-                               segments alone, two in lockstep; 1 warp-
-                               cooperative 32-ary window search (galloping-
-                               like); 2 adaptive: the 32 entries after a
-                               segment's cursor first (merge-like), else the
-                               window search; 3 the tile search when the
-                               segment's rest fits 32 entries, else a lane's
-                               own binary search                          */
+  uint32_t isect;           /* set-intersection strategy, 0..3.  Every value
+                               runs the one there is, in which a warp's lanes
+                               test candidates of up to 32 partial embeddings:
+                               the warp-cooperative searches this chose among
+                               need one segment for the whole warp        */
   uint32_t refine_coop;     /* refinement: a candidate's neighbour segment
                                longer than this is scanned by the whole warp
                                (warp per candidate), shorter ones by the
