@@ -35,6 +35,7 @@ struct DeviceGraph {
   uint32_t* adj_old = nullptr;     // [nadj] caller id of each adj entry (for the result hash); null without lseg
   uint32_t* lseg = nullptr;        // [V*(L+1)]; null: segments are found by binary search in the rows
   uint4* sig = nullptr;            // [V*4] 64-byte signature per vertex
+  uint16_t* filt = nullptr;        // [nadj] membership filter, in the arena's tail; valid while that is kept
   std::vector<uint32_t> h_base;    // host copy of base
   uint64_t arena_mark = 0;         // arena top after the graph store
 };
@@ -50,10 +51,9 @@ struct Engine {
   // pinned host staging for batches
   void* pinned = nullptr;
   uint64_t pinned_bytes = 0;
-  // enumeration kernel: resident blocks per SM at 1..8 warps per block and 1..31
-  // depths with a buffer (0 until queried), with and without a segment table
-  int enum_per_sm[9][32] = {};
-  int enum_per_sm_rows[9][32] = {};
+  // enumeration kernel: resident blocks per SM (0 until first queried)
+  int enum_per_sm[9] = {0};       // resident blocks per SM at 1..8 warps per block (0 until queried)
+  int enum_per_sm_rows[9] = {0};  // the same for a graph store without a segment table
   int seg_index = 0;              // segment index of the next graph build (FSIG_SEGMENTS_*)
   // timing events
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};

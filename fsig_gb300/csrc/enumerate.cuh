@@ -10,8 +10,8 @@
 // every depth it keeps a buffer of up to 32 mapped vertices in shared memory,
 // each with the slot of its parent in the previous depth's buffer; an entry's
 // earlier vertices are found by walking its parents.  Lane j holds depth j's
-// cursor (cnt_j entries, it_j the first one not wholly extended, off_j how
-// much of that one's driver range is examined).
+// cursor (cnt_j entries from sp_j on, it_j the first one not wholly extended,
+// off_j how much of that one's driver range is examined).
 //
 // Filling the buffer of depth i from depth i-1's entries: each lane takes one
 // entry, finds the label-l(i) segments of its backward neighbours' rows
@@ -21,10 +21,11 @@
 // from the bits where a driver begins in this window.  A candidate passes
 // when its bit in depth i's candidate bitmap is set, it differs from the
 // entry's earlier vertices of the same label (adjacent ones differ anyway),
-// and it lies in each of the entry's other backward segments, two per-lane
-// binary searches in lockstep (two independent loads in flight).  Candidates
-// that pass the first two tests are appended to depth i's buffer and searched
-// for once it is full, so that the searches run on all lanes; those found stay.
+// and it lies in each of the entry's other backward segments.  The store's
+// membership filter settles most of these by one load (common.cuh); candidates
+// that pass every filter are appended to depth i's buffer and, where a filter
+// is not exact, searched for once the buffer is full, so that the searches (two
+// per-lane binary searches in lockstep) run on all lanes; those found stay.
 // A buffer with enough entries is extended in turn, and later the fill goes on
 // where it stopped.  At the leaf the passing candidates are counted and hashed.
 //
@@ -34,8 +35,11 @@
 // neighbours after another) and paid the set-up of a range, some 300
 // instructions, for each.  200 eight-vertex queries there 115 -> 34 ms of
 // kernel, 512 queries of 4-32 vertices 69 -> 34 ms, 253 instructions a window
-// at 79 % of the issue rate.  On 2^26 edges, where the searches dominate, it is
-// bound by their latency at 24 warps an SM (49 % of the issue rate).
+// at 79 % of the issue rate.  With the filter, a leaf loop of its own for
+// leaves of one segment, and buffers of one pool per warp (4 blocks an SM also
+// for 32-vertex queries, 3 with 32 entries for each depth): 27 and 23 ms, 198
+// instructions a window at 70 % of the issue rate; 512 queries of 12-32 vertices
+// on 2^26 edges 305 -> 146 ms, 279 instructions a window at 64 %.
 //
 // Work stealing: a warp that runs out of input takes a ticket, one atomicAdd
 // on the queue's head, and waits for the record of that number, polling the
@@ -109,7 +113,6 @@ struct EnumArgs {
   // written but never published, so the warp that takes it waits out
   // ready_wait_ns and the pass reports a timeout
   uint32_t unpublished;
-  uint32_t levels;  // depths with a buffer: the batch's largest query minus one, at least 1
 };
 
 constexpr uint32_t kErrTimeout = 1u;
@@ -136,19 +139,33 @@ constexpr uint32_t kFillWindows = 64;
 // Windows between two checks of the work limit and of the waiting warps.
 constexpr uint32_t kCheckWindows = 32;
 
-// Per warp; followed by cand[levels][kBuf] and par[levels][kBuf], levels = the
-// batch's largest query minus one.
+constexpr uint32_t kPool = 512;      // entries of all buffers of a warp (see below)
+
+// Per warp.  The depths' buffers lie one after another in the pool, each as
+// long as it is filled; a fill takes at most kBuf entries and leaves one for
+// each depth below it.  (A fixed 32 entries for each of 31 depths would allow 3
+// blocks an SM instead of 4.)
 struct WarpSmem {
   Plan plan;
   uint2 owner[kBuf];                // entries with a driver: its place relative to the window index, the entry
   unsigned long long sown[kBuf];    // leaf: partial hash of each entry being extended
   unsigned long long sbase[kBuf];   // partial hashes of depth n-3's buffer
-  uint32_t scratch[kScratch];
-  uint8_t drv[kBuf];                // driver of each entry being extended (its place in scratch)
+  uint2 scratch[kScratch / 2];      // per entry being extended: segments (start, length), then earlier vertices
+  uint32_t cand[kPool];             // mapped vertex
+  uint8_t par[kPool];               // its parent's place in the previous depth's buffer
+  // event counters of the warp's share of one launch, kept here for the registers
+  // (lane 0): tasks, records popped, hand-offs, records written, windows
+  uint32_t ev[5];
+  uint32_t pend;                    // driver entries examined, not yet published to res.work (lane 0)
+  uint32_t task_lo, task_hi;        // driver range of the task at its first depth
 };
+static_assert(sizeof(WarpSmem) % 16 == 0, "the next warp's part is aligned");
 
-constexpr size_t warp_smem_bytes(uint32_t levels) {
-  return (sizeof(WarpSmem) + size_t(levels) * kBuf * 5 + 15) & ~size_t(15);
+// 1 << s, 0 for s >= 32
+__device__ __forceinline__ uint32_t bit_or_zero(uint32_t s) {
+  uint32_t r;
+  asm("shl.b32 %0, %1, %2;" : "=r"(r) : "r"(1u), "r"(s));
+  return r;
 }
 
 // Segment [lo, hi) of row v's neighbours with label l (0 <= l < L): two loads
@@ -168,12 +185,12 @@ __device__ __forceinline__ void row_segment(const GraphView& g, uint32_t v, int3
   }
 }
 
-// Whether x lies in both sorted segments a[lo0, hi0) and a[lo1, hi1) (in the
-// first alone without `two`): two binary searches in lockstep, so that a step
+// Whether x lies in both sorted segments a[lo0, lo0 + n0) and a[lo1, lo1 + n1)
+// (in the first alone without `two`): two binary searches in lockstep, so that a step
 // has two independent loads in flight.
-__device__ __forceinline__ bool in_segments(const uint32_t* __restrict__ a, uint32_t lo0, uint32_t hi0, uint32_t lo1,
-                                            uint32_t hi1, bool two, uint32_t x, uint32_t& bytes) {
-  uint32_t n0 = hi0 - lo0, n1 = two ? hi1 - lo1 : 1;
+__device__ __forceinline__ bool in_segments(const uint32_t* __restrict__ a, uint32_t lo0, uint32_t n0, uint32_t lo1,
+                                            uint32_t n1, bool two, uint32_t x, uint32_t& bytes) {
+  if (!two) n1 = 1;
   if (n0 == 0 || n1 == 0) return false;
 #pragma unroll 1
   while (n0 > 1 || n1 > 1) {
@@ -195,9 +212,7 @@ __device__ __forceinline__ bool in_segments(const uint32_t* __restrict__ a, uint
 template <bool kRows>
 __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_kernel(EnumArgs A) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  WarpSmem& ws = *reinterpret_cast<WarpSmem*>(smem_raw + warp_smem_bytes(A.levels) * (threadIdx.x >> 5));
-  uint32_t* const cand = reinterpret_cast<uint32_t*>(&ws + 1);              // [levels][kBuf]
-  uint8_t* const par = reinterpret_cast<uint8_t*>(cand + A.levels * kBuf);  // [levels][kBuf]
+  WarpSmem& ws = reinterpret_cast<WarpSmem*>(smem_raw)[threadIdx.x >> 5];
   const uint32_t lane = threadIdx.x & 31;
   const GraphView& g = A.g;
   const uint64_t W1 = uint64_t(g.L) + 1;
@@ -205,14 +220,14 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
   const uint32_t T_in = A.in_tasks ? A.in_count : min(A.chunk_off[nroots], A.t_end);
 
   // lane-distributed level state; f is the task's prefix (lane j: f_j)
-  uint32_t f = 0, cnt = 0, it = 0, off = 0;
+  uint32_t f = 0, cnt = 0, it = 0, off = 0, sp = 0;  // sp: where depth j's buffer starts in the pool
   unsigned long long my_hash = 0;
   bool s_valid = false;  // sbase holds depth n-3's current buffer
   unsigned long long lc = 0;  // lane j: partial embeddings of length j + 1 found (lane n-1: embeddings)
   uint32_t bytes = 0;         // drained into the 64-bit total before it can overflow
-  uint32_t pend = 0;          // driver entries examined, not yet published to res.work (lane 0)
-  // event counters (lane 0); a warp's share of one launch fits 32 bits
-  uint32_t n_tasks = 0, n_pops = 0, n_handoffs = 0, n_recs = 0, n_examine = 0;
+  if (lane < 5) ws.ev[lane] = 0;
+  if (lane == 0) ws.pend = 0;
+  __syncwarp();
   uint32_t cur_q = kInvalid;
 
   // Publishes the driver entries this warp examined for the current query.
@@ -220,9 +235,9 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
   // (every driver entry counts once), so whether it exceeds the limit does not
   // either.
   auto publish = [&]() {
-    if (lane == 0 && pend) {
-      const unsigned long long tot = atomicAdd(&A.res[cur_q].work, (unsigned long long)pend) + pend;
-      pend = 0;
+    if (lane == 0 && ws.pend) {
+      const unsigned long long tot = atomicAdd(&A.res[cur_q].work, (unsigned long long)ws.pend) + ws.pend;
+      ws.pend = 0;
       if (tot > A.work_cap) atomicExch(&A.res[cur_q].aborted, 1u);
     }
   };
@@ -232,10 +247,11 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
     uint32_t v = 0;
 #pragma unroll 1
     for (uint32_t k = p;; k--) {
-      const uint32_t x = cand[k * kBuf + slot];
+      const uint32_t at = __shfl_sync(kFull, sp, k) + slot;
+      const uint32_t x = ws.cand[at];
       if (lane == k) v = x;
       if (k == 0) break;
-      slot = par[k * kBuf + slot];
+      slot = ws.par[at];
     }
     return v;
   };
@@ -328,7 +344,10 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
     for (uint32_t k = base + lane; k < base + total; k += 32)
       if (!(hold && k == base))
         atomicExch(&A.out_ready[k & (A.out_cap - 1)], 2 * (k >> (31 - __clz(A.out_cap))) + 1);
-    if (lane == 0) { n_handoffs++; n_recs += total; }
+    if (lane == 0) {
+      ws.ev[2]++;
+      ws.ev[3] += total;
+    }
     return true;
   };
 
@@ -346,19 +365,21 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
   };
 
   // Writes the embeddings completed by one leaf window: lanes in m hold a
-  // leaf's caller id in xo and its entry's slot in depth n-2's buffer.
+  // leaf's caller id in xo and its entry's place in depth n-2's buffer.
   auto emit_rows = [&](uint32_t m, uint32_t n, uint32_t xo, uint32_t slot) {
     unsigned long long base = 0;
     if (lane == 0) base = atomicAdd(A.emit_ctr, (unsigned long long)__popc(m));
     base = __shfl_sync(kFull, base, 0);
     const unsigned long long row = base + __popc(m & lanemask_lt());
-    if (((m >> lane) & 1u) && row < A.emit_cap) {
-      uint32_t* dst = A.emit + row * n;
-      dst[ws.plan.qv[n - 1]] = xo;
+    const bool mine = ((m >> lane) & 1u) && row < A.emit_cap;
+    uint32_t* dst = A.emit + row * n;
+    if (mine) dst[ws.plan.qv[n - 1]] = xo;
 #pragma unroll 1
-      for (uint32_t k = n - 1; k-- > 0;) {
-        dst[ws.plan.qv[k]] = __ldg(g.old_of_new + cand[k * kBuf + slot]);
-        slot = par[k * kBuf + slot];
+    for (uint32_t k = n - 1; k-- > 0;) {
+      const uint32_t at = __shfl_sync(kFull, sp, k) + slot;
+      if (mine) {
+        dst[ws.plan.qv[k]] = __ldg(g.old_of_new + ws.cand[at]);
+        slot = ws.par[at];
       }
     }
   };
@@ -369,75 +390,86 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
   // entry there is.  Returns the windows examined; the cursors of depths lv - 1
   // and lv say where it stopped.
   auto fill = [&](uint32_t lv, uint32_t lo_set, uint32_t hi_set) -> uint32_t {
-    const bool leaf = lv + 1 == ws.plan.n;
-    const uint32_t p = lv - 1;
+    const uint32_t n = ws.plan.n, p = lv - 1;
+    const bool leaf = lv + 1 == n;
     const uint32_t bwd = ws.plan.bwd[lv], inj = ws.plan.same[lv] & ~bwd;
     const int32_t lab = ws.plan.lab[lv];
     const uint32_t nb = __popc(bwd), ni = __popc(inj);
     const uint32_t stride = min(kBuf, kScratch / (2 * nb + ni));  // entries per group
+    uint32_t* const other = reinterpret_cast<uint32_t*>(ws.scratch + nb * stride);  // [ni][stride]
     const uint32_t bmbase = ws.plan.bmbase[lv];
     const uint32_t* __restrict__ bm = A.pool + ws.plan.bmoff[lv];
-    const uint32_t cntp = __shfl_sync(kFull, cnt, p);
+    // segments from this length on have an exact filter
+    const uint32_t dense = g.filt ? filter_dense_len(__ldg(g.base + lab + 1) - bmbase) : kInvalid;
+    const uint32_t cntp = __shfl_sync(kFull, cnt, p), spp = __shfl_sync(kFull, sp, p);
+    const uint32_t spl = spp + cntp;                              // depth lv's buffer
+    const uint32_t room = min(kBuf, kPool - spl - (n - 2 - min(lv, n - 2)));
+    // Entries that end a fill.  With further segments to search the room left
+    // decides how many lanes search, so half the buffer is enough.
+    const uint32_t enough = nb > 1 || room < 16 ? (room + 1) / 2 : room - 8;
     uint32_t itp = __shfl_sync(kFull, it, p), offp = __shfl_sync(kFull, off, p);
-    uint32_t have = 0, sure = 0, used = 0;  // entries appended; of them, searched for in every segment
+    uint32_t have = 0, sure = 0;  // entries appended; of them, searched for in every segment
+    uint32_t used = 0, seen = 0, hits = 0;
     bool stop = false;
     if (leaf && !s_valid && lv >= 2) {  // partial hashes of depth n-3's entries
-      const uint32_t c = __shfl_sync(kFull, cnt, lv - 2);
-      if (lane < c) {
-        unsigned long long sum = 0;
-        uint32_t slot = lane;
+      unsigned long long sum = 0;
+      uint32_t slot = min(lane, __shfl_sync(kFull, cnt, lv - 2) - 1);
 #pragma unroll 1
-        for (uint32_t k = lv - 1; k-- > 0;) {
-          sum += fmix64((uint64_t(ws.plan.qv[k]) << 32) | __ldg(g.old_of_new + cand[k * kBuf + slot]));
-          slot = par[k * kBuf + slot];
-        }
-        ws.sbase[lane] = sum;
+      for (uint32_t k = lv - 1; k-- > 0;) {
+        const uint32_t at = __shfl_sync(kFull, sp, k) + slot;
+        sum += fmix64((uint64_t(ws.plan.qv[k]) << 32) | __ldg(g.old_of_new + ws.cand[at]));
+        slot = ws.par[at];
       }
+      ws.sbase[lane] = sum;
       s_valid = true;
       __syncwarp();
     }
     while (itp < cntp && !stop) {
-      // the group: lane c takes entry itp + c
+      // the group: lane c takes entry itp + c (lanes past the group repeat its last one)
       uint32_t group = min(cntp - itp, stride);
-      uint32_t dlo = 0, dhi = 0, drv = 0;
-      if (lane < group) {
-        uint32_t slot = itp + lane, need = bwd | inj, wb = 0, wi = 2 * nb, best = kInvalid;
+      const bool mine = lane < group;
+      const uint32_t own = spp + itp + min(lane, group - 1);
+      uint32_t dlo = 0, len = kInvalid, drv = 0;
+      {
+        uint32_t at = own, need = bwd | inj, wb = 0, wi = 0;
 #pragma unroll 1
         for (uint32_t k = p;; k--) {
+          const uint32_t v = ws.cand[at];
           if ((bwd >> k) & 1u) {
             uint32_t a, b;
-            row_segment<kRows>(g, cand[k * kBuf + slot], lab, W1, a, b);
-            ws.scratch[wb * stride + lane] = a;
-            ws.scratch[(wb + 1) * stride + lane] = b;
-            if (b - a < best) {
-              best = b - a;
+            row_segment<kRows>(g, v, lab, W1, a, b);
+            if (mine) ws.scratch[wb * stride + lane] = make_uint2(a, b - a);
+            if (b - a < len) {
+              len = b - a;
               dlo = a;
-              dhi = b;
               drv = wb;
             }
-            wb += 2;
-            bytes += 8;
+            wb++;
           } else if ((inj >> k) & 1u) {
-            ws.scratch[wi++ * stride + lane] = cand[k * kBuf + slot];
+            if (mine) other[wi * stride + lane] = v;
+            wi++;
           }
           need &= ~(1u << k);
           if (!need) break;
-          slot = par[k * kBuf + slot];
+          at = __shfl_sync(kFull, sp, k - 1) + ws.par[at];
         }
+        bytes += 8 * nb;
+        if (mine && drv) ws.scratch[drv * stride + lane] = ws.scratch[lane];  // the others: places 1 .. nb - 1
         if (lo_set != kInvalid) {
           dlo = lo_set;
-          dhi = hi_set;
+          len = hi_set - lo_set;
         }
-        if (lane == 0) dlo = min(dlo + offp, dhi);
-        if (leaf) {
-          unsigned long long sum =
-              fmix64((uint64_t(ws.plan.qv[p]) << 32) | __ldg(g.old_of_new + cand[p * kBuf + itp + lane]));
-          if (p > 0) sum += ws.sbase[par[p * kBuf + itp + lane]];
-          ws.sown[lane] = sum;
-          bytes += 4;
+        if (lane == 0) {
+          dlo += offp;
+          len -= offp;
         }
+        if (!mine) len = 0;
       }
-      uint32_t len = dhi - dlo;
+      if (leaf) {
+        unsigned long long sum = fmix64((uint64_t(ws.plan.qv[p]) << 32) | __ldg(g.old_of_new + ws.cand[own]));
+        if (p > 0) sum += ws.sbase[ws.par[own]];
+        ws.sown[lane] = sum;
+      }
       if (__any_sync(kFull, len >= (1u << 27))) {  // the group's total has to fit 32 bits
         group = 1;
         if (lane) len = 0;
@@ -448,125 +480,165 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
         const uint32_t y = __shfl_up_sync(kFull, incl, o);
         if (lane >= uint32_t(o)) incl += y;
       }
-      const uint32_t start = incl - len, T = __shfl_sync(kFull, incl, 31);
-      const uint32_t full = __ballot_sync(kFull, len > 0);
-      if (len > 0) ws.owner[__popc(full & lanemask_lt())] = make_uint2(dlo - start, lane);
-      ws.drv[lane] = uint8_t(drv);
+      const uint32_t T = __shfl_sync(kFull, incl, 31);
+      const uint32_t start = len ? incl - len : kInvalid;
+      {
+        const uint32_t rank = __popc(__ballot_sync(kFull, len != 0) & lanemask_lt());
+        if (len) ws.owner[rank] = make_uint2(dlo - start, lane);
+      }
       __syncwarp();
-      uint32_t pos = 0, begun = 0;  // begun: drivers that start before pos
-      while (pos < T && !stop) {
-        const uint32_t at = start - pos;
-        const uint32_t heads = __reduce_or_sync(kFull, (len > 0 && start >= pos && at < 32) ? 1u << at : 0u);
-        const uint32_t r = begun + __popc(heads & (lanemask_lt() | (1u << lane))) - 1;
-        const uint32_t e = pos + lane;
-        bool pred = e < T;
-        uint32_t x = 0xffffffffu, xo = 0, c = 0;
-        if (pred) {
-          const uint2 o = ws.owner[r];
-          c = o.y;
-          x = __ldg(g.adj + (o.x + e));
-          if (leaf && !kRows) xo = __ldg(g.adj_old + (o.x + e));
-          const uint32_t bit = x - bmbase;
-          bytes += leaf ? 12 : 8;
-          pred = (__ldg(bm + (bit >> 5)) >> (bit & 31)) & 1u;
-        }
+      uint32_t pos = 0, begun = kInvalid;  // begun: drivers that start before pos, minus one
+      if (leaf && nb == 1 && !A.emit) {
+        // the common leaf: nothing to search, all lanes alike
+        const uint64_t tq = uint64_t(ws.plan.qv[lv]) << 32;
 #pragma unroll 1
-        for (uint32_t i = 0; i < ni; i++) pred = pred && x != ws.scratch[(2 * nb + i) * stride + c];
+        while (pos < T && !stop) {
+          const uint32_t heads = __reduce_or_sync(kFull, bit_or_zero(start - pos));
+          const uint2 o = ws.owner[begun + __popc(heads & lanemask_le())];
+          const uint32_t e = pos + lane, at = o.x + min(e, T - 1);
+          const uint32_t x = __ldg(g.adj + at);
+          const uint32_t xo = kRows ? __ldg(g.old_of_new + x) : __ldg(g.adj_old + at);
+          const uint32_t bit = x - bmbase;
+          bool pred = e < T && ((__ldg(bm + (bit >> 5)) >> (bit & 31)) & 1u);
+#pragma unroll 1
+          for (uint32_t i = 0; i < ni; i++) pred = pred && x != other[i * stride + o.y];
+          const uint64_t h = fmix64(A.seed + ws.sown[o.y] + fmix64(tq | xo));
+          my_hash += pred ? h : 0;
+          hits += pred;
+          begun += __popc(heads);
+          pos += 32;
+          stop = ++used >= kFillWindows;
+        }
+        pos = min(pos, T);
+        seen += pos;
+      }
+#pragma unroll 1
+      while (pos < T && !stop) {
+        const uint32_t heads = __reduce_or_sync(kFull, bit_or_zero(start - pos));
+        const uint2 o = ws.owner[begun + __popc(heads & lanemask_le())];
+        const uint32_t e = pos + lane, at = o.x + min(e, T - 1);
+        uint32_t x = __ldg(g.adj + at), c = o.y;
+        const uint32_t bit = x - bmbase;
+        bool pred = e < T && ((__ldg(bm + (bit >> 5)) >> (bit & 31)) & 1u);
+#pragma unroll 1
+        for (uint32_t i = 0; i < ni; i++) pred = pred && x != other[i * stride + c];
+        if (nb > 1 && g.filt) {
+          // the other segments' filters, two at a time
+          const uint32_t hash = filter_hash(x), bits = filter_bits(x);
+#pragma unroll 1
+          for (uint32_t k = 1; k < nb && __any_sync(kFull, pred); k += 2) {
+            const uint2 a = ws.scratch[k * stride + c], b = ws.scratch[min(k + 1, nb - 1) * stride + c];
+            const bool da = a.y >= dense, db = b.y >= dense;
+            uint32_t wa = 0, wb = 0;
+            if (pred) {
+              wa = __ldg(g.filt + a.x + filter_word(da, bit, hash, a.y));
+              wb = __ldg(g.filt + b.x + filter_word(db, bit, hash, b.y));
+              bytes += 4;
+            }
+            pred = ((~wa & filter_mask(da, bit, bits)) | (~wb & filter_mask(db, bit, bits))) == 0;
+          }
+        }
         uint32_t step = min(32u, T - pos);
         bool searching = leaf && nb > 1;
         used++;
         if (!leaf) {
           uint32_t m = __ballot_sync(kFull, pred);
-          const uint32_t got = __popc(m), rank = __popc(m & lanemask_lt());
-          if (have + got > kBuf) {  // take what fits; go on from the first one that does not
-            step = __ffs(__ballot_sync(kFull, pred && have + rank == kBuf)) - 1;
+          const uint32_t rank = have + __popc(m & lanemask_lt());
+          if (have + __popc(m) > room) {  // take what fits; go on from the first one that does not
+            step = __ffs(__ballot_sync(kFull, pred && rank == room)) - 1;
             m &= (1u << step) - 1;
           }
           if ((m >> lane) & 1u) {
-            cand[lv * kBuf + have + rank] = x;
-            par[lv * kBuf + have + rank] = uint8_t(itp + c);
+            ws.cand[spl + rank] = x;
+            ws.par[spl + rank] = uint8_t(itp + c);
           }
           have += __popc(m);
-          searching = nb > 1 && have > sure && (have == kBuf || pos + step >= T || used >= kFillWindows);
-          __syncwarp();
+          searching = nb > 1 && have > sure && (have == room || pos + step >= T || used >= kFillWindows);
           if (searching) {  // the entries not yet searched for, one per lane
+            __syncwarp();
             pred = lane >= sure && lane < have;
             if (pred) {
-              x = cand[lv * kBuf + lane];
-              c = par[lv * kBuf + lane] - itp;
+              x = ws.cand[spl + lane];
+              c = ws.par[spl + lane] - itp;
             }
           }
         }
         if (searching && pred) {
-          // the entry's other segments, two at a time
-          const uint32_t dseg = ws.drv[c];
-          uint32_t s = dseg == 0 ? 2 : 0;
+          // the other segments whose filter is not exact, two at a time
+          uint32_t k = 1;
 #pragma unroll 1
-          while (pred && s < 2 * nb) {
-            const uint32_t s1 = s + 2 == dseg ? s + 4 : s + 2;
-            const bool two = s1 < 2 * nb;
-            const uint32_t s2 = two ? s1 : s;
-            pred = in_segments(g.adj, ws.scratch[s * stride + c], ws.scratch[(s + 1) * stride + c],
-                               ws.scratch[s2 * stride + c], ws.scratch[(s2 + 1) * stride + c], two, x, bytes);
-            s = s1 + 2 == dseg ? s1 + 4 : s1 + 2;
+          while (pred && k < nb) {
+            uint2 a = ws.scratch[k++ * stride + c];
+            if (a.y >= dense) continue;
+            uint2 b = a;
+            bool two = false;
+#pragma unroll 1
+            while (k < nb && !two) {
+              b = ws.scratch[k++ * stride + c];
+              two = b.y < dense;
+            }
+            pred = in_segments(g.adj, a.x, a.y, b.x, b.y, two, x, bytes);
           }
         }
         __syncwarp();
         if (leaf) {
-          const uint32_t m = __ballot_sync(kFull, pred);
-          if (pred) {
-            if (kRows) xo = __ldg(g.old_of_new + x);
-            my_hash += fmix64(A.seed + ws.sown[c] + fmix64((uint64_t(ws.plan.qv[lv]) << 32) | xo));
+          const uint32_t xo = kRows ? __ldg(g.old_of_new + x) : __ldg(g.adj_old + at);
+          const uint64_t h = fmix64(A.seed + ws.sown[c] + fmix64((uint64_t(ws.plan.qv[lv]) << 32) | xo));
+          my_hash += pred ? h : 0;
+          hits += pred;
+          if (A.emit) {
+            const uint32_t m = __ballot_sync(kFull, pred);
+            if (m) emit_rows(m, n, xo, itp + c);
           }
-          if (A.emit && m) emit_rows(m, lv + 1, xo, itp + c);
-          if (lane == lv) lc += __popc(m);
         } else {
           if (searching) {
             const uint32_t m = __ballot_sync(kFull, pred);
-            have = sure + __popc(m);
             if (pred) {
-              cand[lv * kBuf + sure + __popc(m & lanemask_lt())] = x;
-              par[lv * kBuf + sure + __popc(m & lanemask_lt())] = uint8_t(itp + c);
+              const uint32_t to = spl + sure + __popc(m & lanemask_lt());
+              ws.cand[to] = x;
+              ws.par[to] = uint8_t(itp + c);
             }
-            sure = have;
+            have = sure + __popc(m);
             __syncwarp();
           }
-          // enough entries: with further segments to search the room that is
-          // left decides how many lanes search
-          if (nb == 1) sure = have;
-          stop = sure >= (nb > 1 ? kBuf / 2 : kBuf - 8);
-        }
-        if (lane == 0) {
-          n_examine++;
-          if (A.work_cap) pend += step;
+          if (searching || nb == 1) sure = have;
+          stop = sure >= enough;
         }
         begun += __popc(step < 32 ? heads & ((1u << step) - 1) : heads);
         pos += step;
+        seen += step;
         stop = stop || used >= kFillWindows;
       }
       if (pos >= T) {
         itp += group;
         offp = 0;
       } else {  // inside the last driver begun at or before pos
-        const uint32_t o = 31 - __clz(__ballot_sync(kFull, len > 0 && start <= pos));
+        const uint32_t o = 31 - __clz(__ballot_sync(kFull, start <= pos));
         offp = pos - __shfl_sync(kFull, start, o) + (o == 0 ? offp : 0u);
         itp += o;
       }
       __syncwarp();
     }
+    if (leaf) have = __reduce_add_sync(kFull, hits);
     if (lane == p) {
       it = itp;
       off = offp;
     }
-    if (!leaf) {
-      if (lane == lv) {
+    if (lane == lv) {
+      lc += have;
+      if (!leaf) {
         cnt = have;
         it = 0;
         off = 0;
-        lc += have;
+        sp = spl;
       }
-      if (lv + 3 == ws.plan.n) s_valid = false;
     }
+    if (lv + 3 == n) s_valid = false;
+    if (lane == 0) {
+      ws.ev[4] += used;
+      if (A.work_cap) ws.pend += seen;
+    }
+    bytes += leaf ? 12 * used : 8 * used;
     return used;
   };
 
@@ -646,7 +718,7 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
       slot = __shfl_sync(kFull, slot, 0);
       if (slot != kInvalid) {
         __threadfence();
-        if (lane == 0) n_pops++;
+        if (lane == 0) ws.ev[1]++;
         rec = A.out_tasks + (slot & (A.out_cap - 1));
         ready = A.out_ready + (slot & (A.out_cap - 1));
         free_word = 2 * (slot >> (31 - __clz(A.out_cap))) + 2;
@@ -706,7 +778,7 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
         hi = min(lo + A.split, hi);
       }
     }
-    if (lane == 0) n_tasks++;
+    if (lane == 0) ws.ev[0]++;
     if (d == n) {  // a complete embedding (single-vertex queries)
       if (lane == 0) {
         const uint32_t xo = __ldg(g.old_of_new + f);
@@ -723,9 +795,14 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
     const uint32_t t_start = uint32_t(clock());
     __syncwarp();
     if (lane < d) {
-      cand[lane * kBuf] = f;
-      par[lane * kBuf] = 0;
+      ws.cand[lane] = f;
+      ws.par[lane] = 0;
     }
+    if (lane == 0) {
+      ws.task_lo = lo;
+      ws.task_hi = hi;
+    }
+    sp = lane;
     cnt = lane < d ? 1u : 0u;
     it = lane + 1 < d ? 1u : 0u;
     off = 0;
@@ -755,7 +832,7 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
         if (hungry) {
           // the entries of the leaf's ranges are handed off only when those are long
           const uint32_t last = (lv + 1 == n && used >= kFillWindows) ? n - 1 : n - 2;  // plus one
-          if (last >= d) donate(d, min(lv, last - 1), hungry, lo, hi);
+          if (last >= d) donate(d, min(lv, last - 1), hungry, ws.task_lo, ws.task_hi);
         }
       }
       if (__shfl_sync(kFull, it, lv - 1) >= __shfl_sync(kFull, cnt, lv - 1)) {
@@ -763,7 +840,7 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
         lv--;
         continue;
       }
-      used = fill(lv, lv == d ? lo : kInvalid, hi);
+      used = fill(lv, lv == d ? ws.task_lo : kInvalid, ws.task_hi);
       windows += used + 1;
       if (lv + 1 < n && __shfl_sync(kFull, cnt, lv) > 0) lv++;
     }
@@ -771,11 +848,8 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
   const unsigned long long all_bytes = warp_sum((unsigned long long)bytes);
   if (lane == 0) {
     atomicAdd(A.algo_bytes, all_bytes);
-    atomicAdd(&A.ev[0], (unsigned long long)n_tasks);
-    atomicAdd(&A.ev[1], (unsigned long long)n_pops);
-    atomicAdd(&A.ev[2], (unsigned long long)n_handoffs);
-    atomicAdd(&A.ev[3], (unsigned long long)n_recs);
-    atomicAdd(&A.ev[4], (unsigned long long)n_examine);
+#pragma unroll 1
+    for (int i = 0; i < 5; i++) atomicAdd(&A.ev[i], (unsigned long long)ws.ev[i]);
   }
 }
 

@@ -289,6 +289,53 @@ __global__ void signature_from_rows_kernel(const int32_t* __restrict__ label, co
   }
 }
 
+// Membership filter (common.cuh), a warp per 256 adjacency entries, one entry
+// per lane and step; the lane's row is found from the previous one by
+// galloping (rows average a step or two apart).  Bound by the atomics, all to
+// words near the entry's own position: L2.
+constexpr uint32_t kFilterRun = 256;
+__global__ void __launch_bounds__(256) membership_filter_kernel(
+    const uint32_t* __restrict__ off, const uint32_t* __restrict__ adj, const int32_t* __restrict__ label,
+    const uint32_t* __restrict__ base, const uint32_t* __restrict__ lseg, uint32_t V, int32_t L, uint32_t nadj,
+    uint32_t* __restrict__ filt) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint64_t nwarps = (uint64_t(gridDim.x) * blockDim.x) >> 5;
+  for (uint64_t run = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; run * kFilterRun < nadj; run += nwarps) {
+    uint32_t lo = 0, hi = V;  // row of the run's first entry: the last v with off[v] <= k
+    const uint32_t first = uint32_t(run * kFilterRun);
+    while (hi - lo > 1) {
+      const uint32_t mid = (lo + hi) >> 1;
+      if (off[mid] <= first) lo = mid; else hi = mid;
+    }
+    uint32_t v = lo;
+    const uint32_t last = uint32_t(min(uint64_t(first) + kFilterRun, uint64_t(nadj)));
+    for (uint32_t k = first + lane; k < last; k += 32) {
+      uint32_t step = 1;
+      while (v + step < V && off[v + step] <= k) {
+        v += step;
+        step <<= 1;
+      }
+      for (; step; step >>= 1)
+        if (v + step < V && off[v + step] <= k) v += step;
+      const uint32_t x = adj[k];
+      const int32_t l = label[x];
+      uint32_t a, b;
+      if (lseg) {
+        const uint32_t* s = lseg + uint64_t(v) * (uint64_t(L) + 1) + l;
+        a = s[0];
+        b = s[1];
+      } else {
+        a = lower_bound_u32(adj, off[v], k, base[l]);
+        b = lower_bound_u32(adj, k, off[v + 1], base[l + 1]);
+      }
+      const uint32_t first_id = base[l] & ~31u, rel = x - first_id;
+      const bool dense = b - a >= filter_dense_len(base[l + 1] - first_id);
+      const uint32_t w = a + filter_word(dense, rel, filter_hash(x), b - a);
+      atomicOr(&filt[w >> 1], filter_mask(dense, rel, filter_bits(x)) << ((w & 1u) * 16));
+    }
+  }
+}
+
 __global__ void gather_kernel(const uint32_t* __restrict__ idx, uint64_t n, const uint32_t* __restrict__ table,
                               uint32_t* out) {
   for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n; i += uint64_t(gridDim.x) * blockDim.x)
@@ -355,6 +402,25 @@ int build_rows(Engine& e, const uint2* d_edges, uint64_t E, uint32_t V, const ui
   return FSIG_OK;
 }
 
+// Arena bytes left free beside the membership filter when it is built: a
+// batch's work queues and room for a batch.
+constexpr uint64_t kFilterSpare = 1ull << 30;
+
+// The membership filter in the arena's tail, when there is room to spare;
+// without it the enumeration searches the segments themselves.
+int build_membership_filter(Engine& e, DeviceGraph& g) {
+  g.filt = nullptr;
+  if (!g.nadj) return FSIG_OK;
+  uint32_t* filt = e.arena.take_tail<uint32_t>((g.nadj + 1) / 2, kFilterSpare);
+  if (!filt) return FSIG_OK;
+  FSIG_CUDA_TRY(cudaMemsetAsync(filt, 0, sizeof(uint32_t) * ((g.nadj + 1) / 2), e.stream));
+  membership_filter_kernel<<<grid_for((g.nadj + kFilterRun - 1) / kFilterRun * 32, 256, e.num_sms), 256, 0, e.stream>>>(
+      g.off, g.adj, g.label, g.base, g.lseg, g.V, g.L, uint32_t(g.nadj), filt);
+  FSIG_CUDA_TRY(cudaGetLastError());
+  g.filt = reinterpret_cast<uint16_t*>(filt);
+  return FSIG_OK;
+}
+
 }  // namespace
 
 bool use_segment_table(int mode, uint32_t V, int32_t L, uint64_t nadj) {
@@ -376,6 +442,7 @@ int build_device_graph(Engine& e, uint32_t V, const int32_t* h_labels, uint64_t 
   if (2 * E > 0xffffffffull) return fail(FSIG_EINVAL, "graph has 2^31 or more edges");
   // Reset any previous graph.
   e.arena.release(0);
+  e.arena.tail = 0;
   e.has_graph = false;
   DeviceGraph g;
   g.V = V;
@@ -500,6 +567,8 @@ int build_device_graph(Engine& e, uint32_t V, const int32_t* h_labels, uint64_t 
     e.arena.release(mm);
   }
   g.arena_mark = e.arena.mark();
+  rc = build_membership_filter(e, g);
+  if (rc) return rc;
   e.g = g;
   e.has_graph = true;
   return FSIG_OK;
@@ -584,6 +653,7 @@ int load_graph_cache(Engine& e, const char* path) {
     return fail(FSIG_EIO, std::string(path) + " is not a graph cache of this engine");
   }
   e.arena.release(0);
+  e.arena.tail = 0;
   e.has_graph = false;
   DeviceGraph g;
   g.V = h.V;
@@ -623,6 +693,9 @@ int load_graph_cache(Engine& e, const char* path) {
   g.h_base.resize(L1);
   FSIG_CUDA_TRY(cudaMemcpy(g.h_base.data(), g.base, 4 * L1, cudaMemcpyDeviceToHost));
   g.arena_mark = e.arena.mark();
+  const int rc = build_membership_filter(e, g);
+  if (rc) return rc;
+  FSIG_CUDA_TRY(cudaStreamSynchronize(e.stream));
   e.g = g;
   e.has_graph = true;
   return FSIG_OK;

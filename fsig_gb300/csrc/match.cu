@@ -32,6 +32,7 @@ struct GraphView {
   const uint32_t* __restrict__ old_of_new;
   const uint32_t* __restrict__ adj_old;  // null when lseg is
   const uint32_t* __restrict__ base;     // [L+1] first id of each label class
+  const uint16_t* __restrict__ filt;     // membership filter, or null
 };
 
 namespace {
@@ -39,7 +40,7 @@ namespace {
 constexpr uint32_t kFull = 0xffffffffu;
 
 GraphView view_of(const DeviceGraph& g) {
-  return GraphView{g.V, g.L, g.label, g.off, g.adj, g.lseg, g.sig, g.old_of_new, g.adj_old, g.base};
+  return GraphView{g.V, g.L, g.label, g.off, g.adj, g.lseg, g.sig, g.old_of_new, g.adj_old, g.base, g.filt};
 }
 
 // Segment [lo, hi) of row v's neighbours with label l (0 <= l < L), from the
@@ -770,28 +771,30 @@ struct EnumRun {
   unsigned long long* d_ev = nullptr;
   uint32_t* h_ctr = nullptr;  // pinned, 4 counters kCtrStride apart
   uint32_t grid = 0, block = 0, active = 0, first_task = 0, pass = 0;
-  uint32_t levels = 1;  // EnumArgs::levels
   size_t smem = 0;
   bool timed = true;  // every pass's kernel time was measured
 };
 
-// Kernel attributes and occupancy for a batch of this depth (host calls, kept
-// out of captures; remembered per block size and depth).
-int enum_configure(Engine& e, bool rows, uint32_t wpb, uint32_t levels) {
-  int& per_sm = (rows ? e.enum_per_sm_rows : e.enum_per_sm)[wpb][levels];
-  if (per_sm) return FSIG_OK;
-  const auto kernel = rows ? enumerate_kernel<true> : enumerate_kernel<false>;
-  FSIG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     int(warp_smem_bytes(kMaxQ - 1) * kEnumWarps)));
-  int per = 0;
-  FSIG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, int(wpb * 32),
-                                                              warp_smem_bytes(levels) * wpb));
-  per_sm = std::max(per, 1);
+// One-time kernel attributes and occupancy (host calls, kept out of captures).
+template <bool kRows>
+int enum_configure_one(int* per_sm) {
+  FSIG_CUDA_TRY(cudaFuncSetAttribute(enumerate_kernel<kRows>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     int(sizeof(WarpSmem) * kEnumWarps)));
+  for (uint32_t w = 1; w <= kEnumWarps; w++) {
+    int per = 0;
+    FSIG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, enumerate_kernel<kRows>, int(w * 32),
+                                                                sizeof(WarpSmem) * w));
+    per_sm[w] = std::max(per, 1);
+  }
   return FSIG_OK;
 }
 
-uint32_t warps_per_block(const BatchOptions& opt) {
-  return std::max<uint32_t>(1, std::min<uint32_t>(opt.warps_per_block, kEnumWarps));
+int enum_configure(Engine& e) {
+  if (e.enum_per_sm[kEnumWarps]) return FSIG_OK;
+  int rc = enum_configure_one<false>(e.enum_per_sm);
+  if (!rc) rc = enum_configure_one<true>(e.enum_per_sm_rows);
+  if (rc) e.enum_per_sm[kEnumWarps] = 0;
+  return rc;
 }
 
 int enum_prepare(Engine& e, const BatchOptions& opt, const GraphView& gv, const Plan* d_plans, const uint32_t* pool,
@@ -809,9 +812,9 @@ int enum_prepare(Engine& e, const BatchOptions& opt, const GraphView& gv, const 
     return fail(FSIG_EADMISSION, "work queues do not fit the device arena");
   FSIG_CUDA_TRY(cudaMemsetAsync(R.d_ev, 0, 64, s));
   FSIG_CUDA_TRY(cudaMemsetAsync(d_misc + 1, 0, sizeof(unsigned long long), s));
-  const uint32_t wpb = warps_per_block(opt);
-  const int per_sm = (gv.lseg ? e.enum_per_sm : e.enum_per_sm_rows)[wpb][R.levels];
-  R.smem = warp_smem_bytes(R.levels) * wpb;
+  const uint32_t wpb = std::max<uint32_t>(1, std::min<uint32_t>(opt.warps_per_block, kEnumWarps));
+  const int per_sm = gv.lseg ? e.enum_per_sm[wpb] : e.enum_per_sm_rows[wpb];
+  R.smem = sizeof(WarpSmem) * wpb;
   R.grid = uint32_t(e.num_sms * per_sm);
   R.block = wpb * 32;
   R.active = R.grid * wpb;  // every warp starts active; idle warps are counted as they wait
@@ -820,6 +823,8 @@ int enum_prepare(Engine& e, const BatchOptions& opt, const GraphView& gv, const 
   R.pass = 0;
   EnumArgs& A = R.A;
   A.g = gv;
+  // every buffer of the call is taken by now: the filter's room is still its own, or not
+  if (!e.arena.tail) A.g.filt = nullptr;
   A.plans = d_plans;
   A.pool = pool;
   A.Q = Q;
@@ -847,7 +852,6 @@ int enum_prepare(Engine& e, const BatchOptions& opt, const GraphView& gv, const 
   A.ready_wait_ns = e.ready_wait_ns;
   A.idle_wait_ns = e.idle_wait_ns;
   A.unpublished = e.inject_unpublished;
-  A.levels = R.levels;
   R.out = qa;
   R.ready = ra;
   R.other = qb;
@@ -973,8 +977,7 @@ int run_batch(Engine& e, const std::vector<HostQuery>& qs, const BatchOptions& o
   uint64_t d2h = 0;
   uint32_t launches = 0;
   EnumRun R;
-  for (const HostQuery& q : qs) R.levels = std::max(R.levels, q.n - 1);
-  int rc = enum_configure(e, g.lseg == nullptr, warps_per_block(opt), R.levels);
+  int rc = enum_configure(e);
   if (rc) return rc;
   if (opt.learned) {
     rc = mpnn_configure(e);

@@ -86,8 +86,7 @@ struct QueryResult {
 constexpr uint32_t kRefineCoopDefault = 32;
 
 // Enumeration launch shape: at most kEnumWarps warps per block, compiled for
-// kEnumMinBlocks resident blocks per SM (which caps registers per thread);
-// batches with queries of more than about 20 vertices have room for 3 blocks.
+// kEnumMinBlocks resident blocks per SM (which caps registers per thread).
 constexpr uint32_t kEnumWarps = 8;
 constexpr uint32_t kEnumMinBlocks = 4;
 

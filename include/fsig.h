@@ -153,7 +153,8 @@ int fsig_graph_info(const fsig_engine* e, uint32_t* num_vertices, uint64_t* num_
  * PCSR units are sized per label pair (graph_format_transformer.cc:39-215). */
 int fsig_set_segment_index(fsig_engine* e, int mode);
 /* The resident store's index (FSIG_SEGMENTS_TABLE or _ROWS) and its device
- * bytes (every array kept for matching). */
+ * bytes (every array kept for matching; not the membership filter, which lies
+ * in arena room that calls take back when they need it). */
 int fsig_graph_layout(const fsig_engine* e, int* segment_index, uint64_t* store_bytes);
 
 /* Binary cache of the resident graph store (the device arrays as built: the
