@@ -115,51 +115,102 @@ __global__ void scatter_kernel(const uint2* __restrict__ edges, uint64_t E, uint
 }
 
 // ---- segmented sort of rows ------------------------------------------------------
-constexpr uint32_t kWarpRow = 32, kBlockRow = 2048, kSmemRow = 16384;
+// A row of up to kWarpRow entries is sorted by a warp in registers, of up to
+// kBlockRow by a small block and of up to kSmemRow by a large one in shared
+// memory; longer ones in chunks of kSmemRow.  (A 256-thread block for every row
+// above 32 entries spent most of its time in barriers: 135,000 rows of 33 to
+// 2048 entries took 1.5 ms, and 0.2 ms with the warps.)
+constexpr uint32_t kWarpRow = 512, kBlockRow = 2048, kSmemRow = 16384;
 
+// Rows by class of length, and the longest length.  One atomic per warp and
+// class (one per row took 228 us for 2^20 rows, all on five words; this 52 us).
 __global__ void classify_rows_kernel(const uint32_t* __restrict__ off, uint32_t V, uint32_t* lists,
                                      uint32_t* counts, uint32_t* max_len) {
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
-    uint32_t len = off[v + 1] - off[v];
-    if (len > 0) atomicMax(max_len, len);
-    if (len <= 1) continue;
-    int c = len <= kWarpRow ? 0 : (len <= kBlockRow ? 1 : (len <= kSmemRow ? 2 : 3));
-    uint32_t p = atomicAdd(&counts[c], 1u);
-    lists[uint64_t(c) * V + p] = v;
+  const uint32_t lane = threadIdx.x & 31;
+  uint32_t longest = 0;
+  for (uint64_t base = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) & ~31ull; base < V;
+       base += uint64_t(gridDim.x) * blockDim.x) {
+    const uint32_t v = uint32_t(base) + lane;
+    const uint32_t len = v < V ? off[v + 1] - off[v] : 0;
+    longest = max(longest, len);
+    const int c = len <= 1 ? -1 : (len <= kWarpRow ? 0 : (len <= kBlockRow ? 1 : (len <= kSmemRow ? 2 : 3)));
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const uint32_t m = __ballot_sync(0xffffffffu, c == k);
+      if (!m) continue;
+      uint32_t first = 0;
+      if (lane == 0) first = atomicAdd(&counts[k], uint32_t(__popc(m)));
+      first = __shfl_sync(0xffffffffu, first, 0);
+      if (c == k) lists[uint64_t(k) * V + first + __popc(m & lanemask_lt())] = v;
+    }
   }
+  longest = __reduce_max_sync(0xffffffffu, longest);
+  if (lane == 0 && longest) atomicMax(max_len, longest);
 }
 
-__global__ void sort_rows_warp_kernel(const uint32_t* __restrict__ rows, const uint32_t* __restrict__ count,
-                                      const uint32_t* __restrict__ off, uint32_t* adj) {
+// Bitonic sort of the up to 32 R entries at p by one warp: entry r * 32 + lane
+// in register r of the lane.
+template <int R>
+__device__ __forceinline__ void warp_sort_row(uint32_t* p, uint32_t len, uint32_t lane) {
+  uint32_t x[R];
+#pragma unroll
+  for (int r = 0; r < R; r++) x[r] = r * 32 + lane < len ? p[r * 32 + lane] : kInvalid;
+#pragma unroll
+  for (int k = 2; k <= 32 * R; k <<= 1) {
+#pragma unroll
+    for (int j = k >> 1; j >= 32; j >>= 1) {
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        const int o = r ^ (j >> 5);
+        if (o > r) {
+          const uint32_t lo = min(x[r], x[o]), hi = max(x[r], x[o]);
+          const bool up = ((r * 32) & k) == 0;
+          x[r] = up ? lo : hi;
+          x[o] = up ? hi : lo;
+        }
+      }
+    }
+#pragma unroll
+    for (int j = k >> 1 < 16 ? k >> 1 : 16; j > 0; j >>= 1) {
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        const uint32_t y = __shfl_xor_sync(0xffffffffu, x[r], j);
+        const bool up = ((r * 32 + lane) & k) == 0, lower = (lane & j) == 0;
+        x[r] = lower == up ? min(x[r], y) : max(x[r], y);
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < R; r++)
+    if (r * 32 + lane < len) p[r * 32 + lane] = x[r];
+}
+
+__global__ void __launch_bounds__(256) sort_rows_warp_kernel(const uint32_t* __restrict__ rows,
+                                                             const uint32_t* __restrict__ count,
+                                                             const uint32_t* __restrict__ off, uint32_t* adj) {
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t n = *count;
   for (uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n; r += (gridDim.x * blockDim.x) >> 5) {
-    uint32_t v = rows[r];
-    uint32_t b = off[v], len = off[v + 1] - b;
-    uint32_t x = lane < len ? adj[b + lane] : kInvalid;
-#pragma unroll
-    for (int k = 2; k <= 32; k <<= 1) {
-#pragma unroll
-      for (int j = k >> 1; j > 0; j >>= 1) {
-        uint32_t y = __shfl_xor_sync(0xffffffffu, x, j);
-        bool up = (lane & k) == 0;
-        bool lower = (lane & j) == 0;
-        x = (lower == up) ? min(x, y) : max(x, y);
-      }
-    }
-    if (lane < len) adj[b + lane] = x;
+    const uint32_t v = rows[r], b = off[v], len = off[v + 1] - b;
+    if (len <= 32) warp_sort_row<1>(adj + b, len, lane);
+    else if (len <= 64) warp_sort_row<2>(adj + b, len, lane);
+    else if (len <= 128) warp_sort_row<4>(adj + b, len, lane);
+    else if (len <= 256) warp_sort_row<8>(adj + b, len, lane);
+    else warp_sort_row<16>(adj + b, len, lane);
   }
 }
 
+// n a power of two; every thread has a pair to compare.
 __device__ void block_bitonic(uint32_t* s, uint32_t n) {
   for (uint32_t k = 2; k <= n; k <<= 1) {
     for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-      for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-        uint32_t p = i ^ j;
-        if (p > i) {
-          uint32_t a = s[i], b = s[p];
-          bool up = (i & k) == 0;
-          if ((a > b) == up) { s[i] = b; s[p] = a; }
+      for (uint32_t t = threadIdx.x; t < n >> 1; t += blockDim.x) {
+        const uint32_t i = 2 * t - (t & (j - 1)), p = i + j;
+        const uint32_t a = s[i], b = s[p];
+        const bool up = (i & k) == 0;
+        if ((a > b) == up) {
+          s[i] = b;
+          s[p] = a;
         }
       }
       __syncthreads();
@@ -167,10 +218,9 @@ __device__ void block_bitonic(uint32_t* s, uint32_t n) {
   }
 }
 
-// One block per row; rows of class c are sorted in shared memory (padded to a
-// power of two) or, for the longest rows, in a global scratch buffer.
+// One block per row; the row is sorted in shared memory, padded to a power of two.
 __global__ void sort_rows_block_kernel(const uint32_t* __restrict__ rows, const uint32_t* __restrict__ count,
-                                       const uint32_t* __restrict__ off, uint32_t* adj, uint32_t* gscratch) {
+                                       const uint32_t* __restrict__ off, uint32_t* adj) {
   extern __shared__ uint32_t sm[];
   const uint32_t n = *count;
   for (uint32_t r = blockIdx.x; r < n; r += gridDim.x) {
@@ -178,38 +228,136 @@ __global__ void sort_rows_block_kernel(const uint32_t* __restrict__ rows, const 
     uint32_t b = off[v], len = off[v + 1] - b;
     uint32_t p2 = 1;
     while (p2 < len) p2 <<= 1;
-    uint32_t* s = gscratch ? gscratch + uint64_t(blockIdx.x) * 0 : sm;
-    if (gscratch) s = gscratch;  // a single block handles the global class
-    for (uint32_t i = threadIdx.x; i < p2; i += blockDim.x) s[i] = i < len ? adj[b + i] : kInvalid;
+    for (uint32_t i = threadIdx.x; i < p2; i += blockDim.x) sm[i] = i < len ? adj[b + i] : kInvalid;
     __syncthreads();
-    block_bitonic(s, p2);
-    for (uint32_t i = threadIdx.x; i < len; i += blockDim.x) adj[b + i] = s[i];
+    block_bitonic(sm, p2);
+    for (uint32_t i = threadIdx.x; i < len; i += blockDim.x) adj[b + i] = sm[i];
     __syncthreads();
   }
 }
 
-// Unique entries per sorted row.
+// Rows longer than kSmemRow, in chunks of kSmemRow entries: the chunks are
+// sorted in shared memory, then merged pairwise, an entry's place being its own
+// index plus its rank in the sibling run by binary search (equal entries: the
+// left run's first).  Every entry of every pass is independent, so the longest
+// row no longer runs on one block: the 21 rows above 16384 entries of a 2^24-
+// edge R-MAT graph took 15 ms by one block's bitonic sort in global memory, and
+// 0.27 ms this way.
+__global__ void long_chunks_kernel(const uint32_t* __restrict__ rows, uint32_t n, const uint32_t* __restrict__ off,
+                                   uint32_t* chunks) {
+  for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x)
+    chunks[r] = (off[rows[r] + 1] - off[rows[r]] + kSmemRow - 1) / kSmemRow;
+}
+
+// Row (its first entry, length) and first entry within it of chunk c.
+__device__ __forceinline__ void chunk_of(const uint32_t* __restrict__ rows, uint32_t n,
+                                         const uint32_t* __restrict__ chunk_off, const uint32_t* __restrict__ off,
+                                         uint32_t c, uint32_t& b, uint32_t& len, uint32_t& first) {
+  uint32_t lo = 0, hi = n;  // last row with chunk_off <= c
+  while (hi - lo > 1) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (chunk_off[mid] <= c) lo = mid; else hi = mid;
+  }
+  b = off[rows[lo]];
+  len = off[rows[lo] + 1] - b;
+  first = (c - chunk_off[lo]) * kSmemRow;
+}
+
+__global__ void __launch_bounds__(1024) sort_chunks_kernel(const uint32_t* __restrict__ rows, uint32_t n,
+                                                           const uint32_t* __restrict__ chunk_off, uint32_t total,
+                                                           const uint32_t* __restrict__ off, uint32_t* adj) {
+  extern __shared__ uint32_t sm[];
+  for (uint32_t c = blockIdx.x; c < total; c += gridDim.x) {
+    uint32_t b, len, first;
+    chunk_of(rows, n, chunk_off, off, c, b, len, first);
+    const uint32_t m = min(kSmemRow, len - first);
+    uint32_t p2 = 1;
+    while (p2 < m) p2 <<= 1;
+    for (uint32_t i = threadIdx.x; i < p2; i += blockDim.x) sm[i] = i < m ? adj[b + first + i] : kInvalid;
+    __syncthreads();
+    block_bitonic(sm, p2);
+    for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) adj[b + first + i] = sm[i];
+    __syncthreads();
+  }
+}
+
+// One merge pass over runs of `width` entries (a power of two); width 0 copies.
+__global__ void __launch_bounds__(1024) merge_runs_kernel(const uint32_t* __restrict__ rows, uint32_t n,
+                                                          const uint32_t* __restrict__ chunk_off, uint32_t total,
+                                                          const uint32_t* __restrict__ off, uint64_t width,
+                                                          const uint32_t* __restrict__ in, uint32_t* __restrict__ out) {
+  for (uint32_t c = blockIdx.x; c < total; c += gridDim.x) {
+    uint32_t b, len, first;
+    chunk_of(rows, n, chunk_off, off, c, b, len, first);
+    const uint32_t last = first + min(kSmemRow, len - first);
+    uint64_t run = 0, lo = len, hi = len;  // the chunk lies in one run; its sibling is [lo, hi)
+    if (width) {
+      run = first / width;
+      lo = min((run ^ 1) * width, uint64_t(len));
+      hi = min(lo + width, uint64_t(len));
+    }
+    for (uint32_t i = first + threadIdx.x; i < last; i += blockDim.x) {
+      const uint32_t x = in[b + i];
+      uint32_t to = i;
+      if (lo < hi) {
+        // entries of the sibling that go first: the smaller ones, and from a left sibling the equal ones
+        const bool right = run & 1;
+        uint32_t l = uint32_t(lo), h = uint32_t(hi);
+        while (l < h) {
+          const uint32_t mid = (l + h) >> 1;
+          const uint32_t y = in[b + mid];
+          if (y < x || (right && y == x)) l = mid + 1; else h = mid;
+        }
+        to = (right ? i - uint32_t(width) : i) + (l - uint32_t(lo));
+      }
+      out[b + to] = x;
+    }
+  }
+}
+
+// Repeated entries of all sorted rows: equal neighbours in the adjacency, less
+// the pairs that straddle two rows.  Most graphs have none, and then nothing of
+// the two kernels below runs (a thread walking each row took 1.7 ms on a 2^24-
+// edge R-MAT graph, hubs last; this 0.06 ms).
+__global__ void repeats_kernel(const uint32_t* __restrict__ off, const uint32_t* __restrict__ adj, uint32_t V,
+                               uint64_t n, unsigned long long* repeats) {
+  long long c = 0;
+  const uint64_t t0 = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x, step = uint64_t(gridDim.x) * blockDim.x;
+  for (uint64_t k = t0 + 1; k < n; k += step) c += adj[k] == adj[k - 1];
+  for (uint64_t v = t0; v < V; v += step) {
+    const uint32_t b = off[v];
+    if (b > 0 && b < off[v + 1]) c -= adj[b] == adj[b - 1];
+  }
+  c = warp_sum(c);
+  if ((threadIdx.x & 31) == 0 && c) atomicAdd(repeats, (unsigned long long)c);
+}
+
+// Unique entries per sorted row, a warp per row.
 __global__ void unique_count_kernel(const uint32_t* __restrict__ off, const uint32_t* __restrict__ adj, uint32_t V,
                                     uint32_t* ucount) {
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
-    uint32_t b = off[v], e = off[v + 1], c = 0, prev = kInvalid;
-    for (uint32_t i = b; i < e; i++) {
-      uint32_t x = adj[i];
-      c += x != prev;
-      prev = x;
-    }
-    ucount[v] = c;
+  const uint32_t lane = threadIdx.x & 31;
+  for (uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < V; v += (gridDim.x * blockDim.x) >> 5) {
+    const uint32_t b = off[v], e = off[v + 1];
+    uint32_t c = 0;
+    for (uint32_t i = b + lane; i < e; i += 32) c += i == b || adj[i] != adj[i - 1];
+    c = __reduce_add_sync(0xffffffffu, c);
+    if (lane == 0) ucount[v] = c;
   }
 }
 
 __global__ void unique_copy_kernel(const uint32_t* __restrict__ off, const uint32_t* __restrict__ adj, uint32_t V,
                                    const uint32_t* __restrict__ noff, uint32_t* out) {
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
-    uint32_t b = off[v], e = off[v + 1], w = noff[v], prev = kInvalid;
-    for (uint32_t i = b; i < e; i++) {
-      uint32_t x = adj[i];
-      if (x != prev) out[w++] = x;
-      prev = x;
+  const uint32_t lane = threadIdx.x & 31;
+  for (uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < V; v += (gridDim.x * blockDim.x) >> 5) {
+    const uint32_t b = off[v], e = off[v + 1];
+    uint32_t w = noff[v];
+    for (uint32_t i0 = b; i0 < e; i0 += 32) {
+      const uint32_t i = i0 + lane;
+      const uint32_t x = i < e ? adj[i] : 0;
+      const bool keep = i < e && (i == b || x != adj[i - 1]);
+      const uint32_t m = __ballot_sync(0xffffffffu, keep);
+      if (keep) out[w + __popc(m & lanemask_lt())] = x;
+      w += __popc(m);
     }
   }
 }
@@ -262,30 +410,32 @@ __global__ void signature_from_segments_kernel(const int32_t* __restrict__ label
 
 // Reference-layout signature: one saturating increment per adjacency entry
 // (duplicates counted as the reference counts them).
-__global__ void signature_from_rows_kernel(const int32_t* __restrict__ label, const uint32_t* __restrict__ off,
-                                           const uint32_t* __restrict__ adj, uint32_t V, int column_oriented,
-                                           uint32_t* out) {
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
-    uint32_t w[kSigWords];
-#pragma unroll
-    for (int i = 0; i < kSigWords; i++) w[i] = 0;
-    w[0] = uint32_t(label[v]);
-    for (uint32_t e = off[v]; e < off[v + 1]; e++) {
+// A warp per row, its counters in shared memory: a neighbour's first increment
+// sets the counter's low bit, every later one its high bit, whatever the order.
+// (A thread per row walked hubs alone: 514 us for 320k rows of up to 1478
+// entries, now 64 us.)
+__global__ void __launch_bounds__(256) signature_from_rows_kernel(const int32_t* __restrict__ label,
+                                                                  const uint32_t* __restrict__ off,
+                                                                  const uint32_t* __restrict__ adj, uint32_t V,
+                                                                  int column_oriented, uint32_t* out) {
+  __shared__ uint32_t words[8][kSigWords];
+  const uint32_t lane = threadIdx.x & 31;
+  uint32_t* w = words[threadIdx.x >> 5];
+  for (uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < V; v += (gridDim.x * blockDim.x) >> 5) {
+    if (lane < kSigWords) w[lane] = lane == 0 ? uint32_t(label[v]) : 0u;
+    __syncwarp();
+    const uint32_t end = off[v + 1];
+    for (uint32_t e = off[v] + lane; e < end; e += 32) {
       uint32_t word, sh;
       sig_slot(label[adj[e]], word, sh);
-#pragma unroll
-      for (int i = 1; i < kSigWords; i++) {
-        if (uint32_t(i) == word) {
-          uint32_t cur = (w[i] >> sh) & 3u;
-          w[i] |= (cur == 0 ? 1u : 3u) << sh;
-        }
-      }
+      if ((atomicOr(&w[word], 1u << sh) >> sh) & 1u) atomicOr(&w[word], 2u << sh);
     }
-#pragma unroll
-    for (int i = 0; i < kSigWords; i++) {
-      if (column_oriented) out[uint64_t(i) * V + v] = w[i];
-      else out[uint64_t(v) * kSigWords + i] = w[i];
+    __syncwarp();
+    if (lane < kSigWords) {
+      if (column_oriented) out[uint64_t(lane) * V + v] = w[lane];
+      else out[uint64_t(v) * kSigWords + lane] = w[lane];
     }
+    __syncwarp();
   }
 }
 
@@ -350,9 +500,10 @@ inline unsigned grid_for(uint64_t n, int threads, int sms) {
 }
 
 // Builds offsets/adjacency (rows sorted) from an edge list already on the
-// device.  map == nullptr keeps caller ids.  Returns the row data in adj.
-int build_rows(Engine& e, const uint2* d_edges, uint64_t E, uint32_t V, const uint32_t* map, bool drop_loops,
-               uint32_t* off, uint32_t* adj, uint32_t* d_flags) {
+// device.  map == nullptr keeps caller ids.  Returns the row data in adj and
+// the longest row's length; the edge list's memory serves as scratch.
+int build_rows(Engine& e, uint2* d_edges, uint64_t E, uint32_t V, const uint32_t* map, bool drop_loops, uint32_t* off,
+               uint32_t* adj, uint32_t* d_flags, uint32_t* longest = nullptr) {
   cudaStream_t s = e.stream;
   uint64_t m = e.arena.mark();
   uint32_t* deg = e.arena.take<uint32_t>(uint64_t(V) + 1);
@@ -380,26 +531,51 @@ int build_rows(Engine& e, const uint2* d_edges, uint64_t E, uint32_t V, const ui
   }
   if (h[1]) {
     sort_rows_block_kernel<<<std::min<uint32_t>(h[1], e.num_sms * 8), 256, kBlockRow * 4, s>>>(
-        lists + uint64_t(V), small + 1, off, adj, nullptr);
+        lists + uint64_t(V), small + 1, off, adj);
     FSIG_CUDA_TRY(cudaGetLastError());
   }
   if (h[2]) {
     FSIG_CUDA_TRY(cudaFuncSetAttribute(sort_rows_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        kSmemRow * 4));
     sort_rows_block_kernel<<<std::min<uint32_t>(h[2], e.num_sms * 2), 1024, kSmemRow * 4, s>>>(
-        lists + 2 * uint64_t(V), small + 2, off, adj, nullptr);
+        lists + 2 * uint64_t(V), small + 2, off, adj);
     FSIG_CUDA_TRY(cudaGetLastError());
   }
   if (h[3]) {
-    uint32_t p2 = 1;
-    while (p2 < h[4]) p2 <<= 1;
-    uint32_t* gs = e.arena.take<uint32_t>(p2);
-    if (!gs) return fail(FSIG_EADMISSION, "row sort scratch does not fit the arena");
-    sort_rows_block_kernel<<<1, 1024, 0, s>>>(lists + 3 * uint64_t(V), small + 3, off, adj, gs);
+    // chunk counts of the long rows and their prefix sums, over the shorter classes' lists
+    const uint32_t* rows = lists + 3 * uint64_t(V);
+    uint32_t *chunks = deg, *chunk_off = deg;  // deg held the scatter's cursors: done with
+    long_chunks_kernel<<<grid_for(h[3], T, e.num_sms), T, 0, s>>>(rows, h[3], off, chunks);
     FSIG_CUDA_TRY(cudaGetLastError());
+    rc = device_exclusive_scan<uint32_t>(e.arena, chunks, chunk_off, h[3], small + 5, s);
+    if (rc) return rc;
+    uint32_t total = 0;
+    FSIG_CUDA_TRY(cudaMemcpyAsync(&total, small + 5, sizeof(total), cudaMemcpyDeviceToHost, s));
+    FSIG_CUDA_TRY(cudaStreamSynchronize(s));
+    FSIG_CUDA_TRY(cudaFuncSetAttribute(sort_chunks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemRow * 4));
+    sort_chunks_kernel<<<std::min<uint32_t>(total, e.num_sms * 2), 1024, kSmemRow * 4, s>>>(rows, h[3], chunk_off, total,
+                                                                                          off, adj);
+    FSIG_CUDA_TRY(cudaGetLastError());
+    // the edge list (2E words) is scattered by now: its memory is the other buffer
+    uint32_t *in = adj, *out = reinterpret_cast<uint32_t*>(d_edges);
+    const unsigned grid = std::min<uint32_t>(total, e.num_sms * 2);
+    for (uint64_t width = kSmemRow; width < h[4] || in != adj; width <<= 1) {
+      merge_runs_kernel<<<grid, 1024, 0, s>>>(rows, h[3], chunk_off, total, off, width < h[4] ? width : 0, in, out);
+      FSIG_CUDA_TRY(cudaGetLastError());
+      std::swap(in, out);
+    }
   }
+  if (longest) *longest = h[4];
   e.arena.release(m);
   return FSIG_OK;
+}
+
+__global__ void max_row_kernel(const uint32_t* __restrict__ off, uint32_t V, uint32_t* longest) {
+  uint32_t m = 0;
+  for (uint64_t v = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; v < V; v += uint64_t(gridDim.x) * blockDim.x)
+    m = max(m, off[v + 1] - off[v]);
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0 && m) atomicMax(longest, m);
 }
 
 // Arena bytes left free beside the membership filter when it is built: a
@@ -494,30 +670,40 @@ int build_device_graph(Engine& e, uint32_t V, const int32_t* h_labels, uint64_t 
   FSIG_CUDA_TRY(cudaMemcpyAsync(g.h_base.data(), base_tmp, sizeof(uint32_t) * (L + 1), cudaMemcpyDeviceToHost, s));
 
   // Rows in new-id space, self-loops dropped, then duplicates removed.
-  rc = build_rows(e, d_edges, E, V, g.new_of_old, true, g.off, g.adj, flags);
+  rc = build_rows(e, d_edges, E, V, g.new_of_old, true, g.off, g.adj, flags, &g.max_deg);
   if (rc) return rc;
   uint32_t* ucount = e.arena.take<uint32_t>(uint64_t(V) + 1);
   uint32_t* noff = e.arena.take<uint32_t>(uint64_t(V) + 1);
-  uint32_t* totals = e.arena.take<uint32_t>(2);
+  unsigned long long* totals = e.arena.take<unsigned long long>(2);
   if (!ucount || !noff || !totals) return fail(FSIG_EADMISSION, "arena");
-  FSIG_CUDA_TRY(cudaMemsetAsync(ucount, 0, sizeof(uint32_t) * (uint64_t(V) + 1), s));
-  unique_count_kernel<<<grid_for(V, 256, e.num_sms), 256, 0, s>>>(g.off, g.adj, V, ucount);
-  FSIG_CUDA_TRY(cudaGetLastError());
-  rc = device_exclusive_scan<uint32_t>(e.arena, ucount, noff, uint64_t(V) + 1, totals, s);
-  if (rc) return rc;
-  uint32_t h_tot[2] = {0, 0};
-  FSIG_CUDA_TRY(cudaMemcpyAsync(h_tot, totals, 4, cudaMemcpyDeviceToHost, s));
+  uint32_t h_tot[2] = {0, 0};  // entries without and with repeats
+  unsigned long long repeats = 0;
   FSIG_CUDA_TRY(cudaMemcpyAsync(h_tot + 1, g.off + V, 4, cudaMemcpyDeviceToHost, s));
   FSIG_CUDA_TRY(cudaMemcpyAsync(hf, flags, 4, cudaMemcpyDeviceToHost, s));
   FSIG_CUDA_TRY(cudaStreamSynchronize(s));
   if (hf[0] & 2u) return fail(FSIG_EINVAL, "edge endpoint out of range");
-  if (h_tot[0] != h_tot[1]) {
+  FSIG_CUDA_TRY(cudaMemsetAsync(totals, 0, 16, s));
+  repeats_kernel<<<grid_for(std::max<uint64_t>(h_tot[1], V), 256, e.num_sms), 256, 0, s>>>(g.off, g.adj, V, h_tot[1],
+                                                                                          totals);
+  FSIG_CUDA_TRY(cudaGetLastError());
+  FSIG_CUDA_TRY(cudaMemcpyAsync(&repeats, totals, 8, cudaMemcpyDeviceToHost, s));
+  FSIG_CUDA_TRY(cudaStreamSynchronize(s));
+  h_tot[0] = h_tot[1] - uint32_t(repeats);
+  if (repeats) {
+    FSIG_CUDA_TRY(cudaMemsetAsync(ucount, 0, sizeof(uint32_t) * (uint64_t(V) + 1), s));
+    unique_count_kernel<<<grid_for(uint64_t(V) * 32, 256, e.num_sms), 256, 0, s>>>(g.off, g.adj, V, ucount);
+    FSIG_CUDA_TRY(cudaGetLastError());
+    rc = device_exclusive_scan<uint32_t>(e.arena, ucount, noff, uint64_t(V) + 1, nullptr, s);
+    if (rc) return rc;
     uint32_t* tmp = e.arena.take<uint32_t>(std::max<uint32_t>(h_tot[0], 1));
     if (!tmp) return fail(FSIG_EADMISSION, "arena");
-    unique_copy_kernel<<<grid_for(V, 256, e.num_sms), 256, 0, s>>>(g.off, g.adj, V, noff, tmp);
+    unique_copy_kernel<<<grid_for(uint64_t(V) * 32, 256, e.num_sms), 256, 0, s>>>(g.off, g.adj, V, noff, tmp);
     FSIG_CUDA_TRY(cudaGetLastError());
     FSIG_CUDA_TRY(cudaMemcpyAsync(g.adj, tmp, sizeof(uint32_t) * h_tot[0], cudaMemcpyDeviceToDevice, s));
     FSIG_CUDA_TRY(cudaMemcpyAsync(g.off, noff, sizeof(uint32_t) * (uint64_t(V) + 1), cudaMemcpyDeviceToDevice, s));
+    max_row_kernel<<<grid_for(V, 256, e.num_sms), 256, 0, s>>>(g.off, V, reinterpret_cast<uint32_t*>(totals + 1));
+    FSIG_CUDA_TRY(cudaGetLastError());
+    FSIG_CUDA_TRY(cudaMemcpyAsync(&g.max_deg, totals + 1, 4, cudaMemcpyDeviceToHost, s));
   }
   g.nadj = h_tot[0];
   FSIG_CUDA_TRY(cudaStreamSynchronize(s));
@@ -546,29 +732,14 @@ int build_device_graph(Engine& e, uint32_t V, const int32_t* h_labels, uint64_t 
   } else {
     // one saturating increment per neighbour (rows have no duplicates) gives
     // every label segment's min(count, 2) increments
-    signature_from_rows_kernel<<<grid_for(V, 128, e.num_sms), 128, 0, s>>>(g.label, g.off, g.adj, V, 0,
+    signature_from_rows_kernel<<<grid_for(uint64_t(V) * 32, 256, e.num_sms), 256, 0, s>>>(g.label, g.off, g.adj, V, 0,
                                                                            reinterpret_cast<uint32_t*>(g.sig));
   }
   FSIG_CUDA_TRY(cudaGetLastError());
-  // Maximum degree.
-  uint32_t* mx = e.arena.take<uint32_t>(1);
-  if (!mx) return fail(FSIG_EADMISSION, "arena");
-  FSIG_CUDA_TRY(cudaMemsetAsync(mx, 0, 4, s));
-  {
-    uint64_t mm = e.arena.mark();
-    uint32_t* lists = e.arena.take<uint32_t>(uint64_t(V) * 4);
-    uint32_t* small = e.arena.take<uint32_t>(8);
-    if (!lists || !small) return fail(FSIG_EADMISSION, "arena");
-    FSIG_CUDA_TRY(cudaMemsetAsync(small, 0, 32, s));
-    classify_rows_kernel<<<grid_for(V, 256, e.num_sms), 256, 0, s>>>(g.off, V, lists, small, mx);
-    FSIG_CUDA_TRY(cudaGetLastError());
-    FSIG_CUDA_TRY(cudaMemcpyAsync(&g.max_deg, mx, 4, cudaMemcpyDeviceToHost, s));
-    FSIG_CUDA_TRY(cudaStreamSynchronize(s));
-    e.arena.release(mm);
-  }
   g.arena_mark = e.arena.mark();
   rc = build_membership_filter(e, g);
   if (rc) return rc;
+  FSIG_CUDA_TRY(cudaStreamSynchronize(s));
   e.g = g;
   e.has_graph = true;
   return FSIG_OK;
@@ -738,7 +909,7 @@ int build_reference_signature(Engine& e, uint32_t V, const int32_t* h_labels, co
   FSIG_CUDA_TRY(cudaMemcpyAsync(lab, h_labels, sizeof(int32_t) * V, cudaMemcpyHostToDevice, s));
   FSIG_CUDA_TRY(cudaMemcpyAsync(off, h_off, sizeof(uint32_t) * (uint64_t(V) + 1), cudaMemcpyHostToDevice, s));
   if (nadj) FSIG_CUDA_TRY(cudaMemcpyAsync(adj, h_adj, sizeof(uint32_t) * nadj, cudaMemcpyHostToDevice, s));
-  signature_from_rows_kernel<<<grid_for(V, 128, e.num_sms), 128, 0, s>>>(lab, off, adj, V, column_oriented, sig);
+  signature_from_rows_kernel<<<grid_for(uint64_t(V) * 32, 256, e.num_sms), 256, 0, s>>>(lab, off, adj, V, column_oriented, sig);
   FSIG_CUDA_TRY(cudaGetLastError());
   FSIG_CUDA_TRY(cudaMemcpyAsync(h_sig, sig, sizeof(uint32_t) * kSigWords * V, cudaMemcpyDeviceToHost, s));
   FSIG_CUDA_TRY(cudaStreamSynchronize(s));
