@@ -1,7 +1,9 @@
 // Order-scoring network kernels: features, forward, backward, weight
 // gradients and Adam, all hand-written; matrix products on the tensor cores
-// with mma.sync m16n8k16 (BF16 operands, FP32 accumulation), one warp per
-// query graph (at most 32 vertices = two 16-row tiles).
+// with mma.sync m16n8k16 (BF16 operands, FP32 accumulation), four warps per
+// query graph (at most 32 vertices = two 16-row tiles), each warp 16 of the 64
+// output columns.  (The products are 32 x 64 x 64: far below a tcgen05 tile of
+// 128 rows.)
 //
 //   h0 = relu(x W_in + b_in)                        x: 8 features, padded to 16
 //   h_{l+1} = relu(h_l W_s[l] + (D^-1 A h_l) W_n[l] + b[l]),  l = 0, 1, 2
@@ -13,6 +15,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "match.h"
@@ -21,282 +24,325 @@
 namespace fsig {
 namespace {
 
-constexpr int kWarpsPerBlock = 2;
 constexpr int kWBf = kPB;  // BF16 weight copy covers [0, kPB): W_in, b_in (unused), W_s, W_n
+constexpr int kGraphThreads = 128;  // threads of one graph
+constexpr int kGraphsPerBlock = 2;  // graphs at a time, sharing the block's weights
+// Row strides in shared memory, padded so that the 8 rows of an ldmatrix (or of
+// a fragment's epilogue) fall into different banks.
+constexpr int kLd = kHid + 8, kLdX = kFeatPad + 8, kLdF = kHid + 8;
 
 __device__ __forceinline__ uint16_t f2bf(float x) { return __bfloat16_as_ushort(__float2bfloat16_rn(x)); }
 __device__ __forceinline__ float bf2f(uint16_t x) { return __bfloat162float(__ushort_as_bfloat16(x)); }
-__device__ __forceinline__ uint32_t pack2(uint16_t lo, uint16_t hi) { return uint32_t(lo) | (uint32_t(hi) << 16); }
 
-__device__ __forceinline__ void mma_bf16(float c[4], const uint32_t a[4], const uint32_t b[2]) {
+__device__ __forceinline__ void mma_bf16(float c[4], const uint32_t a[4], uint32_t b0, uint32_t b1) {
   asm volatile(
       "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
       "{%0,%1,%2,%3};"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// acc (C[32][64], fragment layout of m16n8k16) += sum_k A(r, k) B(k, n).
-// A and B return BF16 bit patterns; K is a multiple of 16.
-template <class FA, class FB>
-__device__ __forceinline__ void warp_gemm(int K, FA A, FB B, float acc[2][8][4]) {
-  const int lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
+// Four 8 x 8 BF16 matrices; lane l gives the address of row l % 8 of matrix l / 8.
+template <bool kTrans>
+__device__ __forceinline__ void ldmatrix4(uint32_t r[4], const uint16_t* p) {
+  const uint32_t a = uint32_t(__cvta_generic_to_shared(p));
+  if constexpr (kTrans)
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+  else
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+}
+
+// acc (rows 0..31, columns n0..n0+15 of C, m16n8k16 fragments) += A B, with A
+// [32][K] at row stride lda, and B [K][64] (kTransB: [64][K], i.e. B^T) at row
+// stride kLd.  K ascending in steps of 16.
+template <int K, bool kTransB>
+__device__ __forceinline__ void gemm_cols(const uint16_t* A, int lda, const uint16_t* B, int n0, float acc[2][2][4]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
   for (int kk = 0; kk < K; kk += 16) {
-    const int k0 = kk + 2 * c;
-    uint32_t a[2][4];
+    uint32_t a[2][4], b[4];
 #pragma unroll
-    for (int mt = 0; mt < 2; mt++) {
-      const int r0 = mt * 16 + g, r1 = r0 + 8;
-      a[mt][0] = pack2(A(r0, k0), A(r0, k0 + 1));
-      a[mt][1] = pack2(A(r1, k0), A(r1, k0 + 1));
-      a[mt][2] = pack2(A(r0, k0 + 8), A(r0, k0 + 9));
-      a[mt][3] = pack2(A(r1, k0 + 8), A(r1, k0 + 9));
-    }
+    for (int mt = 0; mt < 2; mt++) ldmatrix4<false>(a[mt], A + (mt * 16 + (lane & 15)) * lda + kk + (lane >> 4) * 8);
+    if constexpr (kTransB)
+      ldmatrix4<false>(b, B + (n0 + (lane & 7) + (lane >> 4) * 8) * kLd + kk + ((lane >> 3) & 1) * 8);
+    else
+      ldmatrix4<true>(b, B + (kk + (lane & 15)) * kLd + n0 + (lane >> 4) * 8);
 #pragma unroll
-    for (int nt = 0; nt < 8; nt++) {
-      const int n = nt * 8 + g;
-      const uint32_t b[2] = {pack2(B(k0, n), B(k0 + 1, n)), pack2(B(k0 + 8, n), B(k0 + 9, n))};
-      mma_bf16(acc[0][nt], a[0], b);
-      mma_bf16(acc[1][nt], a[1], b);
+    for (int nt = 0; nt < 2; nt++) {
+      mma_bf16(acc[0][nt], a[0], b[2 * nt], b[2 * nt + 1]);
+      mma_bf16(acc[1][nt], a[1], b[2 * nt], b[2 * nt + 1]);
     }
   }
 }
 
-__device__ __forceinline__ void zero_acc(float acc[2][8][4]) {
+__device__ __forceinline__ void zero_acc(float acc[2][2][4]) {
 #pragma unroll
   for (int i = 0; i < 2; i++)
 #pragma unroll
-    for (int j = 0; j < 8; j++)
+    for (int j = 0; j < 2; j++)
 #pragma unroll
       for (int k = 0; k < 4; k++) acc[i][j][k] = 0.f;
 }
 
-// Visits every accumulator element as (row, col, value&).
+// Visits every accumulator element as (row, col, value).
 template <class F>
-__device__ __forceinline__ void for_acc(float acc[2][8][4], F f) {
+__device__ __forceinline__ void for_acc(float acc[2][2][4], int n0, F f) {
   const int lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
 #pragma unroll
   for (int mt = 0; mt < 2; mt++)
 #pragma unroll
-    for (int nt = 0; nt < 8; nt++)
+    for (int nt = 0; nt < 2; nt++)
 #pragma unroll
-      for (int j = 0; j < 4; j++) f(mt * 16 + g + (j >= 2 ? 8 : 0), nt * 8 + 2 * c + (j & 1), acc[mt][nt][j]);
+      for (int j = 0; j < 4; j++)
+        f(mt * 16 + g + (j >= 2 ? 8 : 0), n0 + nt * 8 + 2 * c + (j & 1), acc[mt][nt][j]);
 }
 
 struct BlockW {
-  uint16_t win[kFeatPad * kHid];
-  uint16_t ws[kLayers][kHid * kHid];
-  uint16_t wn[kLayers][kHid * kHid];
+  uint16_t win[kFeatPad * kLd];
+  uint16_t ws[kLayers][kHid * kLd];
+  uint16_t wn[kLayers][kHid * kLd];
 };
 
-struct WarpBuf {
-  uint16_t x[32 * kFeatPad];
-  uint16_t h[kLayers + 1][32 * kHid];
-  uint16_t m[kLayers][32 * kHid];
-  uint16_t dz[32 * kHid];
-  float dh[32 * kHid];
-  float q[32 * kHid];
+struct GraphBuf {
+  uint16_t x[32 * kLdX];
+  uint16_t h[kLayers + 1][32 * kLd];
+  uint16_t m[kLayers][32 * kLd];
   uint32_t nbr[32];
   float invdeg[32];
+};
+
+struct GraphBufTrain : GraphBuf {
+  uint16_t dz[32 * kLd];
+  float dh[32 * kLdF];
+  float q[32 * kLdF];
+  float ds[32];
 };
 
 // Per-node record of what the weight-gradient kernel needs (BF16).
 constexpr int kActX = 0, kActH = kFeatPad, kActM = kActH + kLayers * kHid, kActDz = kActM + kLayers * kHid,
               kActW = kActDz + (kLayers + 1) * kHid;
+static_assert(kActW % 8 == 0 && kActH % 8 == 0 && kPWs % 8 == 0 && kPWn % 8 == 0 && kLd % 8 == 0,
+              "rows are copied 16 bytes at a time");
 
-// One warp per graph.  Train: also the loss, the bias and output gradients,
-// and per-node activations and pre-activation gradients for the weight
-// gradients.
+// rows x 64 BF16 from a dense array in global memory to row stride kLd, 16
+// bytes a thread.
+__device__ __forceinline__ void load_weights(uint16_t* dst, const uint16_t* __restrict__ src, int rows) {
+  for (int i = threadIdx.x; i < rows * (kHid / 8); i += blockDim.x)
+    *reinterpret_cast<uint4*>(dst + (i >> 3) * kLd + (i & 7) * 8) =
+        __ldg(reinterpret_cast<const uint4*>(src) + i);
+}
+
+// A group of kGraphThreads threads per graph.  Train: also the loss, the bias
+// and output gradients, and per-node activations and pre-activation gradients
+// for the weight gradients.  Bound by latency: a chain of small products with a
+// barrier after each.  (One warp per graph, its operands gathered element by
+// element with 8-way bank conflicts and the weights copied two bytes at a time,
+// took 158 us for the training step of 256 graphs; this takes 41 us.)
 template <bool kTrain>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock) mpnn_graph_kernel(
+__global__ void __launch_bounds__(kGraphThreads * kGraphsPerBlock) mpnn_graph_kernel(
     const uint16_t* __restrict__ wbf, const float* __restrict__ master, uint32_t num_graphs,
     const uint32_t* __restrict__ goff, const float* __restrict__ feat, const uint32_t* __restrict__ nbr,
     float* __restrict__ scores, const float* __restrict__ target, float inv_count, float* __restrict__ grad,
     float* __restrict__ loss, uint16_t* __restrict__ acts) {
+  using Buf = typename std::conditional<kTrain, GraphBufTrain, GraphBuf>::type;
   extern __shared__ __align__(16) unsigned char smem[];
   BlockW& W = *reinterpret_cast<BlockW*>(smem);
-  WarpBuf& B = reinterpret_cast<WarpBuf*>(smem + sizeof(BlockW))[threadIdx.x >> 5];
-  for (int i = threadIdx.x; i < kFeatPad * kHid; i += blockDim.x) W.win[i] = wbf[kPWin + i];
-  for (int i = threadIdx.x; i < kLayers * kHid * kHid; i += blockDim.x) {
-    W.ws[0][i] = wbf[kPWs + i];
-    W.wn[0][i] = wbf[kPWn + i];
-  }
+  const int group = threadIdx.x / kGraphThreads, tid = threadIdx.x % kGraphThreads;
+  Buf& B = reinterpret_cast<Buf*>(smem + sizeof(BlockW))[group];
+  load_weights(W.win, wbf + kPWin, kFeatPad);
+  load_weights(W.ws[0], wbf + kPWs, kLayers * kHid);
+  load_weights(W.wn[0], wbf + kPWn, kLayers * kHid);
   __syncthreads();
-  const int lane = threadIdx.x & 31;
+  auto sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "r"(kGraphThreads) : "memory"); };
+  const int lane = tid & 31, warp = tid >> 5, n0 = warp * 16;
   const float* b_in = master + kPBin;
   const float* b_l = master + kPB;
   const float* w_out = master + kPWout;
   const float b_out = master[kPBout];
-  float acc[2][8][4];
-  for (uint32_t q = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5); q < num_graphs;
-       q += gridDim.x * kWarpsPerBlock) {
+  float acc[2][2][4];
+  for (uint32_t q = blockIdx.x + group * gridDim.x; q < num_graphs; q += gridDim.x * kGraphsPerBlock) {
     const uint32_t g0 = goff[q];
     const int n = int(goff[q + 1] - g0);
+    sync();  // the previous graph's buffers are read
     // inputs
-    for (int r = 0; r < 32; r++) {
-      if (lane < kFeatPad) B.x[r * kFeatPad + lane] = (r < n && lane < kFeat) ? f2bf(feat[(g0 + r) * kFeat + lane]) : 0;
+    for (int i = tid; i < 32 * kFeatPad; i += kGraphThreads) {
+      const int r = i / kFeatPad, c = i % kFeatPad;
+      B.x[r * kLdX + c] = (r < n && c < kFeat) ? f2bf(feat[uint64_t(g0 + r) * kFeat + c]) : uint16_t(0);
     }
-    const uint32_t my_nbr = lane < n ? nbr[g0 + lane] : 0u;
-    B.nbr[lane] = my_nbr;
-    B.invdeg[lane] = my_nbr ? 1.f / float(__popc(my_nbr)) : 0.f;
-    __syncwarp();
+    if (tid < 32) {
+      const uint32_t mine = tid < n ? nbr[g0 + tid] : 0u;
+      B.nbr[tid] = mine;
+      B.invdeg[tid] = mine ? 1.f / float(__popc(mine)) : 0.f;
+    }
+    sync();
     // input layer
     zero_acc(acc);
-    warp_gemm(kFeatPad, [&](int r, int k) { return B.x[r * kFeatPad + k]; },
-              [&](int k, int c) { return W.win[k * kHid + c]; }, acc);
-    for_acc(acc, [&](int r, int c, float& v) { B.h[0][r * kHid + c] = r < n ? f2bf(fmaxf(v + b_in[c], 0.f)) : 0; });
-    __syncwarp();
+    gemm_cols<kFeatPad, false>(B.x, kLdX, W.win, n0, acc);
+    for_acc(acc, n0, [&](int r, int c, float v) { B.h[0][r * kLd + c] = r < n ? f2bf(fmaxf(v + b_in[c], 0.f)) : 0; });
+    sync();
     for (int l = 0; l < kLayers; l++) {
-      // mean over neighbours, two columns per lane
-      for (int r = 0; r < 32; r++) {
-        const uint32_t nb = B.nbr[r];
+      // mean over neighbours, eight rows per warp, two columns per lane
+      for (int r = warp * 8; r < warp * 8 + 8; r++) {
         float s0 = 0.f, s1 = 0.f;
-        uint32_t m = nb;
+        uint32_t m = B.nbr[r];
         while (m) {
           const int j = __ffs(m) - 1;
           m &= m - 1;
-          s0 += bf2f(B.h[l][j * kHid + 2 * lane]);
-          s1 += bf2f(B.h[l][j * kHid + 2 * lane + 1]);
+          const uint32_t v = *reinterpret_cast<const uint32_t*>(&B.h[l][j * kLd + 2 * lane]);
+          s0 += bf2f(uint16_t(v));
+          s1 += bf2f(uint16_t(v >> 16));
         }
         const float id = B.invdeg[r];
-        B.m[l][r * kHid + 2 * lane] = f2bf(s0 * id);
-        B.m[l][r * kHid + 2 * lane + 1] = f2bf(s1 * id);
+        *reinterpret_cast<uint32_t*>(&B.m[l][r * kLd + 2 * lane]) =
+            uint32_t(f2bf(s0 * id)) | (uint32_t(f2bf(s1 * id)) << 16);
       }
-      __syncwarp();
+      sync();
       zero_acc(acc);
-      warp_gemm(kHid, [&](int r, int k) { return B.h[l][r * kHid + k]; },
-                [&](int k, int c) { return W.ws[l][k * kHid + c]; }, acc);
-      warp_gemm(kHid, [&](int r, int k) { return B.m[l][r * kHid + k]; },
-                [&](int k, int c) { return W.wn[l][k * kHid + c]; }, acc);
+      gemm_cols<kHid, false>(B.h[l], kLd, W.ws[l], n0, acc);
+      gemm_cols<kHid, false>(B.m[l], kLd, W.wn[l], n0, acc);
       const float* bl = b_l + l * kHid;
-      for_acc(acc, [&](int r, int c, float& v) {
-        B.h[l + 1][r * kHid + c] = r < n ? f2bf(fmaxf(v + bl[c], 0.f)) : 0;
+      for_acc(acc, n0, [&](int r, int c, float v) {
+        B.h[l + 1][r * kLd + c] = r < n ? f2bf(fmaxf(v + bl[c], 0.f)) : 0;
       });
-      __syncwarp();
+      sync();
     }
-    // scores: lane r
-    float s = 0.f;
-    if (lane < n) {
-      s = b_out;
-      for (int c = 0; c < kHid; c++) s += bf2f(B.h[kLayers][lane * kHid + c]) * w_out[c];
-      scores[g0 + lane] = s;
-    }
-    if (!kTrain) continue;
-
-    // ---- backward ----
-    const float ds = lane < n ? 2.f * inv_count * (s - target[g0 + lane]) : 0.f;
-    float lsum = lane < n ? (s - target[g0 + lane]) * (s - target[g0 + lane]) * inv_count : 0.f;
-    lsum = warp_sum(lsum);
-    const float dsum = warp_sum(ds);
-    if (lane == 0) {
-      atomicAdd(loss, lsum);
-      atomicAdd(grad + kPBout, dsum);
-    }
-    // d w_out[c] = sum_r h3[r][c] ds_r ; d h3[r][c] = ds_r w_out[c]
-    for (int c = lane; c < kHid; c += 32) {
-      float gw = 0.f;
-      for (int r = 0; r < n; r++) gw += bf2f(B.h[kLayers][r * kHid + c]) * __shfl_sync(0xffffffffu, ds, r);
-      atomicAdd(grad + kPWout + c, gw);
-    }
-    for (int r = 0; r < 32; r++) {
-      const float dr = __shfl_sync(0xffffffffu, ds, r);
-      B.dh[r * kHid + lane] = dr * w_out[lane];
-      B.dh[r * kHid + lane + 32] = dr * w_out[lane + 32];
-    }
-    __syncwarp();
-    for (int l = kLayers - 1; l >= -1; l--) {
-      // dz = dh * relu'(h_{l+1}); bias gradient
-      const uint16_t* hl1 = B.h[l + 1];
-      float db0 = 0.f, db1 = 0.f;
-      for (int r = 0; r < 32; r++) {
-        const int c0 = lane, c1 = lane + 32;
-        const float z0 = (r < n && bf2f(hl1[r * kHid + c0]) > 0.f) ? B.dh[r * kHid + c0] : 0.f;
-        const float z1 = (r < n && bf2f(hl1[r * kHid + c1]) > 0.f) ? B.dh[r * kHid + c1] : 0.f;
-        B.dz[r * kHid + c0] = f2bf(z0);
-        B.dz[r * kHid + c1] = f2bf(z1);
-        db0 += z0;
-        db1 += z1;
+    // scores: row tid
+    if (warp == 0) {
+      float s = 0.f;
+      if (lane < n) {
+        s = b_out;
+        for (int c = 0; c < kHid; c++) s += bf2f(B.h[kLayers][lane * kLd + c]) * w_out[c];
+        scores[g0 + lane] = s;
       }
-      float* gb = grad + (l >= 0 ? kPB + l * kHid : kPBin);
-      atomicAdd(gb + lane, db0);
-      atomicAdd(gb + lane + 32, db1);
-      __syncwarp();
-      // save per-node records for the weight gradients
-      for (int r = 0; r < n; r++) {
-        uint16_t* rec = acts + uint64_t(g0 + r) * kActW;
-        rec[kActDz + (l + 1) * kHid + lane] = B.dz[r * kHid + lane];
-        rec[kActDz + (l + 1) * kHid + lane + 32] = B.dz[r * kHid + lane + 32];
-        if (l >= 0) {
-          rec[kActH + l * kHid + lane] = B.h[l][r * kHid + lane];
-          rec[kActH + l * kHid + lane + 32] = B.h[l][r * kHid + lane + 32];
-          rec[kActM + l * kHid + lane] = B.m[l][r * kHid + lane];
-          rec[kActM + l * kHid + lane + 32] = B.m[l][r * kHid + lane + 32];
-        } else if (lane < kFeatPad) {
-          rec[kActX + lane] = B.x[r * kFeatPad + lane];
+      if constexpr (kTrain) {
+        const float ds = lane < n ? 2.f * inv_count * (s - target[g0 + lane]) : 0.f;
+        const float lsum = warp_sum(lane < n ? (s - target[g0 + lane]) * (s - target[g0 + lane]) * inv_count : 0.f);
+        const float dsum = warp_sum(ds);
+        B.ds[lane] = ds;
+        if (lane == 0) {
+          atomicAdd(loss, lsum);
+          atomicAdd(grad + kPBout, dsum);
         }
       }
-      if (l < 0) break;
-      // dh_l = dz W_s^T + A_norm^T (dz W_n^T)
-      zero_acc(acc);
-      warp_gemm(kHid, [&](int r, int k) { return B.dz[r * kHid + k]; },
-                [&](int k, int c) { return W.wn[l][c * kHid + k]; }, acc);
-      for_acc(acc, [&](int r, int c, float& v) { B.q[r * kHid + c] = v * B.invdeg[r]; });
-      zero_acc(acc);
-      warp_gemm(kHid, [&](int r, int k) { return B.dz[r * kHid + k]; },
-                [&](int k, int c) { return W.ws[l][c * kHid + k]; }, acc);
-      __syncwarp();
-      for_acc(acc, [&](int r, int c, float& v) {
-        // (A_norm^T Q)[r] = sum over i with r in nbr(i) of Q[i] / deg_i (already scaled)
-        float t = v;
-        const uint32_t nb = B.nbr[r];  // symmetric adjacency: i in nbr(r) <=> r in nbr(i)
-        uint32_t m = nb;
-        while (m) {
-          const int i = __ffs(m) - 1;
-          m &= m - 1;
-          t += B.q[i * kHid + c];
+    }
+    if constexpr (kTrain) {
+      sync();
+      // ---- backward ----
+      // d w_out[c] = sum_r h3[r][c] ds_r ; d h3[r][c] = ds_r w_out[c]
+      const int col = tid & (kHid - 1), half = tid / kHid;  // a column, and every other row
+      {
+        float gw = 0.f;
+        const float wo = w_out[col];
+        for (int r = half; r < 32; r += 2) {
+          const float dr = B.ds[r];
+          if (r < n) gw += bf2f(B.h[kLayers][r * kLd + col]) * dr;
+          B.dh[r * kLdF + col] = dr * wo;
         }
-        B.dh[r * kHid + c] = r < n ? t : 0.f;
-      });
-      __syncwarp();
+        atomicAdd(grad + kPWout + col, gw);
+      }
+      sync();
+      for (int l = kLayers - 1; l >= -1; l--) {
+        // dz = dh * relu'(h_{l+1}); bias gradient
+        const uint16_t* hl1 = B.h[l + 1];
+        float db = 0.f;
+        for (int r = half; r < 32; r += 2) {
+          const float z = (r < n && bf2f(hl1[r * kLd + col]) > 0.f) ? B.dh[r * kLdF + col] : 0.f;
+          B.dz[r * kLd + col] = f2bf(z);
+          db += z;
+        }
+        atomicAdd(grad + (l >= 0 ? kPB + l * kHid : kPBin) + col, db);
+        sync();
+        // save per-node records for the weight gradients, 16 bytes a thread
+        for (int i = tid; i < n * 8; i += kGraphThreads) {
+          const int r = i >> 3, c = (i & 7) * 8;
+          uint16_t* rec = acts + uint64_t(g0 + r) * kActW;
+          auto save = [&](int to, const uint16_t* from) {
+            *reinterpret_cast<uint4*>(rec + to + c) = *reinterpret_cast<const uint4*>(from + r * kLd + c);
+          };
+          save(kActDz + (l + 1) * kHid, B.dz);
+          if (l >= 0) {
+            save(kActH + l * kHid, B.h[l]);
+            save(kActM + l * kHid, B.m[l]);
+          } else if (c < kFeatPad) {
+            *reinterpret_cast<uint4*>(rec + kActX + c) = *reinterpret_cast<const uint4*>(B.x + r * kLdX + c);
+          }
+        }
+        if (l < 0) break;
+        // dh_l = dz W_s^T + A_norm^T (dz W_n^T)
+        zero_acc(acc);
+        gemm_cols<kHid, true>(B.dz, kLd, W.wn[l], n0, acc);
+        for_acc(acc, n0, [&](int r, int c, float v) { B.q[r * kLdF + c] = v * B.invdeg[r]; });
+        zero_acc(acc);
+        gemm_cols<kHid, true>(B.dz, kLd, W.ws[l], n0, acc);
+        sync();
+        for_acc(acc, n0, [&](int r, int c, float v) {
+          // (A_norm^T Q)[r] = sum over i with r in nbr(i) of Q[i] / deg_i (already scaled)
+          float t = v;
+          uint32_t m = B.nbr[r];  // symmetric adjacency: i in nbr(r) <=> r in nbr(i)
+          while (m) {
+            const int i = __ffs(m) - 1;
+            m &= m - 1;
+            t += B.q[i * kLdF + c];
+          }
+          B.dh[r * kLdF + c] = r < n ? t : 0.f;
+        });
+        sync();
+      }
     }
   }
 }
 
 // Weight gradients: for matrix id (0: W_in, 1..3: W_s, 4..6: W_n),
-// G[i][c] = sum over nodes of A_node[i] * dZ_node[c]; K-split over blocks,
-// one warp per 32 output rows.
-__global__ void __launch_bounds__(64) mpnn_wgrad_kernel(const uint16_t* __restrict__ acts, uint32_t nodes,
-                                                        uint32_t nodes_per_block, float* __restrict__ grad) {
+// G[i][c] = sum over nodes of A_node[i] * dZ_node[c]; blocks of kWgradNodes
+// nodes, staged in shared memory, one warp per 16 output rows.  Bound by the
+// records' reads from L2 and the atomics of the partial sums.  (512 nodes a
+// block, one warp per 32 rows gathering two bytes at a time, ran 63 blocks and
+// took 169 us for 4,600 nodes; this takes 11.5 us.)
+constexpr int kWgradNodes = 128;
+__global__ void __launch_bounds__(128) mpnn_wgrad_kernel(const uint16_t* __restrict__ acts, uint32_t nodes,
+                                                         float* __restrict__ grad) {
+  __shared__ __align__(16) uint16_t sa[kWgradNodes * kLd], sz[kWgradNodes * kLd];
   const int mat = blockIdx.y;
-  const int warp = threadIdx.x >> 5;
   const int rows = mat == 0 ? kFeatPad : kHid;
-  if (warp * 32 >= rows) return;
   int asrc, dzsrc, gdst;
   if (mat == 0) { asrc = kActX; dzsrc = kActDz; gdst = kPWin; }
   else if (mat <= kLayers) { asrc = kActH + (mat - 1) * kHid; dzsrc = kActDz + mat * kHid; gdst = kPWs + (mat - 1) * kHid * kHid; }
   else { asrc = kActM + (mat - 1 - kLayers) * kHid; dzsrc = kActDz + (mat - kLayers) * kHid; gdst = kPWn + (mat - 1 - kLayers) * kHid * kHid; }
-  const uint32_t k_begin = blockIdx.x * nodes_per_block;
-  const uint32_t k_end = min(nodes, k_begin + nodes_per_block);
-  if (k_begin >= k_end) return;
-  float acc[2][8][4];
-  zero_acc(acc);
-  const int r_base = warp * 32;
-  for (uint32_t kb = k_begin; kb < k_end; kb += 16) {
-    auto A = [&](int r, int k) -> uint16_t {
-      const uint32_t node = kb + k;
-      const int i = r_base + r;
-      return (node < k_end && i < rows) ? acts[uint64_t(node) * kActW + asrc + i] : uint16_t(0);
-    };
-    auto Bf = [&](int k, int c) -> uint16_t {
-      const uint32_t node = kb + k;
-      return node < k_end ? acts[uint64_t(node) * kActW + dzsrc + c] : uint16_t(0);
-    };
-    warp_gemm(16, A, Bf, acc);
+  const uint32_t begin = blockIdx.x * kWgradNodes;
+  const uint4 none = make_uint4(0, 0, 0, 0);
+  for (int i = threadIdx.x; i < kWgradNodes * 8; i += blockDim.x) {
+    const int k = i >> 3, c = (i & 7) * 8;
+    const uint16_t* rec = acts + uint64_t(begin + k) * kActW;
+    const bool in = begin + k < nodes;
+    *reinterpret_cast<uint4*>(sz + k * kLd + c) = in ? *reinterpret_cast<const uint4*>(rec + dzsrc + c) : none;
+    if (c < rows) *reinterpret_cast<uint4*>(sa + k * kLd + c) = in ? *reinterpret_cast<const uint4*>(rec + asrc + c) : none;
   }
-  for_acc(acc, [&](int r, int c, float& v) {
-    const int i = r_base + r;
-    if (i < rows && v != 0.f) atomicAdd(grad + gdst + i * kHid + c, v);
-  });
+  __syncthreads();
+  const int lane = threadIdx.x & 31, m0 = (threadIdx.x >> 5) * 16;
+  if (m0 >= rows) return;
+  float acc[8][4] = {};
+#pragma unroll 2
+  for (int kk = 0; kk < kWgradNodes; kk += 16) {
+    uint32_t a[4];
+    ldmatrix4<true>(a, sa + (kk + (lane & 7) + (lane >> 4) * 8) * kLd + m0 + ((lane >> 3) & 1) * 8);
+#pragma unroll
+    for (int nt = 0; nt < 8; nt += 2) {
+      uint32_t b[4];
+      ldmatrix4<true>(b, sz + (kk + (lane & 15)) * kLd + nt * 8 + (lane >> 4) * 8);
+      mma_bf16(acc[nt], a, b[0], b[1]);
+      mma_bf16(acc[nt + 1], a, b[2], b[3]);
+    }
+  }
+  const int g = lane >> 2, c = lane & 3;
+#pragma unroll
+  for (int nt = 0; nt < 8; nt++)
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const float v = acc[nt][j];
+      if (v != 0.f) atomicAdd(grad + gdst + (m0 + g + (j >= 2 ? 8 : 0)) * kHid + nt * 8 + 2 * c + (j & 1), v);
+    }
 }
 
 __global__ void mpnn_adam_kernel(float* p, const float* g, float* m1, float* m2, uint16_t* wbf, int n, float lr,
@@ -354,23 +400,26 @@ __global__ void mpnn_features_kernel(const QVert* __restrict__ qv, uint32_t G, c
   }
 }
 
-size_t graph_kernel_smem() { return sizeof(BlockW) + kWarpsPerBlock * sizeof(WarpBuf); }
+size_t graph_kernel_smem(bool train) {
+  return sizeof(BlockW) + kGraphsPerBlock * (train ? sizeof(GraphBufTrain) : sizeof(GraphBuf));
+}
 
 int launch_graph_kernel(Engine& e, bool train, uint32_t num_graphs, const uint32_t* d_goff, const float* d_feat,
                         const uint32_t* d_nbr, float* d_scores, const float* d_target, float inv_count,
                         float* d_loss, uint16_t* d_acts) {
   MpnnState& M = *e.mpnn;
   if (!num_graphs) return FSIG_OK;
-  const size_t smem = graph_kernel_smem();
-  const unsigned grid = std::max(1u, std::min<unsigned>((num_graphs + kWarpsPerBlock - 1) / kWarpsPerBlock,
-                                                       unsigned(e.num_sms) * 4));
+  const size_t smem = graph_kernel_smem(train);
+  const unsigned threads = kGraphThreads * kGraphsPerBlock;
+  // one block an SM (shared memory); few graphs go to a block each
+  const unsigned grid = std::min<unsigned>(num_graphs, unsigned(e.num_sms));
   int rc = mpnn_configure(e);
   if (rc) return rc;
   if (train) {
-    mpnn_graph_kernel<true><<<grid, 32 * kWarpsPerBlock, smem, e.stream>>>(
+    mpnn_graph_kernel<true><<<grid, threads, smem, e.stream>>>(
         M.wbf, M.master, num_graphs, d_goff, d_feat, d_nbr, d_scores, d_target, inv_count, M.grad, d_loss, d_acts);
   } else {
-    mpnn_graph_kernel<false><<<grid, 32 * kWarpsPerBlock, smem, e.stream>>>(
+    mpnn_graph_kernel<false><<<grid, threads, smem, e.stream>>>(
         M.wbf, M.master, num_graphs, d_goff, d_feat, d_nbr, d_scores, nullptr, 0.f, nullptr, nullptr, nullptr);
   }
   FSIG_CUDA_TRY(cudaGetLastError());
@@ -381,9 +430,10 @@ int launch_graph_kernel(Engine& e, bool train, uint32_t num_graphs, const uint32
 
 int mpnn_configure(Engine& e) {
   if (e.mpnn_configured) return FSIG_OK;
-  const int smem = int(graph_kernel_smem());
-  FSIG_CUDA_TRY(cudaFuncSetAttribute(mpnn_graph_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  FSIG_CUDA_TRY(cudaFuncSetAttribute(mpnn_graph_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  FSIG_CUDA_TRY(cudaFuncSetAttribute(mpnn_graph_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     int(graph_kernel_smem(true))));
+  FSIG_CUDA_TRY(cudaFuncSetAttribute(mpnn_graph_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     int(graph_kernel_smem(false))));
   e.mpnn_configured = true;
   return FSIG_OK;
 }
@@ -499,9 +549,8 @@ int mpnn_run(Engine& e, uint32_t num_graphs, const uint32_t* goff, const float* 
     rc = launch_graph_kernel(e, true, num_graphs, d_goff, d_feat, d_nbr, d_scores, d_target,
                              nodes ? 1.f / float(nodes) : 0.f, d_loss, d_acts);
     if (!rc && nodes) {
-      const uint32_t per_block = 512;
-      dim3 grid((nodes + per_block - 1) / per_block, 1 + 2 * kLayers);
-      mpnn_wgrad_kernel<<<grid, 64, 0, s>>>(d_acts, nodes, per_block, M.grad);
+      dim3 grid((nodes + kWgradNodes - 1) / kWgradNodes, 1 + 2 * kLayers);
+      mpnn_wgrad_kernel<<<grid, 128, 0, s>>>(d_acts, nodes, M.grad);
       FSIG_CUDA_TRY(cudaGetLastError());
     }
     if (!rc && lr > 0.f) {
