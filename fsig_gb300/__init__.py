@@ -447,6 +447,23 @@ def _result(r: _Result) -> Result:
                   [int(x) for x in r.level_counts[:n]], float(r.ms_filter), float(r.ms_join), int(r.work))
 
 
+_RESULT_DTYPE = np.dtype({"names": ["count", "hash", "status", "n", "order", "candidates", "levels", "ms_filter",
+                                    "ms_join", "work"],
+                          "formats": ["<u8", "<u8", "<i4", "<u4", ("<u4", MAX_QUERY), ("<u4", MAX_QUERY),
+                                      ("<u8", MAX_QUERY), "<f4", "<f4", "<u8"],
+                          "offsets": [getattr(_Result, f).offset for f, _ in _Result._fields_],
+                          "itemsize": C.sizeof(_Result)})
+
+
+def _results(res, count: int) -> list:
+    """The first `count` results of a batch, column by column: one conversion
+    per field instead of one per element (512 queries: 3.3 -> 1.9 ms)."""
+    a = np.frombuffer(res, _RESULT_DTYPE, count)
+    cols = [a[name].tolist() for name in _RESULT_DTYPE.names]
+    return [Result(c, h, st, o[:n], ca[:n], lv[:n], mf, mj, w)
+            for c, h, st, n, o, ca, lv, mf, mj, w in zip(*cols)]
+
+
 class Engine:
     """One device arena on one GPU; replaces init_GPU + MemoryManager."""
 
@@ -535,7 +552,7 @@ class Engine:
                           max_work, warps_per_block, learned_window, 0 if classes else 1, isect, refine_coop,
                           learned_prefix)
         self._check(self._L.fsig_match_batch(self._h, len(qs), arr, C.byref(opts), res), "match_batch")
-        return [_result(res[i]) for i in range(len(qs))]
+        return _results(res, len(qs))
 
     def set_queue_waits(self, ready_wait_ns: int = 0, idle_wait_ns: int = 0, unpublished: bool = False) -> None:
         """Bounded waits of the enumeration's work queue (0: defaults, 200 ms
@@ -586,7 +603,8 @@ class Engine:
 
     def build_pcsr(self, labels, offsets, adj, num_labels: int) -> list:
         """The reference's PCSR units, built on the device: a list of
-        (keys, list entries, slot table, lists) per unit, as the oracle's pcsr()."""
+        (keys, list entries, slot table, lists) per unit, as the oracle's pcsr();
+        the arrays of all units are parts of two arrays of this call."""
         lab = np.ascontiguousarray(labels, np.int32)
         off = np.ascontiguousarray(offsets, np.uint32)
         a = np.ascontiguousarray(adj, np.uint32)
@@ -604,7 +622,7 @@ class Engine:
         units, ob, eb = [], 0, 0
         for u in range(U):
             k, m = int(keys[u]), int(ne[u])
-            units.append((k, m, table[ob: ob + 32 * k].copy(), edges[eb: eb + m].copy()))
+            units.append((k, m, table[ob: ob + 32 * k], edges[eb: eb + m]))
             ob += 32 * k
             eb += m
         return units
