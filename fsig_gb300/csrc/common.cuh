@@ -49,27 +49,34 @@ __host__ __device__ __forceinline__ void sig_slot(int32_t label, uint32_t& word,
 }
 
 // ---------------------------------------------------------------------------
-// membership filter of the adjacency's label segments: 16 bits per entry, the
-// block of segment [lo, hi) being words [lo, hi).  A segment that is dense in
-// its label class (class extent at most 16 (hi - lo) ids) holds one bit per id of
-// the class, which is exact; another is a Bloom filter whose element x sets two
-// bits of one word, so that 2-3 % of the ids that are not in it pass.  One
+// membership filter of the adjacency's label segments: 1 << s words of 16 bits
+// per entry, the block of segment [lo, hi) being words [lo << s, hi << s).  A
+// segment that is dense in its label class (class extent at most as many ids as
+// its block has bits) holds one bit per id of the class, which is exact; another
+// is a Bloom filter whose element x sets two bits of one word, so that with one
+// word an entry 2-3 % of the ids that are not in it pass.  One
 // probe of a word settles most candidates that a binary search took 7-8
 // dependent loads to refuse: the 512-query batch on 2^26 edges 377 -> 197 ms,
-// house counting on 700 vertices (dense segments) 93 -> 63 ms.  16 bits an
-// entry is half the adjacency; the filter lies in arena room that the next
-// request takes back, so what fitted an arena still fits.
+// house counting on 700 vertices (dense segments) 93 -> 63 ms.  The filter lies
+// in arena room that the next request takes back, so what fitted an arena still
+// fits.  One word an entry is half the adjacency; graphs of at most
+// kFilterSmall entries get four (32 MB then, well inside the L2), which makes
+// segments from a quarter of that length on exact.
 // ---------------------------------------------------------------------------
+constexpr uint64_t kFilterSmall = 1ull << 22;
+__host__ __device__ __forceinline__ uint32_t filter_shift(uint64_t nadj) { return nadj <= kFilterSmall ? 2 : 0; }
 // the shortest dense segment of a class of this extent
-__device__ __forceinline__ uint32_t filter_dense_len(uint32_t extent) { return (extent >> 4) + ((extent & 15u) != 0); }
+__device__ __forceinline__ uint32_t filter_dense_len(uint32_t extent, uint32_t shift) {
+  return ((extent - 1) >> (4 + shift)) + 1;
+}
 __device__ __forceinline__ uint32_t filter_hash(uint32_t x) { return x * 0x9e3779b1u; }
 __device__ __forceinline__ uint32_t filter_bits(uint32_t x) {
   const uint32_t h = x * 0x85ebca6bu;
   return (1u << (h >> 28)) | (1u << ((h >> 24) & 15u));
 }
-// word of x within its segment's block; rel = x - first id of the class's extent
-__device__ __forceinline__ uint32_t filter_word(bool dense, uint32_t rel, uint32_t hash, uint32_t len) {
-  return dense ? rel >> 4 : __umulhi(hash, len);
+// word of x within its segment's block of `words`; rel = x - first id of the class's extent
+__device__ __forceinline__ uint32_t filter_word(bool dense, uint32_t rel, uint32_t hash, uint32_t words) {
+  return dense ? rel >> 4 : __umulhi(hash, words);
 }
 __device__ __forceinline__ uint32_t filter_mask(bool dense, uint32_t rel, uint32_t bits) {
   return dense ? 1u << (rel & 15u) : bits;

@@ -35,7 +35,7 @@ struct DeviceGraph {
   uint32_t* adj_old = nullptr;     // [nadj] caller id of each adj entry (for the result hash); null without lseg
   uint32_t* lseg = nullptr;        // [V*(L+1)]; null: segments are found by binary search in the rows
   uint4* sig = nullptr;            // [V*4] 64-byte signature per vertex
-  uint16_t* filt = nullptr;        // [nadj] membership filter, in the arena's tail; valid while that is kept
+  uint16_t* filt = nullptr;        // [nadj << filter_shift(nadj)] membership filter, in the arena's tail; valid while that is kept
   std::vector<uint32_t> h_base;    // host copy of base
   uint64_t arena_mark = 0;         // arena top after the graph store
 };

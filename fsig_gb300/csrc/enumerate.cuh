@@ -39,7 +39,12 @@
 // leaves of one segment, and buffers of one pool per warp (4 blocks an SM also
 // for 32-vertex queries, 3 with 32 entries for each depth): 27 and 23 ms, 198
 // instructions a window at 70 % of the issue rate; 512 queries of 12-32 vertices
-// on 2^26 edges 305 -> 146 ms, 279 instructions a window at 64 %.
+// on 2^26 edges 305 -> 146 ms, 279 instructions a window at 64 %.  With the first
+// filter tested beside the candidate bit (a third of the windows on 2^26 edges
+// end there), leaves of two segments in the leaf loop, and four earlier vertices
+// a load (a loop of one each took 25 % of the house count): 139 ms there, 21.5 ms
+// for 512 queries of 4-32 vertices, house counting 55 -> 32 ms.  In the leaf loop
+// the hash is 15 % of the time; loading a window ahead gains nothing.
 //
 // Work stealing: a warp that runs out of input takes a ticket, one atomicAdd
 // on the queue's head, and waits for the record of that number, polling the
@@ -150,14 +155,19 @@ struct WarpSmem {
   uint2 owner[kBuf];                // entries with a driver: its place relative to the window index, the entry
   unsigned long long sown[kBuf];    // leaf: partial hash of each entry being extended
   unsigned long long sbase[kBuf];   // partial hashes of depth n-3's buffer
-  uint2 scratch[kScratch / 2];      // per entry being extended: segments (start, length), then earlier vertices
+  // per entry being extended: its earlier vertices of the same label, four in a
+  // word; then its segments (start, length, as filter words)
+  alignas(16) uint2 scratch[kScratch / 2];
   uint32_t cand[kPool];             // mapped vertex
   uint8_t par[kPool];               // its parent's place in the previous depth's buffer
-  // event counters of the warp's share of one launch, kept here for the registers
-  // (lane 0): tasks, records popped, hand-offs, records written, windows
-  uint32_t ev[5];
-  uint32_t pend;                    // driver entries examined, not yet published to res.work (lane 0)
+  // What only fills, tasks and hand-offs touch is kept here for the registers.
+  unsigned long long found[kMaxQ];  // partial embeddings of each length, of the current query, not yet published
+  unsigned long long bytes;         // bytes requested by global loads
+  uint32_t ev[5];                   // events: tasks, records popped, hand-offs, records written, windows
+  uint32_t pend;                    // driver entries examined, not yet published to res.work
   uint32_t task_lo, task_hi;        // driver range of the task at its first depth
+  uint32_t t, t_last;               // input tasks in hand: [t, t_last)
+  uint32_t query, pad[3];
 };
 static_assert(sizeof(WarpSmem) % 16 == 0, "the next warp's part is aligned");
 
@@ -189,7 +199,7 @@ __device__ __forceinline__ void row_segment(const GraphView& g, uint32_t v, int3
 // (in the first alone without `two`): two binary searches in lockstep, so that a step
 // has two independent loads in flight.
 __device__ __forceinline__ bool in_segments(const uint32_t* __restrict__ a, uint32_t lo0, uint32_t n0, uint32_t lo1,
-                                            uint32_t n1, bool two, uint32_t x, uint32_t& bytes) {
+                                            uint32_t n1, bool two, uint32_t x, uint32_t& loads) {
   if (!two) n1 = 1;
   if (n0 == 0 || n1 == 0) return false;
 #pragma unroll 1
@@ -200,9 +210,9 @@ __device__ __forceinline__ bool in_segments(const uint32_t* __restrict__ a, uint
     if (y1 <= x) lo1 += h1;
     n0 -= h0;
     n1 -= h1;
-    bytes += 8;
+    loads += 2;
   }
-  bytes += 8;
+  loads += 2;
   return __ldg(a + lo0) == x && (!two || __ldg(a + lo1) == x);
 }
 
@@ -219,16 +229,19 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
   const uint32_t nroots = A.in_tasks ? 0u : *A.nroots_ptr;
   const uint32_t T_in = A.in_tasks ? A.in_count : min(A.chunk_off[nroots], A.t_end);
 
-  // lane-distributed level state; f is the task's prefix (lane j: f_j)
-  uint32_t f = 0, cnt = 0, it = 0, off = 0, sp = 0;  // sp: where depth j's buffer starts in the pool
+  // lane-distributed level state
+  uint32_t cnt = 0, it = 0, off = 0, sp = 0;  // sp: where depth j's buffer starts in the pool
   unsigned long long my_hash = 0;
   bool s_valid = false;  // sbase holds depth n-3's current buffer
-  unsigned long long lc = 0;  // lane j: partial embeddings of length j + 1 found (lane n-1: embeddings)
-  uint32_t bytes = 0;         // drained into the 64-bit total before it can overflow
+  ws.found[lane] = 0;
   if (lane < 5) ws.ev[lane] = 0;
-  if (lane == 0) ws.pend = 0;
+  if (lane == 0) {
+    ws.bytes = 0;
+    ws.pend = 0;
+    ws.t = ws.t_last = 0;
+    ws.query = kInvalid;
+  }
   __syncwarp();
-  uint32_t cur_q = kInvalid;
 
   // Publishes the driver entries this warp examined for the current query.
   // The total a query examines does not depend on how its work was split
@@ -236,9 +249,9 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
   // either.
   auto publish = [&]() {
     if (lane == 0 && ws.pend) {
-      const unsigned long long tot = atomicAdd(&A.res[cur_q].work, (unsigned long long)ws.pend) + ws.pend;
+      const unsigned long long tot = atomicAdd(&A.res[ws.query].work, (unsigned long long)ws.pend) + ws.pend;
       ws.pend = 0;
-      if (tot > A.work_cap) atomicExch(&A.res[cur_q].aborted, 1u);
+      if (tot > A.work_cap) atomicExch(&A.res[ws.query].aborted, 1u);
     }
   };
 
@@ -322,14 +335,14 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
     for (uint32_t k = 0; k < pieces; k++) {
       TaskRec* r = A.out_tasks + (slot++ & (A.out_cap - 1));
       if (lane <= l) r->f[lane] = fp;
-      if (lane == 0) { r->q = cur_q; r->d = l + 1; r->lo = lo + k * hand; r->hi = min(lo + (k + 1) * hand, hi); }
+      if (lane == 0) { r->q = ws.query; r->d = l + 1; r->lo = lo + k * hand; r->hi = min(lo + (k + 1) * hand, hi); }
     }
 #pragma unroll 1
     for (uint32_t k = first; k < c_l; k++) {
       TaskRec* r = A.out_tasks + (slot++ & (A.out_cap - 1));
       const uint32_t fk = prefix(l, k);
       if (lane <= l) r->f[lane] = fk;
-      if (lane == 0) { r->q = cur_q; r->d = l + 1; r->lo = kInvalid; r->hi = kInvalid; }
+      if (lane == 0) { r->q = ws.query; r->d = l + 1; r->lo = kInvalid; r->hi = kInvalid; }
     }
     if (lane == l) {
       it = cnt;
@@ -394,13 +407,25 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
     const bool leaf = lv + 1 == n;
     const uint32_t bwd = ws.plan.bwd[lv], inj = ws.plan.same[lv] & ~bwd;
     const int32_t lab = ws.plan.lab[lv];
-    const uint32_t nb = __popc(bwd), ni = __popc(inj);
-    const uint32_t stride = min(kBuf, kScratch / (2 * nb + ni));  // entries per group
-    uint32_t* const other = reinterpret_cast<uint32_t*>(ws.scratch + nb * stride);  // [ni][stride]
+    const uint32_t nb = __popc(bwd), n4 = (__popc(inj) + 3) / 4;
+    const uint32_t stride = min(kBuf, kScratch / (2 * nb + 4 * n4));  // entries per group
+    uint4* const other = reinterpret_cast<uint4*>(ws.scratch);  // [n4][stride], padded with kInvalid
+    uint2* const segs = ws.scratch + 2 * n4 * stride;           // [nb][stride]
+    // whether x is none of entry c's earlier vertices
+    auto fresh = [&](uint32_t x, uint32_t c) {
+      bool yes = true;
+#pragma unroll 1
+      for (uint32_t k = 0; k < n4; k++) {
+        const uint4 o = other[k * stride + c];
+        yes = yes && x != o.x && x != o.y && x != o.z && x != o.w;
+      }
+      return yes;
+    };
     const uint32_t bmbase = ws.plan.bmbase[lv];
     const uint32_t* __restrict__ bm = A.pool + ws.plan.bmoff[lv];
-    // segments from this length on have an exact filter
-    const uint32_t dense = g.filt ? filter_dense_len(__ldg(g.base + lab + 1) - bmbase) : kInvalid;
+    // segments are kept in units of their filter's words; from `dense` on it is exact
+    const uint32_t fs = g.filt ? g.fshift : 0;
+    const uint32_t dense = g.filt ? filter_dense_len(__ldg(g.base + lab + 1) - bmbase, fs) << fs : kInvalid;
     const uint32_t cntp = __shfl_sync(kFull, cnt, p), spp = __shfl_sync(kFull, sp, p);
     const uint32_t spl = spp + cntp;                              // depth lv's buffer
     const uint32_t room = min(kBuf, kPool - spl - (n - 2 - min(lv, n - 2)));
@@ -409,7 +434,7 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
     const uint32_t enough = nb > 1 || room < 16 ? (room + 1) / 2 : room - 8;
     uint32_t itp = __shfl_sync(kFull, it, p), offp = __shfl_sync(kFull, off, p);
     uint32_t have = 0, sure = 0;  // entries appended; of them, searched for in every segment
-    uint32_t used = 0, seen = 0, hits = 0;
+    uint32_t used = 0, seen = 0, hits = 0, loads = 0;  // loads: 4-byte loads of the filters and searches
     bool stop = false;
     if (leaf && !s_valid && lv >= 2) {  // partial hashes of depth n-3's entries
       unsigned long long sum = 0;
@@ -432,13 +457,17 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
       uint32_t dlo = 0, len = kInvalid, drv = 0;
       {
         uint32_t at = own, need = bwd | inj, wb = 0, wi = 0;
+        if (mine) {
+#pragma unroll 1
+          for (uint32_t k = 0; k < n4; k++) other[k * stride + lane] = make_uint4(kInvalid, kInvalid, kInvalid, kInvalid);
+        }
 #pragma unroll 1
         for (uint32_t k = p;; k--) {
           const uint32_t v = ws.cand[at];
           if ((bwd >> k) & 1u) {
             uint32_t a, b;
             row_segment<kRows>(g, v, lab, W1, a, b);
-            if (mine) ws.scratch[wb * stride + lane] = make_uint2(a, b - a);
+            if (mine) segs[wb * stride + lane] = make_uint2(a << fs, (b - a) << fs);
             if (b - a < len) {
               len = b - a;
               dlo = a;
@@ -446,15 +475,14 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
             }
             wb++;
           } else if ((inj >> k) & 1u) {
-            if (mine) other[wi * stride + lane] = v;
+            if (mine) reinterpret_cast<uint32_t*>(&other[(wi >> 2) * stride + lane])[wi & 3] = v;
             wi++;
           }
           need &= ~(1u << k);
           if (!need) break;
           at = __shfl_sync(kFull, sp, k - 1) + ws.par[at];
         }
-        bytes += 8 * nb;
-        if (mine && drv) ws.scratch[drv * stride + lane] = ws.scratch[lane];  // the others: places 1 .. nb - 1
+        if (mine && drv) segs[drv * stride + lane] = segs[lane];  // the others: places 1 .. nb - 1
         if (lo_set != kInvalid) {
           dlo = lo_set;
           len = hi_set - lo_set;
@@ -487,9 +515,10 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
         if (len) ws.owner[rank] = make_uint2(dlo - start, lane);
       }
       __syncwarp();
+      const bool filtered = nb > 1 && g.filt;
       uint32_t pos = 0, begun = kInvalid;  // begun: drivers that start before pos, minus one
-      if (leaf && nb == 1 && !A.emit) {
-        // the common leaf: nothing to search, all lanes alike
+      if (leaf && !A.emit && (nb == 1 || (nb == 2 && filtered))) {
+        // the common leaves: at most one segment to look up, all lanes alike
         const uint64_t tq = uint64_t(ws.plan.qv[lv]) << 32;
 #pragma unroll 1
         while (pos < T && !stop) {
@@ -499,9 +528,19 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
           const uint32_t x = __ldg(g.adj + at);
           const uint32_t xo = kRows ? __ldg(g.old_of_new + x) : __ldg(g.adj_old + at);
           const uint32_t bit = x - bmbase;
-          bool pred = e < T && ((__ldg(bm + (bit >> 5)) >> (bit & 31)) & 1u);
-#pragma unroll 1
-          for (uint32_t i = 0; i < ni; i++) pred = pred && x != other[i * stride + o.y];
+          const uint32_t word = __ldg(bm + (bit >> 5));
+          bool pred = e < T && ((word >> (bit & 31)) & 1u);
+          if (nb == 2) {
+            const uint2 a = segs[stride + o.y];
+            const bool da = a.y >= dense;
+            const uint32_t w = __ldg(g.filt + (a.x + filter_word(da, bit, filter_hash(x), a.y)));
+            pred = pred && (~w & filter_mask(da, bit, filter_bits(x))) == 0;
+            if (__any_sync(kFull, pred && !da)) {
+              if (pred && !da) pred = in_segments(g.adj, a.x >> fs, a.y >> fs, a.x >> fs, 1, false, x, loads);
+              __syncwarp();
+            }
+          }
+          if (n4) pred = pred && fresh(x, o.y);
           const uint64_t h = fmix64(A.seed + ws.sown[o.y] + fmix64(tq | xo));
           my_hash += pred ? h : 0;
           hits += pred;
@@ -519,41 +558,52 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
         const uint32_t e = pos + lane, at = o.x + min(e, T - 1);
         uint32_t x = __ldg(g.adj + at), c = o.y;
         const uint32_t bit = x - bmbase;
-        bool pred = e < T && ((__ldg(bm + (bit >> 5)) >> (bit & 31)) & 1u);
+        const uint32_t word = __ldg(bm + (bit >> 5));
+        bool pred = e < T;
+        const uint32_t hash = filter_hash(x), bits = filter_bits(x);
+        if (filtered) {  // the first of the other segments' filters, beside the candidate bit
+          const uint2 a = segs[stride + c];
+          const bool da = a.y >= dense;
+          const uint32_t w = __ldg(g.filt + (a.x + filter_word(da, bit, hash, a.y)));
+          pred = pred && (~w & filter_mask(da, bit, bits)) == 0;
+        }
+        pred = pred && ((word >> (bit & 31)) & 1u);
+        uint32_t step = min(32u, T - pos);
+        used++;
+        const bool final = used >= kFillWindows;
+        if (__any_sync(kFull, pred)) {
+          if (n4) pred = pred && fresh(x, c);
+          if (filtered) {  // the other filters, two at a time
 #pragma unroll 1
-        for (uint32_t i = 0; i < ni; i++) pred = pred && x != other[i * stride + c];
-        if (nb > 1 && g.filt) {
-          // the other segments' filters, two at a time
-          const uint32_t hash = filter_hash(x), bits = filter_bits(x);
-#pragma unroll 1
-          for (uint32_t k = 1; k < nb && __any_sync(kFull, pred); k += 2) {
-            const uint2 a = ws.scratch[k * stride + c], b = ws.scratch[min(k + 1, nb - 1) * stride + c];
-            const bool da = a.y >= dense, db = b.y >= dense;
-            uint32_t wa = 0, wb = 0;
-            if (pred) {
-              wa = __ldg(g.filt + a.x + filter_word(da, bit, hash, a.y));
-              wb = __ldg(g.filt + b.x + filter_word(db, bit, hash, b.y));
-              bytes += 4;
+            for (uint32_t k = 2; k < nb && __any_sync(kFull, pred); k += 2) {
+              const uint2 a = segs[k * stride + c], b = segs[min(k + 1, nb - 1) * stride + c];
+              const bool da = a.y >= dense, db = b.y >= dense;
+              uint32_t wa = 0, wb = 0;
+              if (pred) {
+                wa = __ldg(g.filt + (a.x + filter_word(da, bit, hash, a.y)));
+                wb = __ldg(g.filt + (b.x + filter_word(db, bit, hash, b.y)));
+              }
+              loads++;
+              pred = ((~wa & filter_mask(da, bit, bits)) | (~wb & filter_mask(db, bit, bits))) == 0;
             }
-            pred = ((~wa & filter_mask(da, bit, bits)) | (~wb & filter_mask(db, bit, bits))) == 0;
+          }
+          if (!leaf) {
+            uint32_t m = __ballot_sync(kFull, pred);
+            const uint32_t rank = have + __popc(m & lanemask_lt());
+            if (have + __popc(m) > room) {  // take what fits; go on from the first one that does not
+              step = __ffs(__ballot_sync(kFull, pred && rank == room)) - 1;
+              m &= (1u << step) - 1;
+            }
+            if ((m >> lane) & 1u) {
+              ws.cand[spl + rank] = x;
+              ws.par[spl + rank] = uint8_t(itp + c);
+            }
+            have += __popc(m);
           }
         }
-        uint32_t step = min(32u, T - pos);
         bool searching = leaf && nb > 1;
-        used++;
         if (!leaf) {
-          uint32_t m = __ballot_sync(kFull, pred);
-          const uint32_t rank = have + __popc(m & lanemask_lt());
-          if (have + __popc(m) > room) {  // take what fits; go on from the first one that does not
-            step = __ffs(__ballot_sync(kFull, pred && rank == room)) - 1;
-            m &= (1u << step) - 1;
-          }
-          if ((m >> lane) & 1u) {
-            ws.cand[spl + rank] = x;
-            ws.par[spl + rank] = uint8_t(itp + c);
-          }
-          have += __popc(m);
-          searching = nb > 1 && have > sure && (have == room || pos + step >= T || used >= kFillWindows);
+          searching = nb > 1 && have > sure && (have == room || pos + step >= T || final);
           if (searching) {  // the entries not yet searched for, one per lane
             __syncwarp();
             pred = lane >= sure && lane < have;
@@ -568,16 +618,16 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
           uint32_t k = 1;
 #pragma unroll 1
           while (pred && k < nb) {
-            uint2 a = ws.scratch[k++ * stride + c];
+            uint2 a = segs[k++ * stride + c];
             if (a.y >= dense) continue;
             uint2 b = a;
             bool two = false;
 #pragma unroll 1
             while (k < nb && !two) {
-              b = ws.scratch[k++ * stride + c];
+              b = segs[k++ * stride + c];
               two = b.y < dense;
             }
-            pred = in_segments(g.adj, a.x, a.y, b.x, b.y, two, x, bytes);
+            pred = in_segments(g.adj, a.x >> fs, a.y >> fs, b.x >> fs, b.y >> fs, two, x, loads);
           }
         }
         __syncwarp();
@@ -607,7 +657,7 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
         begun += __popc(step < 32 ? heads & ((1u << step) - 1) : heads);
         pos += step;
         seen += step;
-        stop = stop || used >= kFillWindows;
+        stop = stop || final;
       }
       if (pos >= T) {
         itp += group;
@@ -624,25 +674,23 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
       it = itp;
       off = offp;
     }
-    if (lane == lv) {
-      lc += have;
-      if (!leaf) {
-        cnt = have;
-        it = 0;
-        off = 0;
-        sp = spl;
-      }
+    if (lane == lv && !leaf) {
+      cnt = have;
+      it = 0;
+      off = 0;
+      sp = spl;
     }
     if (lv + 3 == n) s_valid = false;
+    loads = __reduce_add_sync(kFull, loads);
     if (lane == 0) {
+      ws.found[lv] += have;
       ws.ev[4] += used;
+      ws.bytes += 4ull * loads + ((leaf ? 12ull : 8ull) + (nb > 1 && g.filt ? 4ull : 0ull)) * seen;
       if (A.work_cap) ws.pend += seen;
     }
-    bytes += leaf ? 12 * used : 8 * used;
     return used;
   };
 
-  uint32_t t = 0, t_last = 0;  // input tasks in hand: [t, t_last)
 #pragma unroll 1
   for (;;) {
     // ---- the next task: query q, depth d, mapped f (lane-distributed, lanes
@@ -653,13 +701,19 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
     uint32_t q = kInvalid, d = 1, lo = kInvalid, hi = kInvalid, root = kInvalid, chunk = 0;
     const TaskRec* rec = nullptr;
     uint32_t* ready = nullptr;
-    uint32_t free_word = 0;
+    uint32_t free_word = 0, f = 0;
+    uint32_t t = ws.t, t_last = ws.t_last;
+    __syncwarp();
     if (t == t_last) {  // input tasks (after an error every task ends at its first check)
       uint32_t t0 = T_in;
       if (lane == 0 && *(volatile uint32_t*)&A.ctr[0 * kCtrStride] < T_in)
         t0 = atomicAdd(&A.ctr[0 * kCtrStride], A.chunk);
       t = __shfl_sync(kFull, t0, 0);
       t_last = t < T_in ? min(t + A.chunk, T_in) : t;
+    }
+    if (lane == 0) {
+      ws.t = min(t + 1, t_last);
+      ws.t_last = t_last;
     }
     if (t < t_last) {
       if (A.in_tasks) {
@@ -676,7 +730,6 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
         q = A.root_q[a];
         root = A.roots[a];
       }
-      t++;
     } else {
       // input exhausted: take a ticket and wait for its record while others work
       uint32_t slot = kInvalid;
@@ -746,16 +799,19 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
       }
     }
     // ---- its query
+    __syncwarp();
+    const uint32_t cur_q = ws.query;
     if (q != cur_q || q == kInvalid) {
       if (cur_q != kInvalid) {
         publish();
-        const unsigned long long h = warp_sum(my_hash);
+        const unsigned long long h = warp_sum(my_hash), c = ws.found[lane];
         if (lane == 0 && h) atomicAdd(&A.res[cur_q].hash, h);
-        if (lane < ws.plan.n && lc) {
-          atomicAdd(&A.res[cur_q].levels[lane], lc);
-          if (lane + 1 == ws.plan.n) atomicAdd(&A.res[cur_q].count, lc);
+        if (lane < ws.plan.n && c) {
+          atomicAdd(&A.res[cur_q].levels[lane], c);
+          if (lane + 1 == ws.plan.n) atomicAdd(&A.res[cur_q].count, c);
         }
-        my_hash = lc = 0;
+        my_hash = 0;
+        ws.found[lane] = 0;
       }
       if (q == kInvalid) break;
       __syncwarp();
@@ -763,14 +819,14 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
       uint32_t* dst = reinterpret_cast<uint32_t*>(&ws.plan);
 #pragma unroll 1
       for (uint32_t i = lane; i < sizeof(Plan) / 4; i += 32) dst[i] = src[i];
+      if (lane == 0) ws.query = q;
       __syncwarp();
-      cur_q = q;
     }
     const uint32_t n = ws.plan.n;
     if (root != kInvalid) {
       if (lane == 0) {
         f = root;
-        lc += chunk == 0;  // the root itself, once
+        ws.found[0] += chunk == 0;  // the root itself, once
       }
       if (n > 1) {
         row_segment<kRows>(g, root, ws.plan.lab[1], W1, lo, hi);
@@ -783,7 +839,6 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
       if (lane == 0) {
         const uint32_t xo = __ldg(g.old_of_new + f);
         my_hash += fmix64(A.seed + fmix64((uint64_t(ws.plan.qv[0]) << 32) | xo));
-        bytes += 4;
         if (A.emit) {
           const unsigned long long row = atomicAdd(A.emit_ctr, 1ull);
           if (row < A.emit_cap) A.emit[row] = xo;
@@ -815,15 +870,10 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
         // at the start and every kCheckWindows windows: the query's work limit,
         // the pass's error word (the call will fail anyway), and waiting warps
         windows = 0;
-        if (__any_sync(kFull, bytes >= (1u << 30))) {
-          const unsigned long long b = warp_sum((unsigned long long)bytes);
-          if (lane == 0) atomicAdd(A.algo_bytes, b);
-          bytes = 0;
-        }
         int stop = 0;
         if (A.work_cap) {
           publish();
-          if (lane == 0) stop = *(volatile unsigned int*)&A.res[cur_q].aborted != 0;
+          if (lane == 0) stop = *(volatile unsigned int*)&A.res[ws.query].aborted != 0;
         }
         if (lane == 0) stop |= *(volatile uint32_t*)&A.ctr[3 * kCtrStride] != 0;
         if (__shfl_sync(kFull, stop, 0)) break;
@@ -845,9 +895,8 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
       if (lv + 1 < n && __shfl_sync(kFull, cnt, lv) > 0) lv++;
     }
   }
-  const unsigned long long all_bytes = warp_sum((unsigned long long)bytes);
   if (lane == 0) {
-    atomicAdd(A.algo_bytes, all_bytes);
+    atomicAdd(A.algo_bytes, ws.bytes);
 #pragma unroll 1
     for (int i = 0; i < 5; i++) atomicAdd(&A.ev[i], (unsigned long long)ws.ev[i]);
   }

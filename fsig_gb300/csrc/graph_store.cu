@@ -447,7 +447,7 @@ constexpr uint32_t kFilterRun = 256;
 __global__ void __launch_bounds__(256) membership_filter_kernel(
     const uint32_t* __restrict__ off, const uint32_t* __restrict__ adj, const int32_t* __restrict__ label,
     const uint32_t* __restrict__ base, const uint32_t* __restrict__ lseg, uint32_t V, int32_t L, uint32_t nadj,
-    uint32_t* __restrict__ filt) {
+    uint32_t shift, uint32_t* __restrict__ filt) {
   const uint32_t lane = threadIdx.x & 31;
   const uint64_t nwarps = (uint64_t(gridDim.x) * blockDim.x) >> 5;
   for (uint64_t run = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; run * kFilterRun < nadj; run += nwarps) {
@@ -479,8 +479,8 @@ __global__ void __launch_bounds__(256) membership_filter_kernel(
         b = lower_bound_u32(adj, k, off[v + 1], base[l + 1]);
       }
       const uint32_t first_id = base[l] & ~31u, rel = x - first_id;
-      const bool dense = b - a >= filter_dense_len(base[l + 1] - first_id);
-      const uint32_t w = a + filter_word(dense, rel, filter_hash(x), b - a);
+      const bool dense = b - a >= filter_dense_len(base[l + 1] - first_id, shift);
+      const uint32_t w = (a << shift) + filter_word(dense, rel, filter_hash(x), (b - a) << shift);
       atomicOr(&filt[w >> 1], filter_mask(dense, rel, filter_bits(x)) << ((w & 1u) * 16));
     }
   }
@@ -587,11 +587,13 @@ constexpr uint64_t kFilterSpare = 1ull << 30;
 int build_membership_filter(Engine& e, DeviceGraph& g) {
   g.filt = nullptr;
   if (!g.nadj) return FSIG_OK;
-  uint32_t* filt = e.arena.take_tail<uint32_t>((g.nadj + 1) / 2, kFilterSpare);
+  const uint32_t shift = filter_shift(g.nadj);
+  const uint64_t words32 = ((g.nadj << shift) + 1) / 2;
+  uint32_t* filt = e.arena.take_tail<uint32_t>(words32, kFilterSpare);
   if (!filt) return FSIG_OK;
-  FSIG_CUDA_TRY(cudaMemsetAsync(filt, 0, sizeof(uint32_t) * ((g.nadj + 1) / 2), e.stream));
+  FSIG_CUDA_TRY(cudaMemsetAsync(filt, 0, sizeof(uint32_t) * words32, e.stream));
   membership_filter_kernel<<<grid_for((g.nadj + kFilterRun - 1) / kFilterRun * 32, 256, e.num_sms), 256, 0, e.stream>>>(
-      g.off, g.adj, g.label, g.base, g.lseg, g.V, g.L, uint32_t(g.nadj), filt);
+      g.off, g.adj, g.label, g.base, g.lseg, g.V, g.L, uint32_t(g.nadj), shift, filt);
   FSIG_CUDA_TRY(cudaGetLastError());
   g.filt = reinterpret_cast<uint16_t*>(filt);
   return FSIG_OK;

@@ -33,6 +33,7 @@ struct GraphView {
   const uint32_t* __restrict__ adj_old;  // null when lseg is
   const uint32_t* __restrict__ base;     // [L+1] first id of each label class
   const uint16_t* __restrict__ filt;     // membership filter, or null
+  uint32_t fshift;                       // its words per entry, as a shift
 };
 
 namespace {
@@ -40,7 +41,8 @@ namespace {
 constexpr uint32_t kFull = 0xffffffffu;
 
 GraphView view_of(const DeviceGraph& g) {
-  return GraphView{g.V, g.L, g.label, g.off, g.adj, g.lseg, g.sig, g.old_of_new, g.adj_old, g.base, g.filt};
+  return GraphView{g.V, g.L, g.label, g.off, g.adj, g.lseg, g.sig, g.old_of_new, g.adj_old, g.base, g.filt,
+                   filter_shift(g.nadj)};
 }
 
 // Segment [lo, hi) of row v's neighbours with label l (0 <= l < L), from the
