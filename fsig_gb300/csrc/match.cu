@@ -188,13 +188,20 @@ __global__ void __launch_bounds__(kFilterWarps * 32, 8) filter_kernel(GraphView 
 // MMatch_kernels.cuh:28-117, 190-214) with its per-class thresholds.  With
 // every vertex its own class every k is one.  A class dominated by u's (dom)
 // is tested first: C(u) stays within C(dom) through the refinement, so a v
-// outside C(dom) fails one of the counts anyway.  Warps take runs of bitmap
-// words (lane = candidate); class members other than the smallest own no
-// words.  A candidate's segment of at most coop_min entries is scanned by its
-// own lane; a longer one by the whole warp, 32 consecutive entries per step
-// (coalesced loads, one ballot per step), one such candidate after another.
+// outside C(dom) fails one of the counts anyway.  Warps take bitmap words one
+// by one (lane = candidate), neighbouring words on different warps; class
+// members other than the smallest own no words.  A candidate's segment of at
+// most coop_min entries is scanned by its own lane; of a longer one the lane
+// tries the first kRefineOwn, which settle most candidates, and the whole warp
+// scans the rest, 32 consecutive entries per step (coalesced loads, one ballot
+// per step), one such candidate after another.
+// Bound by dependent gathers.  (In runs of eight words a warp got a label's hubs
+// together, all low ids on a power-law graph: on 2^26 edges, 37 queries, 14 of 64
+// warps were busy on average and a step took 2.36 ms; word by word 0.9 ms, and
+// with the lanes trying first 0.5 ms.)
 // ---------------------------------------------------------------------------
-constexpr uint32_t kRefineRun = 8;
+
+constexpr uint32_t kRefineOwn = 16;  // entries of a long segment that the candidate's own lane tries first (4-32: alike)
 
 __global__ void __launch_bounds__(256) refine_kernel(GraphView g, const QVert* __restrict__ qv, uint32_t G,
                                                      const uint64_t* __restrict__ gword, uint64_t total_words,
@@ -202,78 +209,76 @@ __global__ void __launch_bounds__(256) refine_kernel(GraphView g, const QVert* _
                                                      uint32_t coop_min) {
   const uint32_t lane = threadIdx.x & 31;
   const uint64_t nwt = (uint64_t(gridDim.x) * blockDim.x) >> 5;
-  for (uint64_t run = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; run * kRefineRun < total_words;
-       run += nwt) {
-    uint64_t W = run * kRefineRun;
-    const uint64_t Wend = min(W + kRefineRun, total_words);
-    // query vertex owning word W: last g with gword[g] <= W
-    uint32_t lo = 0, hi = G;
-    while (hi - lo > 1) {
-      uint32_t mid = (lo + hi) >> 1;
-      if (gword[mid] <= W) lo = mid; else hi = mid;
+  uint32_t gi = 0;  // query vertex owning word W: the last one with gword <= W
+  for (uint64_t W = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; W < total_words; W += nwt) {
+    {
+      uint32_t step = 1;
+      while (gi + step < G && gword[gi + step] <= W) {
+        gi += step;
+        step <<= 1;
+      }
+      for (; step; step >>= 1)
+        if (gi + step < G && gword[gi + step] <= W) gi += step;
     }
-    uint32_t gi = lo;
-    for (; W < Wend; W++) {
-      while (gword[gi + 1] <= W) gi++;
-      const QVert* q = qv + gi;
-      const uint32_t word = src[W];
-      if (word == 0 || q->adj == 0) {
-        if (lane == 0) dst[W] = word;
+    const QVert* q = qv + gi;
+    const uint32_t word = src[W];
+    if (word == 0 || q->adj == 0) {
+      if (lane == 0) dst[W] = word;
+      continue;
+    }
+    const uint32_t bit0 = uint32_t((W - q->bmoff) << 5) + lane;  // bit of v in every bitmap of u's label
+    const uint32_t v = q->bmbase + bit0;
+    bool alive = (word >> lane) & 1u;
+    const uint32_t gbase = gi - q->u;
+    if (q->dom != kNoClass) {
+      const QVert* qd = qv + gbase + q->dom;
+      alive = alive && ((src[qd->bmoff + (bit0 >> 5)] >> (bit0 & 31)) & 1u);
+    }
+    uint32_t m = q->adj;
+    while (m && __any_sync(kFull, alive)) {
+      const uint32_t wv = __ffs(m) - 1;
+      const QVert* qw = qv + gbase + wv;
+      const uint32_t grp = m & qw->cmask;
+      m &= ~grp;
+      const uint32_t need = __popc(grp);
+      if (qw->words == 0) {  // no data vertex carries the neighbour's label
+        alive = false;
         continue;
       }
-      const uint32_t bit0 = uint32_t((W - q->bmoff) << 5) + lane;  // bit of v in every bitmap of u's label
-      const uint32_t v = q->bmbase + bit0;
-      bool alive = (word >> lane) & 1u;
-      const uint32_t gbase = gi - q->u;
-      if (q->dom != kNoClass) {
-        const QVert* qd = qv + gbase + q->dom;
-        alive = alive && ((src[qd->bmoff + (bit0 >> 5)] >> (bit0 & 31)) & 1u);
-      }
-      uint32_t m = q->adj;
-      while (m && __any_sync(kFull, alive)) {
-        const uint32_t wv = __ffs(m) - 1;
-        const QVert* qw = qv + gbase + wv;
-        const uint32_t grp = m & qw->cmask;
-        m &= ~grp;
-        const uint32_t need = __popc(grp);
-        if (qw->words == 0) {  // no data vertex carries the neighbour's label
-          alive = false;
-          continue;
-        }
-        const uint32_t* __restrict__ nb = src + qw->bmoff;
-        const uint32_t nbase = qw->bmbase;
-        uint32_t k = 0, e = 0;
-        if (alive) segment_of(g, v, qw->label, k, e);
-        const bool coop = alive && e - k > coop_min;
-        if (alive && !coop) {
-          uint32_t have = 0;
-          for (; k < e && have < need; k++) {
-            const uint32_t bit = g.adj[k] - nbase;
-            have += (nb[bit >> 5] >> (bit & 31)) & 1u;
-          }
-          alive = have >= need;
-        }
-        uint32_t cm = __ballot_sync(kFull, coop);
-        while (cm) {
-          const uint32_t c = __ffs(cm) - 1;
-          cm &= cm - 1;
-          const uint32_t ck = __shfl_sync(kFull, k, c), ce = __shfl_sync(kFull, e, c);
-          uint32_t have = 0;
-          for (uint32_t p = ck; p < ce && have < need; p += 32) {
-            const uint32_t idx = p + lane;
-            bool hit = false;
-            if (idx < ce) {
-              const uint32_t bit = g.adj[idx] - nbase;
-              hit = (nb[bit >> 5] >> (bit & 31)) & 1u;
-            }
-            have += __popc(__ballot_sync(kFull, hit));
-          }
-          if (lane == c) alive = have >= need;
+      const uint32_t* __restrict__ nb = src + qw->bmoff;
+      const uint32_t nbase = qw->bmbase;
+      uint32_t k = 0, e = 0;
+      if (alive) segment_of(g, v, qw->label, k, e);
+      uint32_t own = 0;  // supporters found by the lane alone
+      if (alive) {
+        const uint32_t stop = e - k > coop_min ? min(k + kRefineOwn, e) : e;
+        for (; k < stop && own < need; k++) {
+          const uint32_t bit = g.adj[k] - nbase;
+          own += (nb[bit >> 5] >> (bit & 31)) & 1u;
         }
       }
-      const uint32_t nw = __ballot_sync(kFull, alive);
-      if (lane == 0) dst[W] = nw;
+      const bool coop = alive && own < need && k < e;
+      alive = alive && own >= need;
+      uint32_t cm = __ballot_sync(kFull, coop);
+      while (cm) {
+        const uint32_t c = __ffs(cm) - 1;
+        cm &= cm - 1;
+        const uint32_t ck = __shfl_sync(kFull, k, c), ce = __shfl_sync(kFull, e, c);
+        uint32_t have = __shfl_sync(kFull, own, c);
+        for (uint32_t p = ck; p < ce && have < need; p += 32) {
+          const uint32_t idx = p + lane;
+          bool hit = false;
+          if (idx < ce) {
+            const uint32_t bit = g.adj[idx] - nbase;
+            hit = (nb[bit >> 5] >> (bit & 31)) & 1u;
+          }
+          have += __popc(__ballot_sync(kFull, hit));
+        }
+        if (lane == c) alive = have >= need;
+      }
     }
+    const uint32_t nw = __ballot_sync(kFull, alive);
+    if (lane == 0) dst[W] = nw;
   }
 }
 
@@ -667,8 +672,7 @@ int filter_stage(Engine& e, const BatchLayout& b, uint32_t mode, int refine_iter
   uint32_t* cur = p0;
   uint32_t* nxt = p1;
   for (int it = 0; it < refine_iters && b.words; it++) {
-    const uint64_t runs = (b.words + kRefineRun - 1) / kRefineRun;
-    refine_kernel<<<grid_cap(runs * 32, 256, e.num_sms, 16), 256, 0, s>>>(gv, d_qv, b.G, d_gword, b.words, cur, nxt,
+    refine_kernel<<<grid_cap(b.words * 32, 256, e.num_sms, 64), 256, 0, s>>>(gv, d_qv, b.G, d_gword, b.words, cur, nxt,
                                                                            coop_min);
     FSIG_CUDA_TRY(cudaGetLastError());
     std::swap(cur, nxt);
