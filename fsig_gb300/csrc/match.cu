@@ -461,12 +461,17 @@ __global__ void __launch_bounds__(256) roots_kernel(const QVert* __restrict__ qv
 }
 
 // Number of pass-0 tasks per root: its depth-1 driver range in chunks of
-// `split` entries (at least one task per root, so every root is counted).
+// `split` entries (at least one task per root, so every root is counted); 0 in
+// the slots past the last root.
 __global__ void root_chunks_kernel(GraphView g, const Plan* __restrict__ plans, const uint32_t* __restrict__ roots,
                                    const uint32_t* __restrict__ root_q, const uint32_t* __restrict__ total_roots,
-                                   uint32_t split, uint32_t* chunks) {
+                                   uint32_t split, uint64_t slots, uint32_t* chunks) {
   const uint32_t nr = *total_roots;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nr; i += gridDim.x * blockDim.x) {
+  for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < slots; i += uint64_t(gridDim.x) * blockDim.x) {
+    if (i >= nr) {
+      chunks[i] = 0;
+      continue;
+    }
     const Plan* p = plans + root_q[i];
     uint32_t c = 1;
     if (p->n > 1) {
@@ -774,7 +779,6 @@ struct EnumRun {
   EnumArgs A;
   TaskRec *out = nullptr, *other = nullptr;
   uint32_t *ready = nullptr, *other_ready = nullptr, *ctr = nullptr;
-  unsigned long long* d_ev = nullptr;
   uint32_t* h_ctr = nullptr;  // pinned, 4 counters kCtrStride apart
   uint32_t grid = 0, block = 0, active = 0, first_task = 0, pass = 0;
   size_t smem = 0;
@@ -806,18 +810,15 @@ int enum_configure(Engine& e) {
 int enum_prepare(Engine& e, const BatchOptions& opt, const GraphView& gv, const Plan* d_plans, const uint32_t* pool,
                  uint32_t Q, const uint32_t* d_roots, const uint32_t* d_root_q, const uint32_t* d_chunk_off,
                  const uint32_t* d_nroots, uint32_t split, QueryResult* d_res, unsigned long long* d_misc,
-                 uint32_t* d_emit, unsigned long long* d_emit_ctr, uint32_t* h_ctr, EnumRun& R) {
-  cudaStream_t s = e.stream;
+                 unsigned long long* d_ev, uint32_t* d_emit, unsigned long long* d_emit_ctr, uint32_t* h_ctr,
+                 EnumRun& R) {
   TaskRec* qa = e.arena.take<TaskRec>(kOverflowCap);
   TaskRec* qb = e.arena.take<TaskRec>(kOverflowCap);
   uint32_t* ra = e.arena.take<uint32_t>(kOverflowCap);
   uint32_t* rb = e.arena.take<uint32_t>(kOverflowCap);
   R.ctr = e.arena.take<uint32_t>(8 * kCtrStride);
-  R.d_ev = e.arena.take<unsigned long long>(8);
-  if (!qa || !qb || !ra || !rb || !R.ctr || !R.d_ev)
+  if (!qa || !qb || !ra || !rb || !R.ctr)
     return fail(FSIG_EADMISSION, "work queues do not fit the device arena");
-  FSIG_CUDA_TRY(cudaMemsetAsync(R.d_ev, 0, 64, s));
-  FSIG_CUDA_TRY(cudaMemsetAsync(d_misc + 1, 0, sizeof(unsigned long long), s));
   const uint32_t wpb = std::max<uint32_t>(1, std::min<uint32_t>(opt.warps_per_block, kEnumWarps));
   const int per_sm = gv.lseg ? e.enum_per_sm[wpb] : e.enum_per_sm_rows[wpb];
   R.smem = sizeof(WarpSmem) * wpb;
@@ -852,8 +853,8 @@ int enum_prepare(Engine& e, const BatchOptions& opt, const GraphView& gv, const 
   A.budget = (long long)opt.budget_cycles;
   A.res = d_res;
   A.work_cap = opt.max_work;
-  A.algo_bytes = d_misc + 1;
-  A.ev = R.d_ev;
+  A.algo_bytes = d_misc;
+  A.ev = d_ev;
   A.seed = FSIG_HASH_SEED;
   A.ready_wait_ns = e.ready_wait_ns;
   A.idle_wait_ns = e.idle_wait_ns;
@@ -933,26 +934,34 @@ int reserve_pinned(Engine& e, size_t bytes) {
   return FSIG_OK;
 }
 
-template <class T>
-T* stage_upload(Engine& e, Stage& st, const std::vector<T>& v, int& rc) {
-  T* d = e.arena.take<T>(std::max<size_t>(v.size(), 1));
-  if (!d) { rc = fail(FSIG_EADMISSION, "batch does not fit the device arena"); return nullptr; }
-  T* h = st.take<T>(v.size());
-  if (!v.empty()) {
-    std::memcpy(h, v.data(), sizeof(T) * v.size());
-    cudaError_t err = cudaMemcpyAsync(d, h, sizeof(T) * v.size(), cudaMemcpyHostToDevice, e.stream);
-    if (err != cudaSuccess) { rc = fail_cuda(err, "cudaMemcpyAsync", __FILE__, __LINE__); return nullptr; }
-    e.cur_h2d += sizeof(T) * v.size();
+// Parts of one device block and its image in the staging area, each part at a
+// multiple of 256 bytes.  One copy moves the whole block (seven uploads and six
+// downloads of a call each cost 2-3 us, more than their bytes).
+struct Block {
+  uint64_t bytes = 0;
+  uint8_t *dev = nullptr, *host = nullptr;
+  uint64_t add(uint64_t n) {
+    const uint64_t at = bytes;
+    bytes += (std::max<uint64_t>(n, 1) + 255) & ~uint64_t(255);
+    return at;
   }
-  return d;
+  template <class T>
+  T* d(uint64_t at) const { return reinterpret_cast<T*>(dev + at); }
+  template <class T>
+  T* h(uint64_t at) const { return reinterpret_cast<T*>(host + at); }
+};
+
+template <class T>
+void fill_part(const Block& k, uint64_t at, const std::vector<T>& v) {
+  if (!v.empty()) std::memcpy(k.h<T>(at), v.data(), sizeof(T) * v.size());
 }
 
 size_t stage_bytes(const BatchLayout& b) {
   const size_t a = 256;
   const size_t Q = b.Q, G = b.G;
-  return 20 * a + sizeof(QVert) * G + 4 * (Q + 1) + 4 * b.lab_gidx.size() + 4 * b.lab_begin.size() +
-         8 * b.gword.size() + 4 * G + 4 * G + 4 * Q + sizeof(QueryResult) * Q + 4 * G + 4 * Q * kMaxQ + sizeof(Plan) * Q +
-         8 + 4 * 4 * kCtrStride + 64;
+  return 24 * a + sizeof(QVert) * G + 4 * (Q + 1) + 4 * b.lab_gidx.size() + 4 * b.lab_begin.size() +
+         8 * b.gword.size() + 4 * G + 4 * G + 4 * Q + sizeof(QueryResult) * Q + 4 * G + 4 * Q * kMaxQ + 8 + 64 +
+         4 * 4 * kCtrStride;
 }
 }  // namespace
 
@@ -1010,51 +1019,57 @@ int run_batch(Engine& e, const std::vector<HostQuery>& qs, const BatchOptions& o
 
   cudaGraph_t cg = nullptr;
   if (graph) FSIG_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed));
-  QueryResult* h_res = nullptr;
-  uint32_t *h_counts = nullptr, *h_orders = nullptr, *d_chunk_off = nullptr, *d_rootoff = nullptr;
-  Plan* h_plans = nullptr;
-  unsigned long long* h_misc = nullptr;
-  unsigned long long* h_ev = nullptr;
-  QueryResult* d_res = nullptr;
-  unsigned long long* d_misc = nullptr;
-  Plan* d_plans = nullptr;
-  uint32_t *d_counts = nullptr, *d_orders = nullptr, *d_emit = nullptr;
+  Block in, res;  // the call's inputs; its results
+  uint64_t at_res = 0, at_counts = 0, at_orders = 0, at_misc = 0, at_ev = 0, res_bytes = 0;
+  uint32_t* d_chunk_off = nullptr;
+  uint32_t* d_rootoff = nullptr;
+  uint32_t* d_emit = nullptr;
   unsigned long long* d_emit_ctr = nullptr;
 
   // Everything from the uploads to the results' copy back, in stream order.
   auto enqueue = [&]() -> int {
     int rc = FSIG_OK;
     FSIG_CUDA_TRY(record(e.ev[0], s));
-    QVert* d_qv = stage_upload(e, st, b.qv, rc);
-    if (rc) return rc;
-    uint32_t* d_qoff = stage_upload(e, st, b.qoff, rc);
-    if (rc) return rc;
-    uint32_t* d_lab_gidx = stage_upload(e, st, b.lab_gidx, rc);
-    if (rc) return rc;
-    uint32_t* d_lab_begin = stage_upload(e, st, b.lab_begin, rc);
-    if (rc) return rc;
-    uint64_t* d_gword = stage_upload(e, st, b.gword, rc);
-    if (rc) return rc;
-    uint32_t* d_given = stage_upload(e, st, given, rc);
-    if (rc) return rc;
-    float* d_scores = stage_upload(e, st, scores, rc);
-    if (rc) return rc;
-    d_counts = e.arena.take<uint32_t>(std::max<uint32_t>(b.G, 1));
-    d_plans = e.arena.take<Plan>(Q);
-    uint32_t* d_rootcnt = e.arena.take<uint32_t>(uint64_t(Q) + 1);
+    const uint64_t at_qv = in.add(sizeof(QVert) * b.G), at_qoff = in.add(4 * b.qoff.size()),
+                   at_gidx = in.add(4 * b.lab_gidx.size()), at_begin = in.add(4 * b.lab_begin.size()),
+                   at_gword = in.add(8 * b.gword.size()), at_given = in.add(4 * given.size()),
+                   at_scores = in.add(4 * scores.size()), at_has = in.add(4 * has_given.size());
+    in.dev = e.arena.take<uint8_t>(in.bytes);
+    if (!in.dev) return fail(FSIG_EADMISSION, "batch does not fit the device arena");
+    in.host = st.take<uint8_t>(in.bytes);
+    fill_part(in, at_qv, b.qv);
+    fill_part(in, at_qoff, b.qoff);
+    fill_part(in, at_gidx, b.lab_gidx);
+    fill_part(in, at_begin, b.lab_begin);
+    fill_part(in, at_gword, b.gword);
+    fill_part(in, at_given, given);
+    fill_part(in, at_scores, scores);
+    fill_part(in, at_has, has_given);
+    FSIG_CUDA_TRY(cudaMemcpyAsync(in.dev, in.host, in.bytes, cudaMemcpyHostToDevice, s));
+    e.cur_h2d += in.bytes;
+    QVert* d_qv = in.d<QVert>(at_qv);
+    uint32_t* d_qoff = in.d<uint32_t>(at_qoff);
+    uint32_t *d_lab_gidx = in.d<uint32_t>(at_gidx), *d_lab_begin = in.d<uint32_t>(at_begin);
+    uint64_t* d_gword = in.d<uint64_t>(at_gword);
+    uint32_t* d_given = in.d<uint32_t>(at_given);
+    float* d_scores = in.d<float>(at_scores);
+    // results, counters and root counts start at zero; the results come back by one copy
+    at_res = res.add(sizeof(QueryResult) * Q);
+    at_counts = res.add(4 * uint64_t(b.G));
+    at_orders = res.add(4 * uint64_t(Q) * kMaxQ);
+    at_misc = res.add(sizeof(unsigned long long));
+    at_ev = res.add(sizeof(e.last_ev));
+    res_bytes = res.bytes;
+    const uint64_t at_rootcnt = res.add(4 * (uint64_t(Q) + 1));
+    res.dev = e.arena.take<uint8_t>(res.bytes);
+    Plan* d_plans = e.arena.take<Plan>(Q);
     d_rootoff = e.arena.take<uint32_t>(uint64_t(Q) + 1);
-    d_orders = e.arena.take<uint32_t>(uint64_t(Q) * kMaxQ);
-    d_res = e.arena.take<QueryResult>(Q);
-    d_misc = e.arena.take<unsigned long long>(4);  // [1] modelled bytes
-    if (!d_counts || !d_plans || !d_rootcnt || !d_rootoff || !d_orders || !d_res || !d_misc)
-      return fail(FSIG_EADMISSION, "batch does not fit the device arena");
-    h_res = st.take<QueryResult>(Q);
-    h_counts = st.take<uint32_t>(b.G);
-    h_orders = st.take<uint32_t>(size_t(Q) * kMaxQ);
-    h_plans = st.take<Plan>(Q);
-    h_misc = st.take<unsigned long long>(1);
+    if (!res.dev || !d_plans || !d_rootoff) return fail(FSIG_EADMISSION, "batch does not fit the device arena");
+    res.host = st.take<uint8_t>(res_bytes);
     uint32_t* h_ctr = st.take<uint32_t>(4 * kCtrStride);
-    h_ev = st.take<unsigned long long>(8);
+    FSIG_CUDA_TRY(cudaMemsetAsync(res.dev, 0, res.bytes, s));
+    uint32_t *d_counts = res.d<uint32_t>(at_counts), *d_orders = res.d<uint32_t>(at_orders);
+    uint32_t* d_rootcnt = res.d<uint32_t>(at_rootcnt);
 
     uint32_t* pool = nullptr;
     rc = filter_stage(e, b, opt.filter_mode, opt.refine_iters, d_qv, d_gword, d_lab_gidx, d_lab_begin, pool,
@@ -1065,8 +1080,10 @@ int run_batch(Engine& e, const std::vector<HostQuery>& qs, const BatchOptions& o
     uint32_t order_mode = opt.order_mode;
     if (opt.host_order) {
       // Reference-exact orders are computed on the host from the counts.
-      FSIG_CUDA_TRY(cudaMemcpyAsync(out.counts.data(), d_counts, sizeof(uint32_t) * b.G, cudaMemcpyDeviceToHost, s));
+      FSIG_CUDA_TRY(cudaMemcpyAsync(res.h<uint32_t>(at_counts), d_counts, sizeof(uint32_t) * b.G,
+                                    cudaMemcpyDeviceToHost, s));
       FSIG_CUDA_TRY(cudaStreamSynchronize(s));
+      std::memcpy(out.counts.data(), res.h<uint32_t>(at_counts), sizeof(uint32_t) * b.G);
       d2h += sizeof(uint32_t) * b.G;
       for (uint32_t q = 0; q < Q; q++) {
         bool any_zero = false;
@@ -1082,7 +1099,9 @@ int run_batch(Engine& e, const std::vector<HostQuery>& qs, const BatchOptions& o
         }
         opt.host_order(qs[q], out.counts.data() + b.qoff[q], given.data() + b.qoff[q]);
       }
-      FSIG_CUDA_TRY(cudaMemcpyAsync(d_given, given.data(), sizeof(uint32_t) * b.G, cudaMemcpyHostToDevice, s));
+      fill_part(in, at_given, given);
+      FSIG_CUDA_TRY(cudaMemcpyAsync(d_given, in.h<uint32_t>(at_given), sizeof(uint32_t) * b.G, cudaMemcpyHostToDevice,
+                                    s));
       e.cur_h2d += sizeof(uint32_t) * b.G;
       order_mode = kOrderGiven;
     }
@@ -1109,10 +1128,8 @@ int run_batch(Engine& e, const std::vector<HostQuery>& qs, const BatchOptions& o
         launches++;
       }
       if (any_given) {
-        uint32_t* d_has_given = stage_upload(e, st, has_given, rc);
-        if (rc) return rc;
-        given_scores_kernel<<<std::max<uint32_t>(1, (Q + 127) / 128), 128, 0, s>>>(d_qoff, Q, d_has_given, d_given,
-                                                                                 d_lscores);
+        given_scores_kernel<<<std::max<uint32_t>(1, (Q + 127) / 128), 128, 0, s>>>(d_qoff, Q, in.d<uint32_t>(at_has),
+                                                                                 d_given, d_lscores);
         FSIG_CUDA_TRY(cudaGetLastError());
         launches++;
       }
@@ -1125,7 +1142,6 @@ int run_batch(Engine& e, const std::vector<HostQuery>& qs, const BatchOptions& o
     d_chunk_off = e.arena.take<uint32_t>(b.root_cap + 1);
     if (!d_roots || !d_root_q || !d_chunks || !d_chunk_off)
       return fail(FSIG_EADMISSION, "root list does not fit the device arena");
-    FSIG_CUDA_TRY(cudaMemsetAsync(d_rootcnt, 0, sizeof(uint32_t) * (uint64_t(Q) + 1), s));
     order_kernel<<<(Q + 7) / 8, 256, 0, s>>>(d_qv, d_qoff, Q, d_counts, order_mode, d_score_src, d_given, d_plans,
                                              d_rootcnt, d_orders, opt.learned ? opt.learned_prefix : kMaxQ);
     FSIG_CUDA_TRY(cudaGetLastError());
@@ -1139,17 +1155,12 @@ int run_batch(Engine& e, const std::vector<HostQuery>& qs, const BatchOptions& o
     // on the number of roots (the count itself stays on the device).
     // (embedding output may cut the depth-1 ranges as finely as one entry)
     const uint32_t split = std::max<uint32_t>(opt.split, opt.emit_cap ? 1u : 32u);
-    FSIG_CUDA_TRY(cudaMemsetAsync(d_chunks, 0, sizeof(uint32_t) * (b.root_cap + 1), s));
-    if (b.root_cap) {
-      root_chunks_kernel<<<grid_cap(b.root_cap, 256, e.num_sms, 8), 256, 0, s>>>(view_of(g), d_plans, d_roots,
-                                                                                  d_root_q, d_rootoff + Q, split,
-                                                                                  d_chunks);
-      FSIG_CUDA_TRY(cudaGetLastError());
-      launches++;
-    }
+    root_chunks_kernel<<<grid_cap(b.root_cap + 1, 256, e.num_sms, 8), 256, 0, s>>>(
+        view_of(g), d_plans, d_roots, d_root_q, d_rootoff + Q, split, b.root_cap + 1, d_chunks);
+    FSIG_CUDA_TRY(cudaGetLastError());
+    launches++;
     rc = device_exclusive_scan<uint32_t>(e.arena, d_chunks, d_chunk_off, b.root_cap + 1, nullptr, s, &launches);
     if (rc) return rc;
-    FSIG_CUDA_TRY(cudaMemsetAsync(d_res, 0, sizeof(QueryResult) * Q, s));
     if (opt.emit_cap) {
       d_emit_ctr = e.arena.take<unsigned long long>(1);
       d_emit = e.arena.take<uint32_t>(opt.emit_cap * qs[0].n);
@@ -1157,19 +1168,15 @@ int run_batch(Engine& e, const std::vector<HostQuery>& qs, const BatchOptions& o
       FSIG_CUDA_TRY(cudaMemsetAsync(d_emit_ctr, 0, sizeof(unsigned long long), s));
     }
     rc = enum_prepare(e, opt, view_of(g), d_plans, pool, Q, d_roots, d_root_q, d_chunk_off, d_rootoff + Q, split,
-                      d_res, d_misc, d_emit, d_emit_ctr, h_ctr, R);
+                      res.d<QueryResult>(at_res), res.d<unsigned long long>(at_misc),
+                      res.d<unsigned long long>(at_ev), d_emit, d_emit_ctr, h_ctr, R);
     if (rc) return rc;
     return enum_launch(e, R);
   };
   // The results' copy back (after the last pass).
   auto copy_back = [&]() -> int {
     FSIG_CUDA_TRY(record(e.ev[2], s));
-    FSIG_CUDA_TRY(cudaMemcpyAsync(h_res, d_res, sizeof(QueryResult) * Q, cudaMemcpyDeviceToHost, s));
-    FSIG_CUDA_TRY(cudaMemcpyAsync(h_counts, d_counts, sizeof(uint32_t) * b.G, cudaMemcpyDeviceToHost, s));
-    FSIG_CUDA_TRY(cudaMemcpyAsync(h_orders, d_orders, sizeof(uint32_t) * Q * kMaxQ, cudaMemcpyDeviceToHost, s));
-    FSIG_CUDA_TRY(cudaMemcpyAsync(h_misc, d_misc + 1, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-    FSIG_CUDA_TRY(cudaMemcpyAsync(h_plans, d_plans, sizeof(Plan) * Q, cudaMemcpyDeviceToHost, s));
-    FSIG_CUDA_TRY(cudaMemcpyAsync(h_ev, R.d_ev, sizeof(e.last_ev), cudaMemcpyDeviceToHost, s));
+    FSIG_CUDA_TRY(cudaMemcpyAsync(res.host, res.dev, res_bytes, cudaMemcpyDeviceToHost, s));
     return FSIG_OK;
   };
 
@@ -1224,7 +1231,9 @@ int run_batch(Engine& e, const std::vector<HostQuery>& qs, const BatchOptions& o
       FSIG_CUDA_TRY(cudaStreamSynchronize(s));
     }
   } else {
+    // the results come back right behind the first pass; after another one again
     rc = enqueue();
+    if (!rc) rc = copy_back();
     if (rc) {
       // work queued before the failure still reads the staging area and the
       // arena: let it finish before they are reused
@@ -1238,6 +1247,7 @@ int run_batch(Engine& e, const std::vector<HostQuery>& qs, const BatchOptions& o
       if (rc) return rc;
       if (more) {
         rc = enum_launch(e, R);
+        if (!rc) rc = copy_back();
         if (rc) return rc;
       }
     } while (more);
@@ -1257,19 +1267,21 @@ int run_batch(Engine& e, const std::vector<HostQuery>& qs, const BatchOptions& o
       if (rows)
         FSIG_CUDA_TRY(cudaMemcpyAsync(out.rows.data(), d_emit, sizeof(uint32_t) * rows * qs[0].n,
                                       cudaMemcpyDeviceToHost, s));
+      FSIG_CUDA_TRY(cudaStreamSynchronize(s));
       d2h += 8 + sizeof(uint32_t) * rows * qs[0].n;
     }
-    rc = copy_back();
-    if (rc) return rc;
-    FSIG_CUDA_TRY(cudaStreamSynchronize(s));
   }
   launches += out.passes * 2;  // counter reset + enumeration per pass
-  std::memcpy(out.res.data(), h_res, sizeof(QueryResult) * Q);
-  std::memcpy(out.counts.data(), h_counts, sizeof(uint32_t) * b.G);
-  std::memcpy(out.orders.data(), h_orders, sizeof(uint32_t) * Q * kMaxQ);
-  std::memcpy(e.last_ev, h_ev, sizeof(e.last_ev));
-  out.algo_bytes = *h_misc;
-  for (uint32_t q = 0; q < Q; q++) out.ok[q] = h_plans[q].ok;
+  std::memcpy(out.res.data(), res.h<QueryResult>(at_res), sizeof(QueryResult) * Q);
+  std::memcpy(out.counts.data(), res.h<uint32_t>(at_counts), sizeof(uint32_t) * b.G);
+  std::memcpy(out.orders.data(), res.h<uint32_t>(at_orders), sizeof(uint32_t) * Q * kMaxQ);
+  std::memcpy(e.last_ev, res.h<unsigned long long>(at_ev), sizeof(e.last_ev));
+  out.algo_bytes = *res.h<unsigned long long>(at_misc);
+  for (uint32_t q = 0; q < Q; q++) {  // Plan::ok: every vertex has a candidate
+    out.ok[q] = 1;
+    for (uint32_t i = b.qoff[q]; i < b.qoff[q + 1]; i++)
+      if (!out.counts[i]) out.ok[q] = 0;
+  }
   out.ms_filter = elapsed(e.ev[0], e.ev[1]);
   out.ms_join = elapsed(e.ev[1], e.ev[2]);
   if (out.ms_filter < 0.f || out.ms_join < 0.f) {
@@ -1278,8 +1290,7 @@ int run_batch(Engine& e, const std::vector<HostQuery>& qs, const BatchOptions& o
     out.ms_join = graph ? std::max(elapsed(e.ev_outer[0], e.ev_outer[1]), 0.f) : 0.f;
   }
   if (!R.timed) out.ms_enum = -1.f;
-  d2h += sizeof(QueryResult) * Q + sizeof(uint32_t) * b.G + sizeof(uint32_t) * Q * kMaxQ +
-         sizeof(unsigned long long) + sizeof(Plan) * Q + sizeof(e.last_ev);
+  d2h += res_bytes * out.passes;
   out.h2d_bytes = e.cur_h2d;
   out.d2h_bytes = d2h;
   out.launches = launches;
