@@ -140,7 +140,7 @@ constexpr uint32_t kBuf = 32;        // entries of a depth's buffer
 constexpr uint32_t kScratch = 384;   // words for the segments and earlier vertices of the entries being extended
 // Candidate windows one fill examines before it returns, so that the periodic
 // checks and hand-offs come in time on long driver ranges.
-constexpr uint32_t kFillWindows = 64;
+constexpr uint32_t kFillWindows = 96;
 // Windows between two checks of the work limit and of the waiting warps.
 constexpr uint32_t kCheckWindows = 32;
 
@@ -408,7 +408,8 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
     const uint32_t bwd = ws.plan.bwd[lv], inj = ws.plan.same[lv] & ~bwd;
     const int32_t lab = ws.plan.lab[lv];
     const uint32_t nb = __popc(bwd), n4 = (__popc(inj) + 3) / 4;
-    const uint32_t stride = min(kBuf, kScratch / (2 * nb + 4 * n4));  // entries per group
+    const uint32_t words = 2 * nb + 4 * n4;
+    const uint32_t stride = words <= kScratch / kBuf ? kBuf : kScratch / words;  // entries per group
     uint4* const other = reinterpret_cast<uint4*>(ws.scratch);  // [n4][stride], padded with kInvalid
     uint2* const segs = ws.scratch + 2 * n4 * stride;           // [nb][stride]
     // whether x is none of entry c's earlier vertices
@@ -425,7 +426,8 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
     const uint32_t* __restrict__ bm = A.pool + ws.plan.bmoff[lv];
     // segments are kept in units of their filter's words; from `dense` on it is exact
     const uint32_t fs = g.filt ? g.fshift : 0;
-    const uint32_t dense = g.filt ? filter_dense_len(__ldg(g.base + lab + 1) - bmbase, fs) << fs : kInvalid;
+    const uint32_t dense =
+        nb > 1 && g.filt ? filter_dense_len(__ldg(g.base + lab + 1) - bmbase, fs) << fs : kInvalid;
     const uint32_t cntp = __shfl_sync(kFull, cnt, p), spp = __shfl_sync(kFull, sp, p);
     const uint32_t spl = spp + cntp;                              // depth lv's buffer
     const uint32_t room = min(kBuf, kPool - spl - (n - 2 - min(lv, n - 2)));
