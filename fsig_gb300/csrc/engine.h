@@ -3,6 +3,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+#include <cstring>
 #include <string>
 #include <vector>
 
@@ -71,6 +73,28 @@ struct Engine {
   uint32_t inject_unpublished = 0;         // test hook: leave each pass's first hand-off unpublished
 };
 
+// Parts of one device block and its image in the staging area, each part at a
+// multiple of 256 bytes.  One copy moves the whole block (seven uploads and six
+// downloads of a call each cost 2-3 us, more than their bytes).
+struct Block {
+  uint64_t bytes = 0;
+  uint8_t *dev = nullptr, *host = nullptr;
+  uint64_t add(uint64_t n) {
+    const uint64_t at = bytes;
+    bytes += (std::max<uint64_t>(n, 1) + 255) & ~uint64_t(255);
+    return at;
+  }
+  void fill(uint64_t at, const void* src, uint64_t n) const {
+    if (n) std::memcpy(host + at, src, n);
+  }
+  template <class T>
+  T* d(uint64_t at) const { return reinterpret_cast<T*>(dev + at); }
+  template <class T>
+  T* h(uint64_t at) const { return reinterpret_cast<T*>(host + at); }
+};
+
+// match.cu: at least this much page-locked staging (Engine::pinned).
+int reserve_pinned(Engine& e, size_t bytes);
 // graph_store.cu
 int build_device_graph(Engine& e, uint32_t V, const int32_t* labels, uint64_t E, const uint32_t* edges);
 bool use_segment_table(int mode, uint32_t V, int32_t L, uint64_t nadj);

@@ -923,37 +923,9 @@ struct Stage {
   }
 };
 
-int reserve_pinned(Engine& e, size_t bytes) {
-  if (e.pinned_bytes >= bytes) return FSIG_OK;
-  if (e.pinned) cudaFreeHost(e.pinned);
-  e.pinned = nullptr;
-  e.pinned_bytes = 0;
-  const size_t want = std::max<size_t>(bytes + bytes / 4, size_t(1) << 20);
-  FSIG_CUDA_TRY(cudaHostAlloc(&e.pinned, want, cudaHostAllocDefault));
-  e.pinned_bytes = want;
-  return FSIG_OK;
-}
-
-// Parts of one device block and its image in the staging area, each part at a
-// multiple of 256 bytes.  One copy moves the whole block (seven uploads and six
-// downloads of a call each cost 2-3 us, more than their bytes).
-struct Block {
-  uint64_t bytes = 0;
-  uint8_t *dev = nullptr, *host = nullptr;
-  uint64_t add(uint64_t n) {
-    const uint64_t at = bytes;
-    bytes += (std::max<uint64_t>(n, 1) + 255) & ~uint64_t(255);
-    return at;
-  }
-  template <class T>
-  T* d(uint64_t at) const { return reinterpret_cast<T*>(dev + at); }
-  template <class T>
-  T* h(uint64_t at) const { return reinterpret_cast<T*>(host + at); }
-};
-
 template <class T>
 void fill_part(const Block& k, uint64_t at, const std::vector<T>& v) {
-  if (!v.empty()) std::memcpy(k.h<T>(at), v.data(), sizeof(T) * v.size());
+  k.fill(at, v.data(), sizeof(T) * v.size());
 }
 
 size_t stage_bytes(const BatchLayout& b) {
@@ -964,6 +936,17 @@ size_t stage_bytes(const BatchLayout& b) {
          4 * 4 * kCtrStride;
 }
 }  // namespace
+
+int reserve_pinned(Engine& e, size_t bytes) {
+  if (e.pinned_bytes >= bytes) return FSIG_OK;
+  if (e.pinned) cudaFreeHost(e.pinned);
+  e.pinned = nullptr;
+  e.pinned_bytes = 0;
+  const size_t want = std::max<size_t>(bytes + bytes / 4, size_t(1) << 20);
+  FSIG_CUDA_TRY(cudaHostAlloc(&e.pinned, want, cudaHostAllocDefault));
+  e.pinned_bytes = want;
+  return FSIG_OK;
+}
 
 int run_batch(Engine& e, const std::vector<HostQuery>& qs, const BatchOptions& opt, BatchOutput& out) {
   if (!e.has_graph) return fail(FSIG_ENOGRAPH, "no data graph loaded");

@@ -443,7 +443,7 @@ int mpnn_init(Engine& e) {
   auto* M = new MpnnState();
   const size_t pb = sizeof(float) * kParams;
   // One-time state outside the arena (the arena is reset when a graph loads).
-  if (cudaMalloc(&M->master, pb) != cudaSuccess || cudaMalloc(&M->grad, pb) != cudaSuccess ||
+  if (cudaMalloc(&M->master, pb) != cudaSuccess || cudaMalloc(&M->grad, pb + sizeof(float)) != cudaSuccess ||
       cudaMalloc(&M->m1, pb) != cudaSuccess || cudaMalloc(&M->m2, pb) != cudaSuccess ||
       cudaMalloc(&M->wbf, sizeof(uint16_t) * kWBf) != cudaSuccess) {
     cudaFree(M->master);
@@ -523,29 +523,35 @@ int mpnn_run(Engine& e, uint32_t num_graphs, const uint32_t* goff, const float* 
     if (goff[q + 1] < goff[q] || goff[q + 1] - goff[q] > 32) return fail(FSIG_EINVAL, "graphs have 0..32 vertices");
   const uint32_t nodes = goff[num_graphs];
   const uint64_t mark = e.arena.mark();
-  uint32_t* d_goff = e.arena.take<uint32_t>(num_graphs + 1);
-  float* d_feat = e.arena.take<float>(std::max<uint64_t>(uint64_t(nodes) * kFeat, 1));
-  uint32_t* d_nbr = e.arena.take<uint32_t>(std::max<uint32_t>(nodes, 1));
+  // inputs and outputs in one block each, copied at once through the staging area
+  Block in, res;
+  const uint64_t at_goff = in.add(sizeof(uint32_t) * (uint64_t(num_graphs) + 1)),
+                 at_feat = in.add(sizeof(float) * uint64_t(nodes) * kFeat), at_nbr = in.add(sizeof(uint32_t) * nodes),
+                 at_target = in.add(target ? sizeof(float) * nodes : 0);
+  const uint64_t at_scores = scores ? res.add(sizeof(float) * nodes) : 0;
+  const uint64_t out_bytes = target ? sizeof(float) * (kParams + 1) : res.bytes;  // a step's gradients and loss are in M.grad
+  int rc = reserve_pinned(e, in.bytes + std::max<uint64_t>(out_bytes, 1));
+  if (rc) return rc;
+  in.host = static_cast<uint8_t*>(e.pinned);
+  res.host = in.host + in.bytes;
+  in.dev = e.arena.take<uint8_t>(in.bytes);
   float* d_scores = e.arena.take<float>(std::max<uint32_t>(nodes, 1));
-  float* d_target = target ? e.arena.take<float>(std::max<uint32_t>(nodes, 1)) : nullptr;
   uint16_t* d_acts = target ? e.arena.take<uint16_t>(std::max<uint64_t>(uint64_t(nodes) * kActW, 1)) : nullptr;
-  float* d_loss = e.arena.take<float>(1);
-  if (!d_goff || !d_feat || !d_nbr || !d_scores || !d_loss || (target && (!d_target || !d_acts))) {
+  if (!in.dev || !d_scores || (target && !d_acts)) {
     e.arena.release(mark);
     return fail(FSIG_EADMISSION, "order-network batch does not fit the arena");
   }
-  FSIG_CUDA_TRY(cudaMemcpyAsync(d_goff, goff, sizeof(uint32_t) * (num_graphs + 1), cudaMemcpyHostToDevice, s));
-  if (nodes) {
-    FSIG_CUDA_TRY(cudaMemcpyAsync(d_feat, feat, sizeof(float) * nodes * kFeat, cudaMemcpyHostToDevice, s));
-    FSIG_CUDA_TRY(cudaMemcpyAsync(d_nbr, nbr, sizeof(uint32_t) * nodes, cudaMemcpyHostToDevice, s));
-    if (target) FSIG_CUDA_TRY(cudaMemcpyAsync(d_target, target, sizeof(float) * nodes, cudaMemcpyHostToDevice, s));
-  }
-  int rc;
+  in.fill(at_goff, goff, sizeof(uint32_t) * (uint64_t(num_graphs) + 1));
+  in.fill(at_feat, feat, sizeof(float) * uint64_t(nodes) * kFeat);
+  in.fill(at_nbr, nbr, sizeof(uint32_t) * nodes);
+  if (target) in.fill(at_target, target, sizeof(float) * nodes);
+  FSIG_CUDA_TRY(cudaMemcpyAsync(in.dev, in.host, in.bytes, cudaMemcpyHostToDevice, s));
+  uint32_t *d_goff = in.d<uint32_t>(at_goff), *d_nbr = in.d<uint32_t>(at_nbr);
+  float *d_feat = in.d<float>(at_feat), *d_target = in.d<float>(at_target), *d_loss = M.grad + kParams;
   if (!target) {
     rc = launch_graph_kernel(e, false, num_graphs, d_goff, d_feat, d_nbr, d_scores, nullptr, 0.f, nullptr, nullptr);
   } else {
-    FSIG_CUDA_TRY(cudaMemsetAsync(M.grad, 0, sizeof(float) * kParams, s));
-    FSIG_CUDA_TRY(cudaMemsetAsync(d_loss, 0, sizeof(float), s));
+    FSIG_CUDA_TRY(cudaMemsetAsync(M.grad, 0, sizeof(float) * (kParams + 1), s));
     rc = launch_graph_kernel(e, true, num_graphs, d_goff, d_feat, d_nbr, d_scores, d_target,
                              nodes ? 1.f / float(nodes) : 0.f, d_loss, d_acts);
     if (!rc && nodes) {
@@ -561,11 +567,19 @@ int mpnn_run(Engine& e, uint32_t num_graphs, const uint32_t* goff, const float* 
       FSIG_CUDA_TRY(cudaGetLastError());
     }
   }
-  if (rc) { e.arena.release(mark); return rc; }
-  if (scores && nodes) FSIG_CUDA_TRY(cudaMemcpyAsync(scores, d_scores, sizeof(float) * nodes, cudaMemcpyDeviceToHost, s));
-  if (loss) FSIG_CUDA_TRY(cudaMemcpyAsync(loss, d_loss, sizeof(float), cudaMemcpyDeviceToHost, s));
-  if (grads_out) FSIG_CUDA_TRY(cudaMemcpyAsync(grads_out, M.grad, sizeof(float) * kParams, cudaMemcpyDeviceToHost, s));
+  if (rc) {
+    cudaStreamSynchronize(s);  // the queued copy reads the staging area
+    e.arena.release(mark);
+    return rc;
+  }
+  if (scores && nodes)
+    FSIG_CUDA_TRY(cudaMemcpyAsync(res.host + at_scores, d_scores, sizeof(float) * nodes, cudaMemcpyDeviceToHost, s));
+  if (target && (loss || grads_out))
+    FSIG_CUDA_TRY(cudaMemcpyAsync(res.host, M.grad, sizeof(float) * (kParams + 1), cudaMemcpyDeviceToHost, s));
   FSIG_CUDA_TRY(cudaStreamSynchronize(s));
+  if (scores && nodes) std::memcpy(scores, res.host + at_scores, sizeof(float) * nodes);
+  if (target && grads_out) std::memcpy(grads_out, res.host, sizeof(float) * kParams);
+  if (target && loss) std::memcpy(loss, res.host + sizeof(float) * kParams, sizeof(float));
   e.arena.release(mark);
   return FSIG_OK;
 }

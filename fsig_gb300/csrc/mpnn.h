@@ -27,7 +27,7 @@ constexpr int kParams = kPBout + 1;
 
 struct MpnnState {
   float* master = nullptr;   // [kParams]
-  float* grad = nullptr;     // [kParams]
+  float* grad = nullptr;     // [kParams], then the loss
   float* m1 = nullptr;       // Adam moments
   float* m2 = nullptr;
   uint16_t* wbf = nullptr;   // BF16 copies of W_in, W_s, W_n (same offsets as master, up to kPB)
