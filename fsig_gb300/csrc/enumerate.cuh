@@ -9,9 +9,8 @@
 // A warp extends up to 32 partial embeddings at a time, one per lane.  For
 // every depth it keeps a buffer of up to 32 mapped vertices in shared memory,
 // each with the slot of its parent in the previous depth's buffer; an entry's
-// earlier vertices are found by walking its parents.  Lane j holds depth j's
-// cursor (cnt_j entries from sp_j on, it_j the first one not wholly extended,
-// off_j how much of that one's driver range is examined).
+// earlier vertices are found by walking its parents.  LevelState is a depth's
+// cursor.
 //
 // Filling the buffer of depth i from depth i-1's entries: each lane takes one
 // entry, finds the label-l(i) segments of its backward neighbours' rows
@@ -43,8 +42,10 @@
 // filter tested beside the candidate bit (a third of the windows on 2^26 edges
 // end there), leaves of two segments in the leaf loop, and four earlier vertices
 // a load (a loop of one each took 25 % of the house count): 139 ms there, 21.5 ms
-// for 512 queries of 4-32 vertices, house counting 55 -> 32 ms.  In the leaf loop
-// the hash is 15 % of the time; loading a window ahead gains nothing.
+// for 512 queries of 4-32 vertices, house counting 55 -> 32 ms.  With 96 windows a
+// fill and each depth's plan and cursor in one record: 25.4, 20.5 and 132 ms.  Of
+// the first, the leaf loop takes two fifths and the set-up of fills the rest; the
+// hash is 15 %; loading a window ahead gains nothing.
 //
 // Work stealing: a warp that runs out of input takes a ticket, one atomicAdd
 // on the queue's head, and waits for the record of that number, polling the
@@ -140,18 +141,41 @@ constexpr uint32_t kBuf = 32;        // entries of a depth's buffer
 constexpr uint32_t kScratch = 384;   // words for the segments and earlier vertices of the entries being extended
 // Candidate windows one fill examines before it returns, so that the periodic
 // checks and hand-offs come in time on long driver ranges.
+// (64: 139 ms for 512 queries on 2^26 edges, 96: 136; 128 and 256 are slower for
+// batches of a few queries.)
 constexpr uint32_t kFillWindows = 96;
 // Windows between two checks of the work limit and of the waiting warps.
 constexpr uint32_t kCheckWindows = 32;
 
-constexpr uint32_t kPool = 512;      // entries of all buffers of a warp (see below)
+constexpr uint32_t kPool = 384;      // entries of all buffers of a warp (see below)
+
+// What a fill needs to know of its depth, in two 16-byte loads; made from the
+// query's Plan when a warp turns to it.  (Read field by field, with the levels'
+// cursors in registers of lanes, 200 eight-vertex queries on 320k vertices took
+// 26.6 ms instead of 25.4, 512 queries on 2^26 edges 136 instead of 132.)
+struct alignas(16) LevelPlan {
+  const uint32_t* bm;  // candidate bitmap
+  uint32_t bwd;        // earlier depths adjacent to this one
+  uint32_t inj;        // earlier depths of the same label that are not
+  uint32_t bmbase;     // first id of the bitmap
+  uint32_t dense;      // segments from this length on have an exact filter (in filter words)
+  int32_t lab;
+  uint8_t nb, n4;      // segments; earlier vertices to compare, in fours
+  uint8_t stride;      // entries extended at a time
+  uint8_t qv;          // query vertex
+};
+struct alignas(16) LevelState {
+  uint32_t cnt, it, off;  // entries, the first one not wholly extended, how much of its driver range is examined
+  uint32_t sp;            // where the buffer starts in the pool
+};
 
 // Per warp.  The depths' buffers lie one after another in the pool, each as
 // long as it is filled; a fill takes at most kBuf entries and leaves one for
 // each depth below it.  (A fixed 32 entries for each of 31 depths would allow 3
 // blocks an SM instead of 4.)
 struct WarpSmem {
-  Plan plan;
+  LevelPlan plan[kMaxQ];
+  LevelState lev[kMaxQ];
   uint2 owner[kBuf];                // entries with a driver: its place relative to the window index, the entry
   unsigned long long sown[kBuf];    // leaf: partial hash of each entry being extended
   unsigned long long sbase[kBuf];   // partial hashes of depth n-3's buffer
@@ -162,12 +186,12 @@ struct WarpSmem {
   uint8_t par[kPool];               // its parent's place in the previous depth's buffer
   // What only fills, tasks and hand-offs touch is kept here for the registers.
   unsigned long long found[kMaxQ];  // partial embeddings of each length, of the current query, not yet published
-  unsigned long long bytes;         // bytes requested by global loads
+  unsigned long long loads;         // 4-byte loads of the windows, filters and searches
   uint32_t ev[5];                   // events: tasks, records popped, hand-offs, records written, windows
   uint32_t pend;                    // driver entries examined, not yet published to res.work
   uint32_t task_lo, task_hi;        // driver range of the task at its first depth
   uint32_t t, t_last;               // input tasks in hand: [t, t_last)
-  uint32_t query, pad[3];
+  uint32_t query, n, pad[2];
 };
 static_assert(sizeof(WarpSmem) % 16 == 0, "the next warp's part is aligned");
 
@@ -229,14 +253,12 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
   const uint32_t nroots = A.in_tasks ? 0u : *A.nroots_ptr;
   const uint32_t T_in = A.in_tasks ? A.in_count : min(A.chunk_off[nroots], A.t_end);
 
-  // lane-distributed level state
-  uint32_t cnt = 0, it = 0, off = 0, sp = 0;  // sp: where depth j's buffer starts in the pool
   unsigned long long my_hash = 0;
   bool s_valid = false;  // sbase holds depth n-3's current buffer
   ws.found[lane] = 0;
   if (lane < 5) ws.ev[lane] = 0;
   if (lane == 0) {
-    ws.bytes = 0;
+    ws.loads = 0;
     ws.pend = 0;
     ws.t = ws.t_last = 0;
     ws.query = kInvalid;
@@ -248,7 +270,7 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
   // (every driver entry counts once), so whether it exceeds the limit does not
   // either.
   auto publish = [&]() {
-    if (lane == 0 && ws.pend) {
+    if (lane == 0 && A.work_cap && ws.pend) {
       const unsigned long long tot = atomicAdd(&A.res[ws.query].work, (unsigned long long)ws.pend) + ws.pend;
       ws.pend = 0;
       if (tot > A.work_cap) atomicExch(&A.res[ws.query].aborted, 1u);
@@ -260,7 +282,7 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
     uint32_t v = 0;
 #pragma unroll 1
     for (uint32_t k = p;; k--) {
-      const uint32_t at = __shfl_sync(kFull, sp, k) + slot;
+      const uint32_t at = ws.lev[k].sp + slot;
       const uint32_t x = ws.cand[at];
       if (lane == k) v = x;
       if (k == 0) break;
@@ -275,10 +297,11 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
   // done here.  [lo_set, hi_set): the task's own driver range at depth d0, if
   // it has one.  Returns false when no records may be reserved.
   auto donate = [&](uint32_t d0, uint32_t last, uint32_t hungry, uint32_t lo_set, uint32_t hi_set) -> bool {
-    const uint32_t has = __ballot_sync(kFull, lane + 1 >= d0 && lane <= last && it < cnt);
+    const LevelState mine = ws.lev[lane];
+    const uint32_t has = __ballot_sync(kFull, lane + 1 >= d0 && lane <= last && mine.it < mine.cnt);
     if (!has) return true;
     const uint32_t l = __ffs(has) - 1;
-    const uint32_t c_l = __shfl_sync(kFull, cnt, l), i_l = __shfl_sync(kFull, it, l), o_l = __shfl_sync(kFull, off, l);
+    const uint32_t c_l = ws.lev[l].cnt, i_l = ws.lev[l].it, o_l = ws.lev[l].off;
     // the current entry's driver range, when it is partly examined or given
     const bool given = l + 1 == d0 && lo_set != kInvalid;
     const bool part = given || o_l > 0;
@@ -287,8 +310,8 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
       fp = prefix(l, i_l);
       if (!given) {  // the choice a fill makes: the shortest segment, the latest depth on ties
         uint32_t a = 0, b = 0, len = kInvalid;
-        if ((ws.plan.bwd[l + 1] >> lane) & 1u) {
-          row_segment<kRows>(g, fp, ws.plan.lab[l + 1], W1, a, b);
+        if ((ws.plan[l + 1].bwd >> lane) & 1u) {
+          row_segment<kRows>(g, fp, ws.plan[l + 1].lab, W1, a, b);
           len = b - a;
         }
         const uint32_t shortest = __reduce_min_sync(kFull, len);
@@ -344,9 +367,10 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
       if (lane <= l) r->f[lane] = fk;
       if (lane == 0) { r->q = ws.query; r->d = l + 1; r->lo = kInvalid; r->hi = kInvalid; }
     }
-    if (lane == l) {
-      it = cnt;
-      off = 0;
+    __syncwarp();
+    if (lane == 0) {
+      ws.lev[l].it = c_l;
+      ws.lev[l].off = 0;
     }
     __threadfence();
     __syncwarp();
@@ -386,12 +410,12 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
     const unsigned long long row = base + __popc(m & lanemask_lt());
     const bool mine = ((m >> lane) & 1u) && row < A.emit_cap;
     uint32_t* dst = A.emit + row * n;
-    if (mine) dst[ws.plan.qv[n - 1]] = xo;
+    if (mine) dst[ws.plan[n - 1].qv] = xo;
 #pragma unroll 1
     for (uint32_t k = n - 1; k-- > 0;) {
-      const uint32_t at = __shfl_sync(kFull, sp, k) + slot;
+      const uint32_t at = ws.lev[k].sp + slot;
       if (mine) {
-        dst[ws.plan.qv[k]] = __ldg(g.old_of_new + ws.cand[at]);
+        dst[ws.plan[k].qv] = __ldg(g.old_of_new + ws.cand[at]);
         slot = ws.par[at];
       }
     }
@@ -402,14 +426,16 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
   // hashes.  [lo_set, hi_set), unless kInvalid, is the driver range of the one
   // entry there is.  Returns the windows examined; the cursors of depths lv - 1
   // and lv say where it stopped.
+  uint32_t made = 0;  // entries the last fill appended
   auto fill = [&](uint32_t lv, uint32_t lo_set, uint32_t hi_set) -> uint32_t {
-    const uint32_t n = ws.plan.n, p = lv - 1;
+    const uint32_t n = ws.n, p = lv - 1;
     const bool leaf = lv + 1 == n;
-    const uint32_t bwd = ws.plan.bwd[lv], inj = ws.plan.same[lv] & ~bwd;
-    const int32_t lab = ws.plan.lab[lv];
-    const uint32_t nb = __popc(bwd), n4 = (__popc(inj) + 3) / 4;
-    const uint32_t words = 2 * nb + 4 * n4;
-    const uint32_t stride = words <= kScratch / kBuf ? kBuf : kScratch / words;  // entries per group
+    const LevelPlan lp = ws.plan[lv];
+    const LevelState from = ws.lev[p];
+    const uint32_t bwd = lp.bwd, inj = lp.inj, nb = lp.nb, n4 = lp.n4, stride = lp.stride;
+    const uint32_t bmbase = lp.bmbase, dense = lp.dense;
+    const int32_t lab = lp.lab;
+    const uint32_t* __restrict__ bm = lp.bm;
     uint4* const other = reinterpret_cast<uint4*>(ws.scratch);  // [n4][stride], padded with kInvalid
     uint2* const segs = ws.scratch + 2 * n4 * stride;           // [nb][stride]
     // whether x is none of entry c's earlier vertices
@@ -422,29 +448,23 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
       }
       return yes;
     };
-    const uint32_t bmbase = ws.plan.bmbase[lv];
-    const uint32_t* __restrict__ bm = A.pool + ws.plan.bmoff[lv];
-    // segments are kept in units of their filter's words; from `dense` on it is exact
-    const uint32_t fs = g.filt ? g.fshift : 0;
-    const uint32_t dense =
-        nb > 1 && g.filt ? filter_dense_len(__ldg(g.base + lab + 1) - bmbase, fs) << fs : kInvalid;
-    const uint32_t cntp = __shfl_sync(kFull, cnt, p), spp = __shfl_sync(kFull, sp, p);
-    const uint32_t spl = spp + cntp;                              // depth lv's buffer
+    const uint32_t fs = g.filt ? g.fshift : 0;  // segments are kept in units of their filter's words
+    const uint32_t cntp = from.cnt, spp = from.sp, spl = spp + cntp;  // spl: depth lv's buffer
     const uint32_t room = min(kBuf, kPool - spl - (n - 2 - min(lv, n - 2)));
     // Entries that end a fill.  With further segments to search the room left
     // decides how many lanes search, so half the buffer is enough.
     const uint32_t enough = nb > 1 || room < 16 ? (room + 1) / 2 : room - 8;
-    uint32_t itp = __shfl_sync(kFull, it, p), offp = __shfl_sync(kFull, off, p);
+    uint32_t itp = from.it, offp = from.off;
     uint32_t have = 0, sure = 0;  // entries appended; of them, searched for in every segment
     uint32_t used = 0, seen = 0, hits = 0, loads = 0;  // loads: 4-byte loads of the filters and searches
     bool stop = false;
     if (leaf && !s_valid && lv >= 2) {  // partial hashes of depth n-3's entries
       unsigned long long sum = 0;
-      uint32_t slot = min(lane, __shfl_sync(kFull, cnt, lv - 2) - 1);
+      uint32_t slot = min(lane, ws.lev[lv - 2].cnt - 1);
 #pragma unroll 1
       for (uint32_t k = lv - 1; k-- > 0;) {
-        const uint32_t at = __shfl_sync(kFull, sp, k) + slot;
-        sum += fmix64((uint64_t(ws.plan.qv[k]) << 32) | __ldg(g.old_of_new + ws.cand[at]));
+        const uint32_t at = ws.lev[k].sp + slot;
+        sum += fmix64((uint64_t(ws.plan[k].qv) << 32) | __ldg(g.old_of_new + ws.cand[at]));
         slot = ws.par[at];
       }
       ws.sbase[lane] = sum;
@@ -482,7 +502,7 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
           }
           need &= ~(1u << k);
           if (!need) break;
-          at = __shfl_sync(kFull, sp, k - 1) + ws.par[at];
+          at = ws.lev[k - 1].sp + ws.par[at];
         }
         if (mine && drv) segs[drv * stride + lane] = segs[lane];  // the others: places 1 .. nb - 1
         if (lo_set != kInvalid) {
@@ -496,7 +516,7 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
         if (!mine) len = 0;
       }
       if (leaf) {
-        unsigned long long sum = fmix64((uint64_t(ws.plan.qv[p]) << 32) | __ldg(g.old_of_new + ws.cand[own]));
+        unsigned long long sum = fmix64((uint64_t(ws.plan[p].qv) << 32) | __ldg(g.old_of_new + ws.cand[own]));
         if (p > 0) sum += ws.sbase[ws.par[own]];
         ws.sown[lane] = sum;
       }
@@ -521,7 +541,7 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
       uint32_t pos = 0, begun = kInvalid;  // begun: drivers that start before pos, minus one
       if (leaf && !A.emit && (nb == 1 || (nb == 2 && filtered))) {
         // the common leaves: at most one segment to look up, all lanes alike
-        const uint64_t tq = uint64_t(ws.plan.qv[lv]) << 32;
+        const uint64_t tq = uint64_t(lp.qv) << 32;
 #pragma unroll 1
         while (pos < T && !stop) {
           const uint32_t heads = __reduce_or_sync(kFull, bit_or_zero(start - pos));
@@ -635,7 +655,7 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
         __syncwarp();
         if (leaf) {
           const uint32_t xo = kRows ? __ldg(g.old_of_new + x) : __ldg(g.adj_old + at);
-          const uint64_t h = fmix64(A.seed + ws.sown[c] + fmix64((uint64_t(ws.plan.qv[lv]) << 32) | xo));
+          const uint64_t h = fmix64(A.seed + ws.sown[c] + fmix64((uint64_t(lp.qv) << 32) | xo));
           my_hash += pred ? h : 0;
           hits += pred;
           if (A.emit) {
@@ -672,24 +692,19 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
       __syncwarp();
     }
     if (leaf) have = __reduce_add_sync(kFull, hits);
-    if (lane == p) {
-      it = itp;
-      off = offp;
-    }
-    if (lane == lv && !leaf) {
-      cnt = have;
-      it = 0;
-      off = 0;
-      sp = spl;
-    }
     if (lv + 3 == n) s_valid = false;
-    loads = __reduce_add_sync(kFull, loads);
+    if (nb > 1) loads = __reduce_add_sync(kFull, loads);
     if (lane == 0) {
+      ws.lev[p].it = itp;
+      ws.lev[p].off = offp;
+      if (!leaf) ws.lev[lv] = LevelState{have, 0, 0, spl};
       ws.found[lv] += have;
       ws.ev[4] += used;
-      ws.bytes += 4ull * loads + ((leaf ? 12ull : 8ull) + (nb > 1 && g.filt ? 4ull : 0ull)) * seen;
-      if (A.work_cap) ws.pend += seen;
+      ws.pend += seen;
+      ws.loads += loads + seen * ((leaf ? 3 : 2) + (nb > 1 && g.filt ? 1 : 0));
     }
+    __syncwarp();
+    made = have;
     return used;
   };
 
@@ -808,30 +823,49 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
         publish();
         const unsigned long long h = warp_sum(my_hash), c = ws.found[lane];
         if (lane == 0 && h) atomicAdd(&A.res[cur_q].hash, h);
-        if (lane < ws.plan.n && c) {
+        if (lane < ws.n && c) {
           atomicAdd(&A.res[cur_q].levels[lane], c);
-          if (lane + 1 == ws.plan.n) atomicAdd(&A.res[cur_q].count, c);
+          if (lane + 1 == ws.n) atomicAdd(&A.res[cur_q].count, c);
         }
         my_hash = 0;
         ws.found[lane] = 0;
       }
       if (q == kInvalid) break;
       __syncwarp();
-      const uint32_t* src = reinterpret_cast<const uint32_t*>(A.plans + q);
-      uint32_t* dst = reinterpret_cast<uint32_t*>(&ws.plan);
-#pragma unroll 1
-      for (uint32_t i = lane; i < sizeof(Plan) / 4; i += 32) dst[i] = src[i];
+      const Plan& pl = A.plans[q];
+      const uint32_t n = pl.n;
+      if (lane < n) {
+        LevelPlan x;
+        x.bm = A.pool + pl.bmoff[lane];
+        x.bwd = pl.bwd[lane];
+        x.inj = pl.same[lane] & ~x.bwd;
+        x.bmbase = pl.bmbase[lane];
+        x.lab = pl.lab[lane];
+        x.nb = uint8_t(__popc(x.bwd));
+        x.n4 = uint8_t((__popc(x.inj) + 3) / 4);
+        const uint32_t words = 2 * x.nb + 4 * x.n4;
+        x.stride = uint8_t(words <= kScratch / kBuf ? kBuf : kScratch / words);
+        x.qv = uint8_t(pl.qv[lane]);
+        x.dense = kInvalid;
+        if (g.filt && x.lab >= 0 && x.lab < g.L)
+          x.dense = filter_dense_len(__ldg(g.base + x.lab + 1) - x.bmbase, g.fshift) << g.fshift;
+        ws.plan[lane] = x;
+      }
+      if (lane == 0) {
+        ws.n = n;
+        ws.pend = 0;
+      }
       if (lane == 0) ws.query = q;
       __syncwarp();
     }
-    const uint32_t n = ws.plan.n;
+    const uint32_t n = ws.n;
     if (root != kInvalid) {
       if (lane == 0) {
         f = root;
         ws.found[0] += chunk == 0;  // the root itself, once
       }
       if (n > 1) {
-        row_segment<kRows>(g, root, ws.plan.lab[1], W1, lo, hi);
+        row_segment<kRows>(g, root, ws.plan[1].lab, W1, lo, hi);
         lo += chunk * A.split;
         hi = min(lo + A.split, hi);
       }
@@ -840,7 +874,7 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
     if (d == n) {  // a complete embedding (single-vertex queries)
       if (lane == 0) {
         const uint32_t xo = __ldg(g.old_of_new + f);
-        my_hash += fmix64(A.seed + fmix64((uint64_t(ws.plan.qv[0]) << 32) | xo));
+        my_hash += fmix64(A.seed + fmix64((uint64_t(ws.plan[0].qv) << 32) | xo));
         if (A.emit) {
           const unsigned long long row = atomicAdd(A.emit_ctr, 1ull);
           if (row < A.emit_cap) A.emit[row] = xo;
@@ -859,10 +893,7 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
       ws.task_lo = lo;
       ws.task_hi = hi;
     }
-    sp = lane;
-    cnt = lane < d ? 1u : 0u;
-    it = lane + 1 < d ? 1u : 0u;
-    off = 0;
+    ws.lev[lane] = LevelState{lane < d ? 1u : 0u, lane + 1 < d ? 1u : 0u, 0u, lane};
     s_valid = false;
     __syncwarp();
     uint32_t lv = d, windows = kCheckWindows, used = 0;
@@ -887,18 +918,18 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
           if (last >= d) donate(d, min(lv, last - 1), hungry, ws.task_lo, ws.task_hi);
         }
       }
-      if (__shfl_sync(kFull, it, lv - 1) >= __shfl_sync(kFull, cnt, lv - 1)) {
+      if (ws.lev[lv - 1].it >= ws.lev[lv - 1].cnt) {
         if (lv == d) break;
         lv--;
         continue;
       }
       used = fill(lv, lv == d ? ws.task_lo : kInvalid, ws.task_hi);
       windows += used + 1;
-      if (lv + 1 < n && __shfl_sync(kFull, cnt, lv) > 0) lv++;
+      if (lv + 1 < n && made > 0) lv++;
     }
   }
   if (lane == 0) {
-    atomicAdd(A.algo_bytes, ws.bytes);
+    atomicAdd(A.algo_bytes, 4 * ws.loads);
 #pragma unroll 1
     for (int i = 0; i < 5; i++) atomicAdd(&A.ev[i], (unsigned long long)ws.ev[i]);
   }
