@@ -127,8 +127,9 @@ constexpr uint32_t kCtrStride = 32;        // one 128-byte line per counter
 // g = t / out_cap of that slot.  The slot's ready word is 2g while it is free
 // for that use, 2g + 1 from the record's publication until its ticket holder
 // has read it, then 2g + 2 (= free for use g + 1).  Records are reserved only
-// while warps wait, so at most (warps) x (records of one hand-off) numbers lie
-// between the tickets and the tail, far below the ring's 2^20 slots: a
+// while warps wait, so at most (warps) x (records of one hand-off, up to 32 +
+// kLastBuf) numbers lie between the tickets and the tail, fewer than the ring's
+// 2^20 slots: a
 // reserved slot's previous record always has a ticket holder.
 
 __device__ __forceinline__ unsigned long long global_ns() {
@@ -138,6 +139,16 @@ __device__ __forceinline__ unsigned long long global_ns() {
 }
 
 constexpr uint32_t kBuf = 32;        // entries of a depth's buffer
+// Depth n-2, whose entries the leaf loop takes 32 at a time, may keep up to
+// kLastBuf when neither it nor the leaf has a second segment: a fill that ends
+// at 32 entries has set up 32 parents and used three or four of them where each
+// has ten children (200 eight-vertex queries on 320k vertices 25.4 -> 22.9 ms
+// with 128, 23.4 with 64, 22.3 with 192).  It does not where the leaf's ranges are
+// long (from kLongLeaf / 8 windows an entry on, in its last fill), since fewer,
+// longer buffers then only keep work from the warps that wait: 37 queries on
+// 2^26 edges 11.6 ms, 12.5 with 128 always; nor while warps wait.
+constexpr uint32_t kLastBuf = 128;
+constexpr uint32_t kLongLeaf = 6;
 constexpr uint32_t kScratch = 384;   // words for the segments and earlier vertices of the entries being extended
 // Candidate windows one fill examines before it returns, so that the periodic
 // checks and hand-offs come in time on long driver ranges.
@@ -170,9 +181,9 @@ struct alignas(16) LevelState {
 };
 
 // Per warp.  The depths' buffers lie one after another in the pool, each as
-// long as it is filled; a fill takes at most kBuf entries and leaves one for
-// each depth below it.  (A fixed 32 entries for each of 31 depths would allow 3
-// blocks an SM instead of 4.)
+// long as it is filled; a fill takes at most kBuf entries (kLastBuf at depth n-2)
+// and leaves one for each depth below it.  (A fixed 32 entries for each of 31
+// depths would allow 3 blocks an SM instead of 4.)
 struct WarpSmem {
   LevelPlan plan[kMaxQ];
   LevelState lev[kMaxQ];
@@ -191,7 +202,8 @@ struct WarpSmem {
   uint32_t pend;                    // driver entries examined, not yet published to res.work
   uint32_t task_lo, task_hi;        // driver range of the task at its first depth
   uint32_t t, t_last;               // input tasks in hand: [t, t_last)
-  uint32_t query, n, pad[2];
+  uint32_t query, n;
+  uint32_t room, pad;               // longest buffer of depth n-2
 };
 static_assert(sizeof(WarpSmem) % 16 == 0, "the next warp's part is aligned");
 
@@ -450,7 +462,8 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
     };
     const uint32_t fs = g.filt ? g.fshift : 0;  // segments are kept in units of their filter's words
     const uint32_t cntp = from.cnt, spp = from.sp, spl = spp + cntp;  // spl: depth lv's buffer
-    const uint32_t room = min(kBuf, kPool - spl - (n - 2 - min(lv, n - 2)));
+    const uint32_t longest = lv + 2 == n && nb == 1 && ws.plan[lv + 1].nb == 1 ? ws.room : kBuf;
+    const uint32_t room = min(longest, kPool - spl - (n - 2 - min(lv, n - 2)));
     // Entries that end a fill.  With further segments to search the room left
     // decides how many lanes search, so half the buffer is enough.
     const uint32_t enough = nb > 1 || room < 16 ? (room + 1) / 2 : room - 8;
@@ -892,11 +905,12 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
     if (lane == 0) {
       ws.task_lo = lo;
       ws.task_hi = hi;
+      ws.room = kBuf;
     }
     ws.lev[lane] = LevelState{lane < d ? 1u : 0u, lane + 1 < d ? 1u : 0u, 0u, lane};
     s_valid = false;
     __syncwarp();
-    uint32_t lv = d, windows = kCheckWindows, used = 0;
+    uint32_t lv = d, windows = kCheckWindows, used = 0, hungry = 1;
 #pragma unroll 1
     for (;;) {
       if (windows >= kCheckWindows) {
@@ -911,20 +925,25 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
         if (lane == 0) stop |= *(volatile uint32_t*)&A.ctr[3 * kCtrStride] != 0;
         if (__shfl_sync(kFull, stop, 0)) break;
         // (never before the first window: a task handed on untouched would go round)
-        const uint32_t hungry = used ? waiting_warps(t_start) : 0u;
-        if (hungry) {
+        if (used) hungry = waiting_warps(t_start);
+        if (used && hungry) {
           // the entries of the leaf's ranges are handed off only when those are long
           const uint32_t last = (lv + 1 == n && used >= kFillWindows) ? n - 1 : n - 2;  // plus one
           if (last >= d) donate(d, min(lv, last - 1), hungry, ws.task_lo, ws.task_hi);
         }
       }
-      if (ws.lev[lv - 1].it >= ws.lev[lv - 1].cnt) {
+      const uint32_t before = ws.lev[lv - 1].it;
+      if (before >= ws.lev[lv - 1].cnt) {
         if (lv == d) break;
         lv--;
         continue;
       }
       used = fill(lv, lv == d ? ws.task_lo : kInvalid, ws.task_hi);
       windows += used + 1;
+      if (lv + 1 == n) {
+        if (lane == 0) ws.room = hungry || 8 * used >= kLongLeaf * (ws.lev[lv - 1].it - before) ? kBuf : kLastBuf;
+        __syncwarp();
+      }
       if (lv + 1 < n && made > 0) lv++;
     }
   }
