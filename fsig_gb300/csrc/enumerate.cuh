@@ -155,6 +155,7 @@ constexpr uint32_t kScratch = 384;   // words for the segments and earlier verti
 // (64: 139 ms for 512 queries on 2^26 edges, 96: 136; 128 and 256 are slower for
 // batches of a few queries.)
 constexpr uint32_t kFillWindows = 96;
+constexpr uint32_t kJointEntries = 32 * kFillWindows;
 // Windows between two checks of the work limit and of the waiting warps.
 constexpr uint32_t kCheckWindows = 32;
 
@@ -489,7 +490,7 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
       uint32_t group = min(cntp - itp, stride);
       const bool mine = lane < group;
       const uint32_t own = spp + itp + min(lane, group - 1);
-      uint32_t dlo = 0, len = kInvalid, drv = 0;
+      uint32_t dlo = 0, len = kInvalid, drv = 0, anc = 0;  // anc: where the driver's vertex lies in the pool
       {
         uint32_t at = own, need = bwd | inj, wb = 0, wi = 0;
         if (mine) {
@@ -507,6 +508,7 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
               len = b - a;
               dlo = a;
               drv = wb;
+              anc = at;
             }
             wb++;
           } else if ((inj >> k) & 1u) {
@@ -537,6 +539,20 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
         group = 1;
         if (lane) len = 0;
       }
+      // Entries next to one another whose driver belongs to the same vertex: its
+      // candidates are found once for all of them (joint, below).
+      uint32_t joint = 0, run = 0;  // joint: driver entries of the group, before they are shared
+      if (leaf && nb == 1 && !(bwd >> p) && n4 <= 2 && !A.emit && !offp && lo_set == kInvalid) {
+        const uint32_t before = __shfl_up_sync(kFull, anc, 1);
+        const uint32_t firsts = __ballot_sync(kFull, mine && (lane == 0 || anc != before)) | bit_or_zero(group);
+        const uint32_t all = __reduce_add_sync(kFull, len);
+        if (2 * __popc(firsts) <= group + 2 && all <= kJointEntries) {
+          joint = all;
+          const uint32_t later = firsts & ~lanemask_le();
+          run = (later ? __ffs(later) - 1 : 32u) - lane;
+          if (!((firsts >> lane) & 1u)) len = 0;
+        }
+      }
       uint32_t incl = len;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -547,12 +563,62 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
       const uint32_t start = len ? incl - len : kInvalid;
       {
         const uint32_t rank = __popc(__ballot_sync(kFull, len != 0) & lanemask_lt());
-        if (len) ws.owner[rank] = make_uint2(dlo - start, lane);
+        if (len) ws.owner[rank] = make_uint2(dlo - start, lane | run << 8);
       }
       __syncwarp();
       const bool filtered = nb > 1 && g.filt;
       uint32_t pos = 0, begun = kInvalid;  // begun: drivers that start before pos, minus one
-      if (leaf && !A.emit && (nb == 1 || (nb == 2 && filtered))) {
+      if (joint) {
+        uint4* const cands = reinterpret_cast<uint4*>(ws.scratch) + 2 * kBuf;  // candidate, its hash, first entry less first pair
+        const uint64_t tq = uint64_t(lp.qv) << 32;
+#pragma unroll 1
+        while (pos < T) {
+          const uint32_t heads = __reduce_or_sync(kFull, bit_or_zero(start - pos));
+          const uint2 o = ws.owner[begun + __popc(heads & lanemask_le())];
+          const uint32_t e = pos + lane, at = o.x + min(e, T - 1);
+          const uint32_t x = __ldg(g.adj + at);
+          const uint32_t xo = kRows ? __ldg(g.old_of_new + x) : __ldg(g.adj_old + at);
+          const uint32_t bit = x - bmbase;
+          const bool pred = e < T && ((__ldg(bm + (bit >> 5)) >> (bit & 31)) & 1u);
+          const uint32_t pairs = pred ? o.y >> 8 : 0u;
+          uint32_t upto = pairs;
+#pragma unroll
+          for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(kFull, upto, d);
+            if (lane >= uint32_t(d)) upto += y;
+          }
+          const uint32_t P = __shfl_sync(kFull, upto, 31);
+          const uint32_t first = pred ? upto - pairs : kInvalid;
+          const uint32_t rank = __popc(__ballot_sync(kFull, pred) & lanemask_lt());
+          if (pred) {
+            const uint64_t h = fmix64(tq | xo);
+            cands[rank] = make_uint4(x, uint32_t(h), uint32_t(h >> 32), (o.y & 255u) - first);
+          }
+          __syncwarp();
+          uint32_t k = kInvalid;
+#pragma unroll 1
+          for (uint32_t i = 0; i < P; i += 32) {
+            const uint32_t hd = __reduce_or_sync(kFull, bit_or_zero(first - i));
+            const uint4 y = cands[k + __popc(hd & lanemask_le())];
+            const uint32_t c = y.w + min(i + lane, P - 1);
+            bool yes = i + lane < P;
+            if (n4) yes = yes && fresh(y.x, c);
+            const uint64_t h = fmix64(A.seed + ws.sown[c] + (uint64_t(y.z) << 32 | y.y));
+            my_hash += yes ? h : 0;
+            hits += yes;
+            k += __popc(hd);
+            used++;
+          }
+          __syncwarp();
+          begun += __popc(heads);
+          pos += 32;
+          used++;
+        }
+        stop = used >= kFillWindows;
+        if (lane == 0) loads -= 3 * (joint - T);  // counted with the entries seen
+        pos = T;
+        seen += joint;
+      } else if (leaf && !A.emit && (nb == 1 || (nb == 2 && filtered))) {
         // the common leaves: at most one segment to look up, all lanes alike
         const uint64_t tq = uint64_t(lp.qv) << 32;
 #pragma unroll 1
