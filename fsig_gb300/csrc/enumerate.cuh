@@ -27,6 +27,10 @@
 // per-lane binary searches in lockstep) run on all lanes; those found stay.
 // A buffer with enough entries is extended in turn, and later the fill goes on
 // where it stopped.  At the leaf the passing candidates are counted and hashed.
+// A leaf that hangs on an earlier vertex than its parent in the order has the
+// same range for each entry below that vertex, one after another in the buffer:
+// its candidates and their hashes are then found once, and the pairs of a
+// candidate and an entry take the lanes (joint, in fill).
 //
 // What bounds it: instructions and L2 latency (the working set is L2
 // resident), so the aim is full lanes.  A warp per entry, as before, ran 11 of
@@ -43,9 +47,10 @@
 // end there), leaves of two segments in the leaf loop, and four earlier vertices
 // a load (a loop of one each took 25 % of the house count): 139 ms there, 21.5 ms
 // for 512 queries of 4-32 vertices, house counting 55 -> 32 ms.  With 96 windows a
-// fill and each depth's plan and cursor in one record: 25.4, 20.5 and 132 ms.  Of
-// the first, the leaf loop takes two fifths and the set-up of fills the rest; the
-// hash is 15 %; loading a window ahead gains nothing.
+// fill and each depth's plan and cursor in one record: 25.4, 20.5 and 132 ms; of
+// the first the leaf loop took two fifths and the set-up of fills the rest.  With
+// longer last buffers and shared leaf ranges: 19.8, 15.2 and 126 ms.  Loading a
+// window ahead gains nothing.
 //
 // Work stealing: a warp that runs out of input takes a ticket, one atomicAdd
 // on the queue's head, and waits for the record of that number, polling the
@@ -140,7 +145,7 @@ __device__ __forceinline__ unsigned long long global_ns() {
 
 constexpr uint32_t kBuf = 32;        // entries of a depth's buffer
 // Depth n-2, whose entries the leaf loop takes 32 at a time, may keep up to
-// kLastBuf when neither it nor the leaf has a second segment: a fill that ends
+// kLastBuf when it has no second segment itself: a fill that ends
 // at 32 entries has set up 32 parents and used three or four of them where each
 // has ten children (200 eight-vertex queries on 320k vertices 25.4 -> 22.9 ms
 // with 128, 23.4 with 64, 22.3 with 192).  It does not where the leaf's ranges are
@@ -155,7 +160,11 @@ constexpr uint32_t kScratch = 384;   // words for the segments and earlier verti
 // (64: 139 ms for 512 queries on 2^26 edges, 96: 136; 128 and 256 are slower for
 // batches of a few queries.)
 constexpr uint32_t kFillWindows = 96;
-constexpr uint32_t kJointEntries = 32 * kFillWindows;
+// Driver entries of a group up to which its entries' shared ranges are taken
+// together: four fills' worth, since such a group is not interrupted (512 queries
+// on 2^26 edges 131 ms with 3072, 129 with 6144, 126 with this and with eight times
+// it; 200 eight-vertex queries on 320k vertices 19.9 ms with each, 21.0 with 1536).
+constexpr uint32_t kJointEntries = 4 * 32 * kFillWindows;
 // Windows between two checks of the work limit and of the waiting warps.
 constexpr uint32_t kCheckWindows = 32;
 
@@ -463,7 +472,7 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
     };
     const uint32_t fs = g.filt ? g.fshift : 0;  // segments are kept in units of their filter's words
     const uint32_t cntp = from.cnt, spp = from.sp, spl = spp + cntp;  // spl: depth lv's buffer
-    const uint32_t longest = lv + 2 == n && nb == 1 && ws.plan[lv + 1].nb == 1 ? ws.room : kBuf;
+    const uint32_t longest = lv + 2 == n && nb == 1 ? ws.room : kBuf;
     const uint32_t room = min(longest, kPool - spl - (n - 2 - min(lv, n - 2)));
     // Entries that end a fill.  With further segments to search the room left
     // decides how many lanes search, so half the buffer is enough.
@@ -540,7 +549,13 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
         if (lane) len = 0;
       }
       // Entries next to one another whose driver belongs to the same vertex: its
-      // candidates are found once for all of them (joint, below).
+      // candidates are found once for all of them (joint, below).  This pays from
+      // two entries a range on: then the pair loop has no loads from memory and
+      // one hash instead of two.  88 % of the entries of 512 queries of 4-32
+      // vertices on 320k vertices have such a leaf, 27 to a range: 19.5 -> 15.3
+      // ms; of 200 eight-vertex queries 80 %, 14 to a range: 23.0 -> 19.9 ms.  (With
+      // leaves of two segments as well it cost spills and 3 % everywhere, for no
+      // gain on any of these.)
       uint32_t joint = 0, run = 0;  // joint: driver entries of the group, before they are shared
       if (leaf && nb == 1 && !(bwd >> p) && n4 <= 2 && !A.emit && !offp && lo_set == kInvalid) {
         const uint32_t before = __shfl_up_sync(kFull, anc, 1);
