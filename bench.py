@@ -65,9 +65,9 @@ PEAKS = ROOT / "MEASURED_PEAKS.json"
 FALLBACK_HBM_GBS = 6800.0
 
 # DRAM bytes (read + write) of one enumerate_kernel launch on a config-5
-# batch, from an ncu capture (profiles/enumerate_kernel_c5.md: 648.4 MB/s over
-# 392.1 ms); its loads are served from L2 at about 99 %.
-ENUM_TRAFFIC_BYTES_PER_LAUNCH = 257_250_000
+# batch, from an ncu capture (profiles/enumerate_kernel_c5.md: 2872 MB/s over
+# 126.2 ms); its loads are served from L2 at about 98 %.
+ENUM_TRAFFIC_BYTES_PER_LAUNCH = 362_440_000
 
 
 def log(*a):
@@ -410,7 +410,7 @@ def run_ours(args, dist):
                      "peak_source": "measured" if PEAKS.exists() else "fallback",
                      "traffic": ENUM_TRAFFIC_BYTES_PER_LAUNCH if args.workload == "c5" else None,
                      "traffic_note": ("DRAM bytes of one config-5 batch launch (ncu); requested bytes are "
-                                      "served from L2 at about 99% hit: the kernel is issue-bound, not HBM-bound")
+                                      "served from L2 at about 98% hit: the kernel is issue-bound, not HBM-bound")
                                      if args.workload == "c5" else "no ncu capture of this workload",
                      "achieved_basis": "bytes requested by the kernel's global loads / kernel time, "
                                        + roof_basis},
