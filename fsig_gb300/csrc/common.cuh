@@ -141,6 +141,17 @@ __device__ __forceinline__ T warp_sum(T v) {
   return v;
 }
 
+// End of the piece of at most `step` entries that begins at lo in [lo, hi): the
+// sum lo + step may not fit 32 bits (any step a caller gives, positions of large
+// adjacencies).
+__host__ __device__ __forceinline__ uint32_t piece_end(uint32_t lo, uint32_t step, uint32_t hi) {
+  return hi - lo > step ? lo + step : hi;
+}
+// Pieces of at most `step` entries in `len` entries.
+__host__ __device__ __forceinline__ uint32_t piece_count(uint32_t len, uint32_t step) {
+  return len ? (len - 1) / step + 1 : 0;
+}
+
 // first index in [lo, hi) of sorted a[] with a[i] >= key
 __device__ __forceinline__ uint32_t lower_bound_u32(const uint32_t* __restrict__ a, uint32_t lo, uint32_t hi,
                                                     uint32_t key) {

@@ -344,8 +344,8 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
       lo += o_l;
     }
     const uint32_t rest = part ? hi - lo : 0u, takers = min(hungry, 32u);
-    const uint32_t hand = max(32u, (rest + takers - 1) / takers);
-    const uint32_t pieces = (rest + hand - 1) / hand;
+    const uint32_t hand = max(32u, piece_count(rest, takers));
+    const uint32_t pieces = piece_count(rest, hand);
     const uint32_t first = part ? i_l + 1 : i_l;
     const uint32_t total = pieces + (c_l - first);
     uint32_t base = 0;
@@ -380,7 +380,7 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
     for (uint32_t k = 0; k < pieces; k++) {
       TaskRec* r = A.out_tasks + (slot++ & (A.out_cap - 1));
       if (lane <= l) r->f[lane] = fp;
-      if (lane == 0) { r->q = ws.query; r->d = l + 1; r->lo = lo + k * hand; r->hi = min(lo + (k + 1) * hand, hi); }
+      if (lane == 0) { r->q = ws.query; r->d = l + 1; r->lo = lo + k * hand; r->hi = piece_end(lo + k * hand, hand, hi); }
     }
 #pragma unroll 1
     for (uint32_t k = first; k < c_l; k++) {
@@ -961,7 +961,7 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
       if (n > 1) {
         row_segment<kRows>(g, root, ws.plan[1].lab, W1, lo, hi);
         lo += chunk * A.split;
-        hi = min(lo + A.split, hi);
+        hi = piece_end(lo, A.split, hi);
       }
     }
     if (lane == 0) ws.ev[0]++;

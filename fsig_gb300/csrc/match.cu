@@ -477,7 +477,7 @@ __global__ void root_chunks_kernel(GraphView g, const Plan* __restrict__ plans, 
     if (p->n > 1) {
       uint32_t lo, hi;
       segment_of(g, roots[i], p->lab[1], lo, hi);
-      c = max(1u, (hi - lo + split - 1) / split);
+      c = max(1u, piece_count(hi - lo, split));
     }
     chunks[i] = c;
   }
