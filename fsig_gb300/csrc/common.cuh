@@ -152,12 +152,20 @@ __host__ __device__ __forceinline__ uint32_t piece_count(uint32_t len, uint32_t 
   return len ? (len - 1) / step + 1 : 0;
 }
 
+// between lo and hi; their sum may not fit 32 bits
+__host__ __device__ __forceinline__ uint32_t midpoint(uint32_t lo, uint32_t hi) { return lo + ((hi - lo) >> 1); }
+
 // first index in [lo, hi) of sorted a[] with a[i] >= key
-__device__ __forceinline__ uint32_t lower_bound_u32(const uint32_t* __restrict__ a, uint32_t lo, uint32_t hi,
-                                                    uint32_t key) {
+__host__ __device__ __forceinline__ uint32_t lower_bound_u32(const uint32_t* __restrict__ a, uint32_t lo, uint32_t hi,
+                                                             uint32_t key) {
   while (lo < hi) {
-    uint32_t mid = (lo + hi) >> 1;
-    if (__ldg(a + mid) < key) lo = mid + 1; else hi = mid;
+    const uint32_t mid = midpoint(lo, hi);
+#ifdef __CUDA_ARCH__
+    const uint32_t x = __ldg(a + mid);
+#else
+    const uint32_t x = a[mid];
+#endif
+    if (x < key) lo = mid + 1; else hi = mid;
   }
   return lo;
 }

@@ -834,7 +834,7 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
         uint32_t a = 0, b = nroots;  // last i with chunk_off[i] <= t
 #pragma unroll 1
         while (b - a > 1) {
-          const uint32_t mid = (a + b) >> 1;
+          const uint32_t mid = midpoint(a, b);
           if (A.chunk_off[mid] <= t) a = mid; else b = mid;
         }
         chunk = t - A.chunk_off[a];

@@ -246,7 +246,7 @@ __global__ void sort_rows_block_kernel(const uint32_t* __restrict__ rows, const 
 __global__ void long_chunks_kernel(const uint32_t* __restrict__ rows, uint32_t n, const uint32_t* __restrict__ off,
                                    uint32_t* chunks) {
   for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x)
-    chunks[r] = (off[rows[r] + 1] - off[rows[r]] + kSmemRow - 1) / kSmemRow;
+    chunks[r] = piece_count(off[rows[r] + 1] - off[rows[r]], kSmemRow);
 }
 
 // Row (its first entry, length) and first entry within it of chunk c.
@@ -255,7 +255,7 @@ __device__ __forceinline__ void chunk_of(const uint32_t* __restrict__ rows, uint
                                          uint32_t c, uint32_t& b, uint32_t& len, uint32_t& first) {
   uint32_t lo = 0, hi = n;  // last row with chunk_off <= c
   while (hi - lo > 1) {
-    const uint32_t mid = (lo + hi) >> 1;
+    const uint32_t mid = midpoint(lo, hi);
     if (chunk_off[mid] <= c) lo = mid; else hi = mid;
   }
   b = off[rows[lo]];
@@ -289,22 +289,22 @@ __global__ void __launch_bounds__(1024) merge_runs_kernel(const uint32_t* __rest
   for (uint32_t c = blockIdx.x; c < total; c += gridDim.x) {
     uint32_t b, len, first;
     chunk_of(rows, n, chunk_off, off, c, b, len, first);
-    const uint32_t last = first + min(kSmemRow, len - first);
+    const uint32_t count = min(kSmemRow, len - first);
     uint64_t run = 0, lo = len, hi = len;  // the chunk lies in one run; its sibling is [lo, hi)
     if (width) {
       run = first / width;
       lo = min((run ^ 1) * width, uint64_t(len));
       hi = min(lo + width, uint64_t(len));
     }
-    for (uint32_t i = first + threadIdx.x; i < last; i += blockDim.x) {
-      const uint32_t x = in[b + i];
+    for (uint32_t k = threadIdx.x; k < count; k += blockDim.x) {
+      const uint32_t i = first + k, x = in[b + i];
       uint32_t to = i;
       if (lo < hi) {
         // entries of the sibling that go first: the smaller ones, and from a left sibling the equal ones
         const bool right = run & 1;
         uint32_t l = uint32_t(lo), h = uint32_t(hi);
         while (l < h) {
-          const uint32_t mid = (l + h) >> 1;
+          const uint32_t mid = midpoint(l, h);
           const uint32_t y = in[b + mid];
           if (y < x || (right && y == x)) l = mid + 1; else h = mid;
         }
@@ -332,14 +332,17 @@ __global__ void repeats_kernel(const uint32_t* __restrict__ off, const uint32_t*
   if ((threadIdx.x & 31) == 0 && c) atomicAdd(repeats, (unsigned long long)c);
 }
 
-// Unique entries per sorted row, a warp per row.
+// Unique entries per sorted row, a warp per row.  (Here and below, a lane's
+// position is counted from the row's begin or in 64 bits: beyond a row that ends
+// at almost 2^32 it may not fit 32.)
 __global__ void unique_count_kernel(const uint32_t* __restrict__ off, const uint32_t* __restrict__ adj, uint32_t V,
                                     uint32_t* ucount) {
   const uint32_t lane = threadIdx.x & 31;
   for (uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < V; v += (gridDim.x * blockDim.x) >> 5) {
-    const uint32_t b = off[v], e = off[v + 1];
+    const uint32_t* row = adj + off[v];
+    const uint32_t len = off[v + 1] - off[v];  // at most 2^31: one entry per edge
     uint32_t c = 0;
-    for (uint32_t i = b + lane; i < e; i += 32) c += i == b || adj[i] != adj[i - 1];
+    for (uint32_t i = lane; i < len; i += 32) c += i == 0 || row[i] != row[i - 1];
     c = __reduce_add_sync(0xffffffffu, c);
     if (lane == 0) ucount[v] = c;
   }
@@ -349,12 +352,13 @@ __global__ void unique_copy_kernel(const uint32_t* __restrict__ off, const uint3
                                    const uint32_t* __restrict__ noff, uint32_t* out) {
   const uint32_t lane = threadIdx.x & 31;
   for (uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < V; v += (gridDim.x * blockDim.x) >> 5) {
-    const uint32_t b = off[v], e = off[v + 1];
+    const uint32_t* row = adj + off[v];
+    const uint32_t len = off[v + 1] - off[v];
     uint32_t w = noff[v];
-    for (uint32_t i0 = b; i0 < e; i0 += 32) {
+    for (uint32_t i0 = 0; i0 < len; i0 += 32) {
       const uint32_t i = i0 + lane;
-      const uint32_t x = i < e ? adj[i] : 0;
-      const bool keep = i < e && (i == b || x != adj[i - 1]);
+      const uint32_t x = i < len ? row[i] : 0;
+      const bool keep = i < len && (i == 0 || x != row[i - 1]);
       const uint32_t m = __ballot_sync(0xffffffffu, keep);
       if (keep) out[w + __popc(m & lanemask_lt())] = x;
       w += __popc(m);
@@ -425,7 +429,7 @@ __global__ void __launch_bounds__(256) signature_from_rows_kernel(const int32_t*
     if (lane < kSigWords) w[lane] = lane == 0 ? uint32_t(label[v]) : 0u;
     __syncwarp();
     const uint32_t end = off[v + 1];
-    for (uint32_t e = off[v] + lane; e < end; e += 32) {
+    for (uint64_t e = uint64_t(off[v]) + lane; e < end; e += 32) {
       uint32_t word, sh;
       sig_slot(label[adj[e]], word, sh);
       if ((atomicOr(&w[word], 1u << sh) >> sh) & 1u) atomicOr(&w[word], 2u << sh);
@@ -454,12 +458,13 @@ __global__ void __launch_bounds__(256) membership_filter_kernel(
     uint32_t lo = 0, hi = V;  // row of the run's first entry: the last v with off[v] <= k
     const uint32_t first = uint32_t(run * kFilterRun);
     while (hi - lo > 1) {
-      const uint32_t mid = (lo + hi) >> 1;
+      const uint32_t mid = midpoint(lo, hi);
       if (off[mid] <= first) lo = mid; else hi = mid;
     }
     uint32_t v = lo;
-    const uint32_t last = uint32_t(min(uint64_t(first) + kFilterRun, uint64_t(nadj)));
-    for (uint32_t k = first + lane; k < last; k += 32) {
+    const uint32_t count = min(kFilterRun, nadj - first);
+    for (uint32_t i = lane; i < count; i += 32) {
+      const uint32_t k = first + i;
       uint32_t step = 1;
       while (v + step < V && off[v + step] <= k) {
         v += step;

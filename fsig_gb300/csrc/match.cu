@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(256) refine_kernel(GraphView g, const QVert* _
       if (alive) segment_of(g, v, qw->label, k, e);
       uint32_t own = 0;  // supporters found by the lane alone
       if (alive) {
-        const uint32_t stop = e - k > coop_min ? min(k + kRefineOwn, e) : e;
+        const uint32_t stop = e - k > coop_min ? piece_end(k, kRefineOwn, e) : e;
         for (; k < stop && own < need; k++) {
           const uint32_t bit = g.adj[k] - nbase;
           own += (nb[bit >> 5] >> (bit & 31)) & 1u;
@@ -265,8 +265,8 @@ __global__ void __launch_bounds__(256) refine_kernel(GraphView g, const QVert* _
         cm &= cm - 1;
         const uint32_t ck = __shfl_sync(kFull, k, c), ce = __shfl_sync(kFull, e, c);
         uint32_t have = __shfl_sync(kFull, own, c);
-        for (uint32_t p = ck; p < ce && have < need; p += 32) {
-          const uint32_t idx = p + lane;
+        for (uint64_t p = ck; p < ce && have < need; p += 32) {
+          const uint64_t idx = p + lane;
           bool hit = false;
           if (idx < ce) {
             const uint32_t bit = g.adj[idx] - nbase;

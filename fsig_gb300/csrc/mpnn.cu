@@ -372,7 +372,7 @@ __global__ void mpnn_features_kernel(const QVert* __restrict__ qv, uint32_t G, c
     const QVert& x = qv[gi];
     uint32_t lo = 0, hi = Q;  // query of gi: last q with qoff[q] <= gi
     while (hi - lo > 1) {
-      const uint32_t mid = (lo + hi) >> 1;
+      const uint32_t mid = midpoint(lo, hi);
       if (qoff[mid] <= gi) lo = mid; else hi = mid;
     }
     const uint32_t g0 = qoff[lo], n = qoff[lo + 1] - g0;

@@ -36,17 +36,17 @@ __device__ __forceinline__ uint32_t edge_label(int32_t a, int32_t b) {
 __global__ void rows_kernel(const uint32_t* __restrict__ off, uint32_t V, uint32_t* __restrict__ row) {
   const uint32_t lane = threadIdx.x & 31;
   for (uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < V; v += (gridDim.x * blockDim.x) >> 5)
-    for (uint32_t e = off[v] + lane; e < off[v + 1]; e += 32) row[e] = v;
+    for (uint64_t e = uint64_t(off[v]) + lane; e < off[v + 1]; e += 32) row[e] = v;  // ends up to 2^32 - 1
 }
 
 __global__ void units_kernel(const int32_t* __restrict__ lab, const uint32_t* __restrict__ row,
                              const uint32_t* __restrict__ adj, uint32_t n, uint32_t* __restrict__ unit) {
-  for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x)
+  for (uint64_t e = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < n; e += uint64_t(gridDim.x) * blockDim.x)
     unit[e] = edge_label(lab[row[e]], lab[adj[e]]);
 }
 
 __global__ void iota_kernel(uint32_t* __restrict__ p, uint32_t n) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) p[i] = i;
+  for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += uint64_t(gridDim.x) * blockDim.x) p[i] = i;
 }
 
 // zero[t] = 1 when bit `bit` of the sort key of element perm[t] is 0.  The
@@ -54,7 +54,7 @@ __global__ void iota_kernel(uint32_t* __restrict__ p, uint32_t n) {
 __global__ void zero_flags_kernel(const uint32_t* __restrict__ perm, uint32_t n, const uint32_t* __restrict__ lo,
                                   const uint32_t* __restrict__ hi, uint32_t lo_bits, uint32_t bit,
                                   uint32_t* __restrict__ zero) {
-  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+  for (uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < n; t += uint64_t(gridDim.x) * blockDim.x) {
     const uint32_t x = perm[t];
     const uint32_t v = bit < lo_bits ? (lo[x] >> bit) : (hi[x] >> (bit - lo_bits));
     zero[t] = (v & 1u) ? 0u : 1u;
@@ -66,14 +66,14 @@ __global__ void partition_kernel(const uint32_t* __restrict__ perm, uint32_t n, 
                                  const uint32_t* __restrict__ zpos, const uint32_t* __restrict__ zeros_total,
                                  uint32_t* __restrict__ out) {
   const uint32_t Z = *zeros_total;
-  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
+  for (uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < n; t += uint64_t(gridDim.x) * blockDim.x)
     out[zero[t] ? zpos[t] : Z + (t - zpos[t])] = perm[t];
 }
 
 // Key starts among the entries sorted by (unit, row).
 __global__ void key_flags_kernel(const uint32_t* __restrict__ perm, uint32_t n, const uint32_t* __restrict__ unit,
                                  const uint32_t* __restrict__ row, uint32_t* __restrict__ flag) {
-  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+  for (uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < n; t += uint64_t(gridDim.x) * blockDim.x) {
     const uint32_t x = perm[t];
     bool s = t == 0;
     if (!s) {
@@ -88,7 +88,7 @@ __global__ void keys_kernel(const uint32_t* __restrict__ perm, uint32_t n, const
                             const uint32_t* __restrict__ kid, const uint32_t* __restrict__ unit,
                             const uint32_t* __restrict__ row, uint32_t* __restrict__ kpos,
                             uint32_t* __restrict__ kunit, uint32_t* __restrict__ kvert) {
-  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+  for (uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < n; t += uint64_t(gridDim.x) * blockDim.x) {
     if (!flag[t]) continue;
     const uint32_t k = kid[t], x = perm[t];
     kpos[k] = t;
@@ -185,7 +185,7 @@ __global__ void bucket_flags_kernel(const uint32_t* __restrict__ size, uint32_t 
 __device__ __forceinline__ uint32_t unit_of(const uint32_t* __restrict__ ubase, uint32_t U, uint32_t i) {
   uint32_t lo = 0, hi = U;  // last u with ubase[u] <= i
   while (hi - lo > 1) {
-    const uint32_t mid = (lo + hi) >> 1;
+    const uint32_t mid = midpoint(lo, hi);
     if (ubase[mid] <= i) lo = mid; else hi = mid;
   }
   return lo;
