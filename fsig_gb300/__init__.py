@@ -129,6 +129,7 @@ def engine_library() -> C.CDLL:
     L.fsig_last_stats.argtypes = [vp, C.POINTER(_Stats)]
     L.fsig_filter_noalloc.argtypes = [vp, C.POINTER(_Query), C.c_int, C.c_void_p]
     L.fsig_set_queue_waits.argtypes = [vp, C.c_uint64, C.c_uint64, C.c_int]
+    L.fsig_set_queue_test.argtypes = [vp, C.c_uint32]
     L.fsig_set_segment_index.argtypes = [vp, C.c_int]
     L.fsig_graph_layout.argtypes = [vp, C.POINTER(C.c_int), C.POINTER(C.c_uint64)]
     L.fsig_match_range.argtypes = [vp, C.POINTER(_Query), C.c_int, C.c_uint32, C.c_uint32, C.c_uint32,
@@ -154,7 +155,7 @@ def engine_library() -> C.CDLL:
     L.fsig_write_embeddings.argtypes = [vp, C.POINTER(_Query), C.c_int, C.c_char_p, C.POINTER(_Result)]
     for name in ("fsig_mpnn_set_params", "fsig_mpnn_get_params", "fsig_mpnn_features", "fsig_mpnn_forward",
                  "fsig_mpnn_train_step", "fsig_read_graph_file", "fsig_read_graph_file_threads", "fsig_save_graph_cache", "fsig_load_graph_cache", "fsig_graph_file_data", "fsig_match_embeddings",
-                 "fsig_write_embeddings", "fsig_build_pcsr", "fsig_filter_noalloc", "fsig_set_queue_waits", "fsig_set_segment_index", "fsig_graph_layout", "fsig_match_range", "fsig_last_stats", "fsig_plan_order", "fsig_create", "fsig_destroy", "fsig_load_graph", "fsig_load_graph_file", "fsig_graph_info",
+                 "fsig_write_embeddings", "fsig_build_pcsr", "fsig_filter_noalloc", "fsig_set_queue_waits", "fsig_set_queue_test", "fsig_set_segment_index", "fsig_graph_layout", "fsig_match_range", "fsig_last_stats", "fsig_plan_order", "fsig_create", "fsig_destroy", "fsig_load_graph", "fsig_load_graph_file", "fsig_graph_info",
                  "fsig_match", "fsig_match_batch", "fsig_build_csr", "fsig_build_signature", "fsig_filter",
                  "fsig_filter_classes", "fsig_refine_classes"):
         getattr(L, name).restype = C.c_int
@@ -560,6 +561,10 @@ class Engine:
         unpublished (fault injection for tests: the call returns ETIMEOUT)."""
         self._check(self._L.fsig_set_queue_waits(self._h, int(ready_wait_ns), int(idle_wait_ns), int(unpublished)),
                     "set_queue_waits")
+
+    def set_queue_test(self, first_record: int = 0) -> None:
+        """Test hook: numbers the queue's records from first_record on (0: off)."""
+        self._check(self._L.fsig_set_queue_test(self._h, int(first_record)), "set_queue_test")
 
     def match_range(self, q: Query, algo: int = ALGO_FSIG, task_begin: int = 0, task_end: int = 0xFFFFFFFF,
                     split_len: int = 0):

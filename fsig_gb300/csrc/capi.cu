@@ -506,6 +506,12 @@ int fsig_set_queue_waits(fsig_engine* h, uint64_t ready_wait_ns, uint64_t idle_w
   return FSIG_OK;
 }
 
+int fsig_set_queue_test(fsig_engine* h, uint32_t first_record) {
+  if (!h) return FSIG_EINVAL;
+  h->e.queue_first_record = first_record;
+  return FSIG_OK;
+}
+
 int fsig_plan_order(const fsig_query* q, int algo, const uint32_t* cand, uint32_t* order, uint32_t* types,
                     uint32_t* classes) {
   fsig::clear_thread_error();

@@ -70,6 +70,8 @@
 // broadcast.
 #pragma once
 
+#include "queue.cuh"
+
 namespace fsig {
 namespace {
 
@@ -97,7 +99,6 @@ struct EnumArgs {
   // work queue
   TaskRec* out_tasks;
   uint32_t* out_ready;
-  uint32_t out_cap;  // a power of two
   uint32_t* ctr;  // counters, kCtrStride apart: [0] input grab, [1] queue tail (records reserved) and,
                   // in the next word, tickets taken, [2] warps at work + records not taken yet,
                   // [3] error bits, [4] fault injection's one-shot, [5] once a waiting warp has left,
@@ -128,14 +129,10 @@ struct EnumArgs {
 
 constexpr uint32_t kErrTimeout = 1u;
 constexpr uint32_t kCtrStride = 32;        // one 128-byte line per counter
-// The queue is a ring: record number t lies in slot t mod out_cap, use
-// g = t / out_cap of that slot.  The slot's ready word is 2g while it is free
-// for that use, 2g + 1 from the record's publication until its ticket holder
-// has read it, then 2g + 2 (= free for use g + 1).  Records are reserved only
-// while warps wait, so at most (warps) x (records of one hand-off, up to 32 +
-// kLastBuf) numbers lie between the tickets and the tail, fewer than the ring's
-// 2^20 slots: a
-// reserved slot's previous record always has a ticket holder.
+// Records (queue.cuh) are reserved only while warps wait, so at most (warps) x
+// (records of one hand-off, up to 32 + kLastBuf) numbers lie between the tickets
+// and the tail, fewer than the ring's 2^20 slots: a reserved slot's previous
+// record always has a ticket holder.
 
 __device__ __forceinline__ unsigned long long global_ns() {
   unsigned long long t;
@@ -348,25 +345,24 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
     const uint32_t pieces = piece_count(rest, hand);
     const uint32_t first = part ? i_l + 1 : i_l;
     const uint32_t total = pieces + (c_l - first);
-    uint32_t base = 0;
+    uint32_t base = 0;  // any number, 2^32 - 1 too
+    bool full = false;
     if (lane == 0) {
       const uint32_t limit = *(volatile uint32_t*)&A.ctr[5 * kCtrStride];
-      if (limit && *(volatile uint32_t*)&A.ctr[1 * kCtrStride] + total > limit) {
-        base = kInvalid;
-      } else {
+      full = limit && queue_after(*(volatile uint32_t*)&A.ctr[1 * kCtrStride] + total, limit);
+      if (!full) {
         base = atomicAdd(&A.ctr[1 * kCtrStride], total);
         atomicAdd(&A.ctr[2 * kCtrStride], total);
       }
     }
+    if (__any_sync(kFull, full)) return false;
     base = __shfl_sync(kFull, base, 0);
-    if (base == kInvalid) return false;
     // the slots' previous records are read by now, or about to be (see above)
     {
-      const uint32_t mask = A.out_cap - 1, shift = 31 - __clz(A.out_cap);
       const unsigned long long t0 = global_ns();
 #pragma unroll 1
-      for (uint32_t k = base + lane; k < base + total; k += 32) {
-        while (*(volatile uint32_t*)&A.out_ready[k & mask] != 2 * (k >> shift)) {
+      for (uint32_t k = lane; k < total; k += 32) {
+        while (*(volatile uint32_t*)&A.out_ready[queue_slot(base + k)] != ready_free(base + k)) {
           if (global_ns() - t0 > A.ready_wait_ns) {
             atomicOr(&A.ctr[3 * kCtrStride], kErrTimeout);
             break;
@@ -378,13 +374,13 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
     uint32_t slot = base;
 #pragma unroll 1
     for (uint32_t k = 0; k < pieces; k++) {
-      TaskRec* r = A.out_tasks + (slot++ & (A.out_cap - 1));
+      TaskRec* r = A.out_tasks + queue_slot(slot++);
       if (lane <= l) r->f[lane] = fp;
       if (lane == 0) { r->q = ws.query; r->d = l + 1; r->lo = lo + k * hand; r->hi = piece_end(lo + k * hand, hand, hi); }
     }
 #pragma unroll 1
     for (uint32_t k = first; k < c_l; k++) {
-      TaskRec* r = A.out_tasks + (slot++ & (A.out_cap - 1));
+      TaskRec* r = A.out_tasks + queue_slot(slot++);
       const uint32_t fk = prefix(l, k);
       if (lane <= l) r->f[lane] = fk;
       if (lane == 0) { r->q = ws.query; r->d = l + 1; r->lo = kInvalid; r->hi = kInvalid; }
@@ -400,9 +396,8 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
     if (A.unpublished && lane == 0) hold = atomicCAS(&A.ctr[4 * kCtrStride], 0u, 1u) == 0u;
     hold = __shfl_sync(kFull, hold, 0);
 #pragma unroll 1
-    for (uint32_t k = base + lane; k < base + total; k += 32)
-      if (!(hold && k == base))
-        atomicExch(&A.out_ready[k & (A.out_cap - 1)], 2 * (k >> (31 - __clz(A.out_cap))) + 1);
+    for (uint32_t k = lane; k < total; k += 32)
+      if (!(hold && k == 0)) atomicExch(&A.out_ready[queue_slot(base + k)], ready_published(base + k));
     if (lane == 0) {
       ws.ev[2]++;
       ws.ev[3] += total;
@@ -415,10 +410,10 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
   // alone and broadcast.
   auto waiting_warps = [&](uint32_t t_start) -> uint32_t {
     uint32_t w = 0;
-    if (lane == 0 && A.out_cap) {
+    if (lane == 0) {
       uint32_t tail, tickets;
       asm volatile("ld.volatile.global.v2.u32 {%0, %1}, [%2];" : "=r"(tail), "=r"(tickets) : "l"(A.ctr + kCtrStride));
-      if (int32_t(tickets - tail) > 0 && (long long)(uint32_t(clock()) - t_start) > A.budget) w = tickets - tail;
+      if (queue_after(tickets, tail) && (long long)(uint32_t(clock()) - t_start) > A.budget) w = tickets - tail;
     }
     return __shfl_sync(kFull, w, 0);
   };
@@ -843,26 +838,26 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
       }
     } else {
       // input exhausted: take a ticket and wait for its record while others work
-      uint32_t slot = kInvalid;
+      uint32_t mine = 0;
+      bool got = false;
       if (lane == 0) {
-        const uint32_t mine = atomicAdd(&A.ctr[1 * kCtrStride + 1], 1u);
+        mine = atomicAdd(&A.ctr[1 * kCtrStride + 1], 1u);
         atomicSub(&A.ctr[2 * kCtrStride], 1u);
         const unsigned long long t_idle = global_ns();
         unsigned long long t_reserved = 0;  // when the record of this ticket was first seen reserved
         uint32_t sleep_ns = 32;
-        volatile uint32_t* word = A.out_ready + (mine & (A.out_cap - 1));
-        const uint32_t published = 2 * (mine >> (31 - __clz(A.out_cap))) + 1;
+        volatile uint32_t* word = A.out_ready + queue_slot(mine);
 #pragma unroll 1
         for (;;) {
-          if (*word == published) {
-            slot = mine;
+          if (*word == ready_published(mine)) {
+            got = true;
             break;
           }
           // finished when nobody works and every record is taken
           if (*(volatile uint32_t*)&A.ctr[2 * kCtrStride] == 0 || *(volatile uint32_t*)&A.ctr[3 * kCtrStride]) break;
           const unsigned long long now = global_ns();
           const uint32_t tail = *(volatile uint32_t*)&A.ctr[1 * kCtrStride];
-          if (int32_t(tail - mine) > 0) {
+          if (queue_after(tail, mine)) {
             if (!t_reserved) {
               t_reserved = now;
             } else if (now - t_reserved > A.ready_wait_ns) {
@@ -872,20 +867,20 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
           } else if (now - t_idle >= A.idle_wait_ns) {
             // leave: this ticket's record, if it comes, waits for the next pass,
             // so no slot from here on may be used again
-            atomicCAS(&A.ctr[5 * kCtrStride], 0u, max(tail + A.out_cap / 2, 1u));
+            atomicCAS(&A.ctr[5 * kCtrStride], 0u, max(tail + kQueueSlots / 2, 1u));
             break;
           }
           __nanosleep(sleep_ns);
           if (sleep_ns < 1024) sleep_ns <<= 1;
         }
       }
-      slot = __shfl_sync(kFull, slot, 0);
-      if (slot != kInvalid) {
+      if (__any_sync(kFull, got)) {
+        mine = __shfl_sync(kFull, mine, 0);
         __threadfence();
         if (lane == 0) ws.ev[1]++;
-        rec = A.out_tasks + (slot & (A.out_cap - 1));
-        ready = A.out_ready + (slot & (A.out_cap - 1));
-        free_word = 2 * (slot >> (31 - __clz(A.out_cap))) + 2;
+        rec = A.out_tasks + queue_slot(mine);
+        ready = A.out_ready + queue_slot(mine);
+        free_word = ready_next(mine);
       }
     }
     if (rec) {

@@ -695,8 +695,6 @@ int filter_stage(Engine& e, const BatchLayout& b, uint32_t mode, int refine_iter
 }  // namespace
 
 namespace {
-constexpr uint32_t kOverflowCap = 1u << 20;  // slots of a pass's record ring (a power of two)
-
 // Records ev on s.  Inside a stream capture an ordinary record only orders
 // the capture; the external form makes it a node of the graph.
 cudaError_t record(cudaEvent_t ev, cudaStream_t s) {
@@ -747,9 +745,22 @@ __global__ void given_scores_kernel(const uint32_t* __restrict__ qoff, uint32_t 
   }
 }
 
-__global__ void ctr_init_kernel(uint32_t* ctr, uint32_t first_task, uint32_t active) {
-  for (uint32_t i = threadIdx.x; i < 8 * kCtrStride; i += blockDim.x)
-    ctr[i] = i == 0 ? first_task : (i == 2 * kCtrStride ? active : 0u);
+// The pass's counters; records and tickets are numbered from first_record on.
+__global__ void ctr_init_kernel(uint32_t* ctr, uint32_t first_task, uint32_t active, uint32_t first_record) {
+  for (uint32_t i = threadIdx.x; i < 8 * kCtrStride; i += blockDim.x) {
+    uint32_t x = 0;
+    if (i == 0) x = first_task;
+    if (i == kCtrStride || i == kCtrStride + 1) x = first_record;  // the tail, the tickets
+    if (i == 2 * kCtrStride) x = active;
+    ctr[i] = x;
+  }
+}
+
+// Ready words of a queue whose records are numbered from `first` on (from 0 on
+// they are all zero).
+__global__ void ready_init_kernel(uint32_t* ready, uint32_t first) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < kQueueSlots; i += gridDim.x * blockDim.x)
+    ready[i] = ready_free(first + queue_slot(i - first));
 }
 
 // Records of a finished pass that no warp took (waiting warps left before
@@ -812,10 +823,10 @@ int enum_prepare(Engine& e, const BatchOptions& opt, const GraphView& gv, const 
                  const uint32_t* d_nroots, uint32_t split, QueryResult* d_res, unsigned long long* d_misc,
                  unsigned long long* d_ev, uint32_t* d_emit, unsigned long long* d_emit_ctr, uint32_t* h_ctr,
                  EnumRun& R) {
-  TaskRec* qa = e.arena.take<TaskRec>(kOverflowCap);
-  TaskRec* qb = e.arena.take<TaskRec>(kOverflowCap);
-  uint32_t* ra = e.arena.take<uint32_t>(kOverflowCap);
-  uint32_t* rb = e.arena.take<uint32_t>(kOverflowCap);
+  TaskRec* qa = e.arena.take<TaskRec>(kQueueSlots);
+  TaskRec* qb = e.arena.take<TaskRec>(kQueueSlots);
+  uint32_t* ra = e.arena.take<uint32_t>(kQueueSlots);
+  uint32_t* rb = e.arena.take<uint32_t>(kQueueSlots);
   R.ctr = e.arena.take<uint32_t>(8 * kCtrStride);
   if (!qa || !qb || !ra || !rb || !R.ctr)
     return fail(FSIG_EADMISSION, "work queues do not fit the device arena");
@@ -847,7 +858,6 @@ int enum_prepare(Engine& e, const BatchOptions& opt, const GraphView& gv, const 
   A.in_tasks = nullptr;
   A.in_index = nullptr;
   A.in_count = 0;
-  A.out_cap = kOverflowCap;
   A.ctr = R.ctr;
   A.chunk = std::max<uint32_t>(opt.chunk, 1);
   A.budget = (long long)opt.budget_cycles;
@@ -870,8 +880,9 @@ int enum_launch(Engine& e, EnumRun& R) {
   cudaStream_t s = e.stream;
   R.A.out_tasks = R.out;
   R.A.out_ready = R.ready;
-  FSIG_CUDA_TRY(cudaMemsetAsync(R.ready, 0, sizeof(uint32_t) * kOverflowCap, s));
-  ctr_init_kernel<<<1, 256, 0, s>>>(R.ctr, R.pass == 0 ? R.first_task : 0u, R.active);
+  if (e.queue_first_record) ready_init_kernel<<<e.num_sms, 256, 0, s>>>(R.ready, e.queue_first_record);
+  else FSIG_CUDA_TRY(cudaMemsetAsync(R.ready, 0, sizeof(uint32_t) * kQueueSlots, s));
+  ctr_init_kernel<<<1, 256, 0, s>>>(R.ctr, R.pass == 0 ? R.first_task : 0u, R.active, e.queue_first_record);
   FSIG_CUDA_TRY(cudaGetLastError());
   FSIG_CUDA_TRY(record(e.ev_enum[0], s));
   if (R.A.g.lseg) enumerate_kernel<false><<<R.grid, R.block, R.smem, s>>>(R.A);
@@ -895,7 +906,7 @@ int enum_after(Engine& e, EnumRun& R, bool& more, float& ms_enum, uint64_t& d2h)
   if (!more) return FSIG_OK;
   // the records nobody took become the next pass's input
   uint32_t* count = R.ctr + 7 * kCtrStride;
-  untaken_kernel<<<1, 256, 0, e.stream>>>(R.ready, kOverflowCap, count);
+  untaken_kernel<<<1, 256, 0, e.stream>>>(R.ready, kQueueSlots, count);
   FSIG_CUDA_TRY(cudaGetLastError());
   FSIG_CUDA_TRY(cudaMemcpyAsync(R.h_ctr, count, sizeof(uint32_t), cudaMemcpyDeviceToHost, e.stream));
   FSIG_CUDA_TRY(cudaStreamSynchronize(e.stream));

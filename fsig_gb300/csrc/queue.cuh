@@ -1,0 +1,25 @@
+// Numbers, slots and ready words of the enumeration's queue of handed-off
+// records, shared by the kernel, the host code and host tests.
+//
+// The queue is a ring: record number t lies in slot t mod kQueueSlots, use
+// t / kQueueSlots of that slot.  Its ready word says free for that use, then
+// published until its ticket holder has read it, then free for the next use.
+// Numbers wrap from 2^32 - 1 to 0, and uses with them: the slot count divides
+// 2^32.
+#pragma once
+#include <stdint.h>
+
+namespace fsig {
+
+constexpr uint32_t kQueueSlots = 1u << 20;
+
+__host__ __device__ __forceinline__ uint32_t queue_slot(uint32_t number) { return number % kQueueSlots; }
+// the slot's ready word while it is free for record `number`, and from its publication on
+__host__ __device__ __forceinline__ uint32_t ready_free(uint32_t number) { return 2 * (number / kQueueSlots); }
+__host__ __device__ __forceinline__ uint32_t ready_published(uint32_t number) { return ready_free(number) + 1; }
+// once it is read: free for the slot's next record
+__host__ __device__ __forceinline__ uint32_t ready_next(uint32_t number) { return ready_free(number + kQueueSlots); }
+// whether number a comes after number b (they are less than 2^31 apart)
+__host__ __device__ __forceinline__ bool queue_after(uint32_t a, uint32_t b) { return int32_t(a - b) > 0; }
+
+}  // namespace fsig

@@ -8,7 +8,7 @@ from fsig_gb300 import _build
 def run(tmp_path, body: str) -> None:
     """`body` is the inside of main(); check(ok, line) counts failures."""
     src, exe = tmp_path / "t.cu", tmp_path / "t"
-    src.write_text('#include <cstdio>\n#include <cstdlib>\n#include <sys/mman.h>\n#include "common.cuh"\n'
+    src.write_text('#include <cstdio>\n#include <cstdlib>\n#include <sys/mman.h>\n#include "common.cuh"\n#include "queue.cuh"\n'
                    "static int bad = 0;\n"
                    "static void check(bool ok, int line) { if (!ok) { bad++; std::printf(\"line %d\\n\", line); } }\n"
                    "#define CHECK(x) check((x), __LINE__)\nusing namespace fsig;\n"

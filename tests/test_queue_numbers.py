@@ -1,0 +1,21 @@
+"""Record numbers of the enumeration's queue, on the host: the ready words of
+one slot's uses follow each other, across the wrap from 2^32 - 1 to 0 too."""
+import hostcu
+
+
+def test_ready_words_across_the_wrap(tmp_path):
+    hostcu.run(tmp_path, r"""
+  const uint32_t starts[] = {0u, 1u, kQueueSlots - 1, 5 * kQueueSlots + 77, 0u - kQueueSlots, 0u - 3u, 0xffffffffu};
+  for (uint32_t t : starts) {
+    uint32_t n = t;
+    for (int use = 0; use < 9000; use++, n += kQueueSlots) {  // past a whole turn of the uses
+      CHECK(queue_slot(n) == queue_slot(t));
+      CHECK(ready_published(n) == ready_free(n) + 1 && (ready_free(n) & 1u) == 0);
+      CHECK(ready_next(n) == ready_free(n + kQueueSlots));  // what the next writer of the slot waits for
+      CHECK(ready_next(n) != ready_free(n) && ready_next(n) != ready_published(n));
+    }
+    for (uint32_t d : {1u, 160u, kQueueSlots, 0x7fffffffu}) CHECK(queue_after(t + d, t) && !queue_after(t, t + d));
+    CHECK(!queue_after(t, t));
+  }
+  CHECK(ready_next(0xffffffffu) == 0 && ready_free(kQueueSlots - 1) == 0);
+""")
