@@ -103,6 +103,7 @@ struct EnumArgs {
                   // in the next word, tickets taken, [2] warps at work + records not taken yet,
                   // [3] error bits, [4] fault injection's one-shot, [5] once a waiting warp has left,
                   // the record number from which on no more are reserved
+  uint32_t room;  // queue_room of the launch's warps
   uint32_t chunk;
   long long budget;  // cycles on a task before it may be split while warps are idle
   QueryResult* res;
@@ -130,9 +131,9 @@ struct EnumArgs {
 constexpr uint32_t kErrTimeout = 1u;
 constexpr uint32_t kCtrStride = 32;        // one 128-byte line per counter
 // Records (queue.cuh) are reserved only while warps wait, so at most (warps) x
-// (records of one hand-off, up to 32 + kLastBuf) numbers lie between the tickets
-// and the tail, fewer than the ring's 2^20 slots: a reserved slot's previous
-// record always has a ticket holder.
+// (records of one hand-off) numbers lie between the tickets and the tail, fewer
+// than the ring's 2^20 slots: a reserved slot's previous record always has a
+// ticket holder, or one that left, whose slot does not come round (queue_room).
 
 __device__ __forceinline__ unsigned long long global_ns() {
   unsigned long long t;
@@ -151,6 +152,7 @@ constexpr uint32_t kBuf = 32;        // entries of a depth's buffer
 // 2^26 edges 11.6 ms, 12.5 with 128 always; nor while warps wait.
 constexpr uint32_t kLastBuf = 128;
 constexpr uint32_t kLongLeaf = 6;
+static_assert(kHandOff == 32 + kLastBuf, "a hand-off is a range's pieces and a buffer");
 constexpr uint32_t kScratch = 384;   // words for the segments and earlier vertices of the entries being extended
 // Candidate windows one fill examines before it returns, so that the periodic
 // checks and hand-offs come in time on long driver ranges.
@@ -865,9 +867,8 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
               break;
             }
           } else if (now - t_idle >= A.idle_wait_ns) {
-            // leave: this ticket's record, if it comes, waits for the next pass,
-            // so no slot from here on may be used again
-            atomicCAS(&A.ctr[5 * kCtrStride], 0u, max(tail + kQueueSlots / 2, 1u));
+            // leave: this ticket's record, if it comes, waits for the next pass
+            atomicCAS(&A.ctr[5 * kCtrStride], 0u, max(tail + A.room, 1u));
             break;
           }
           __nanosleep(sleep_ns);

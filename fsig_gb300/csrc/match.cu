@@ -833,7 +833,7 @@ int enum_prepare(Engine& e, const BatchOptions& opt, const GraphView& gv, const 
   const uint32_t wpb = std::max<uint32_t>(1, std::min<uint32_t>(opt.warps_per_block, kEnumWarps));
   const int per_sm = gv.lseg ? e.enum_per_sm[wpb] : e.enum_per_sm_rows[wpb];
   R.smem = sizeof(WarpSmem) * wpb;
-  R.grid = uint32_t(e.num_sms * per_sm);
+  R.grid = std::min(uint32_t(e.num_sms * per_sm), kQueueWarps / wpb);
   R.block = wpb * 32;
   R.active = R.grid * wpb;  // every warp starts active; idle warps are counted as they wait
   R.first_task = opt.task_begin;
@@ -859,6 +859,7 @@ int enum_prepare(Engine& e, const BatchOptions& opt, const GraphView& gv, const 
   A.in_index = nullptr;
   A.in_count = 0;
   A.ctr = R.ctr;
+  A.room = queue_room(R.active);
   A.chunk = std::max<uint32_t>(opt.chunk, 1);
   A.budget = (long long)opt.budget_cycles;
   A.res = d_res;

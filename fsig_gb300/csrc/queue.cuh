@@ -19,6 +19,18 @@ __host__ __device__ __forceinline__ uint32_t ready_free(uint32_t number) { retur
 __host__ __device__ __forceinline__ uint32_t ready_published(uint32_t number) { return ready_free(number) + 1; }
 // once it is read: free for the slot's next record
 __host__ __device__ __forceinline__ uint32_t ready_next(uint32_t number) { return ready_free(number + kQueueSlots); }
+// Records of one hand-off, at most: 32 pieces of a range and a buffer's entries.
+constexpr uint32_t kHandOff = 32 + 128;
+// The record of a warp that left is not read in the pass, so its slot must not
+// come round: once one has left, records are reserved only up to the tail of
+// that moment plus this.  Every warp may reserve one hand-off beyond (a warp
+// checks the limit, then adds), and hold one ticket beyond the records: a full
+// ring in all.  (Half a ring as the limit, right for hand-offs of up to 64
+// records, was not for 160: 4,864 warps reserve 778,240.)
+__host__ __device__ constexpr uint32_t queue_room(uint32_t warps) { return kQueueSlots - warps * (kHandOff + 1); }
+// Warps of one launch, at most; a GB300 holds 4,864.
+constexpr uint32_t kQueueWarps = kQueueSlots / 8 * 7 / (kHandOff + 1);
+
 // whether number a comes after number b (they are less than 2^31 apart)
 __host__ __device__ __forceinline__ bool queue_after(uint32_t a, uint32_t b) { return int32_t(a - b) > 0; }
 

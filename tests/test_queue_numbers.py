@@ -19,3 +19,18 @@ def test_ready_words_across_the_wrap(tmp_path):
   }
   CHECK(ready_next(0xffffffffu) == 0 && ready_free(kQueueSlots - 1) == 0);
 """)
+
+
+def test_room_after_a_warp_left(tmp_path):
+    # whatever the number of warps: the last number reserved and the last ticket
+    # stay within a ring of the first ticket given up
+    hostcu.run(tmp_path, r"""
+  CHECK(kQueueWarps >= 152 * 4 * 8);  // a GB300's resident warps
+  for (uint64_t w = 1; w <= kQueueWarps; w++) {
+    const uint64_t limit = queue_room(uint32_t(w));  // beyond the tail when the first warp left
+    CHECK(limit > 0 && limit < kQueueSlots);
+    const uint64_t tail = limit + w * kHandOff;      // every warp checked the limit, then reserved
+    CHECK(tail + w <= kQueueSlots);                  // and took a ticket
+    CHECK(w * kHandOff < kQueueSlots);               // numbers between tickets and tail
+  }
+""")
