@@ -359,19 +359,18 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
     }
     if (__any_sync(kFull, full)) return false;
     base = __shfl_sync(kFull, base, 0);
-    // the slots' previous records are read by now, or about to be (see above)
+    // the slots' previous records are read by now, or about to be (see above); a
+    // record that is not must not be written over while its holder may read it
     {
       const unsigned long long t0 = global_ns();
+      bool late = false;
 #pragma unroll 1
-      for (uint32_t k = lane; k < total; k += 32) {
-        while (*(volatile uint32_t*)&A.out_ready[queue_slot(base + k)] != ready_free(base + k)) {
-          if (global_ns() - t0 > A.ready_wait_ns) {
-            atomicOr(&A.ctr[3 * kCtrStride], kErrTimeout);
-            break;
-          }
-        }
+      for (uint32_t k = lane; k < total && !late; k += 32) {
+        while (!late && *(volatile uint32_t*)&A.out_ready[queue_slot(base + k)] != ready_free(base + k))
+          late = global_ns() - t0 > A.ready_wait_ns;
       }
-      __syncwarp();
+      if (late) atomicOr(&A.ctr[3 * kCtrStride], kErrTimeout);
+      if (__any_sync(kFull, late)) return false;
     }
     uint32_t slot = base;
 #pragma unroll 1
