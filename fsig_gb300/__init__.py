@@ -129,7 +129,7 @@ def engine_library() -> C.CDLL:
     L.fsig_last_stats.argtypes = [vp, C.POINTER(_Stats)]
     L.fsig_filter_noalloc.argtypes = [vp, C.POINTER(_Query), C.c_int, C.c_void_p]
     L.fsig_set_queue_waits.argtypes = [vp, C.c_uint64, C.c_uint64, C.c_int]
-    L.fsig_set_queue_test.argtypes = [vp, C.c_uint32]
+    L.fsig_set_queue_test.argtypes = [vp, C.c_uint32, C.c_int]
     L.fsig_set_segment_index.argtypes = [vp, C.c_int]
     L.fsig_graph_layout.argtypes = [vp, C.POINTER(C.c_int), C.POINTER(C.c_uint64)]
     L.fsig_match_range.argtypes = [vp, C.POINTER(_Query), C.c_int, C.c_uint32, C.c_uint32, C.c_uint32,
@@ -562,9 +562,10 @@ class Engine:
         self._check(self._L.fsig_set_queue_waits(self._h, int(ready_wait_ns), int(idle_wait_ns), int(unpublished)),
                     "set_queue_waits")
 
-    def set_queue_test(self, first_record: int = 0) -> None:
-        """Test hook: numbers the queue's records from first_record on (0: off)."""
-        self._check(self._L.fsig_set_queue_test(self._h, int(first_record)), "set_queue_test")
+    def set_queue_test(self, first_record: int = 0, first_leaves: bool = False) -> None:
+        """Test hooks: numbers the queue's records from first_record on (0: off);
+        first_leaves=True lets each pass's first waiting warp leave at once."""
+        self._check(self._L.fsig_set_queue_test(self._h, int(first_record), int(first_leaves)), "set_queue_test")
 
     def match_range(self, q: Query, algo: int = ALGO_FSIG, task_begin: int = 0, task_end: int = 0xFFFFFFFF,
                     split_len: int = 0):

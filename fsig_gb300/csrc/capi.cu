@@ -506,9 +506,10 @@ int fsig_set_queue_waits(fsig_engine* h, uint64_t ready_wait_ns, uint64_t idle_w
   return FSIG_OK;
 }
 
-int fsig_set_queue_test(fsig_engine* h, uint32_t first_record) {
-  if (!h) return FSIG_EINVAL;
+int fsig_set_queue_test(fsig_engine* h, uint32_t first_record, int first_leaves) {
+  if (!h || (first_leaves != 0 && first_leaves != 1)) return FSIG_EINVAL;
   h->e.queue_first_record = first_record;
+  h->e.inject_first_leaves = uint32_t(first_leaves);
   return FSIG_OK;
 }
 

@@ -72,6 +72,7 @@ struct Engine {
   uint64_t idle_wait_ns = 2000000000ull;   // an idle warp waiting for hand-offs: 2 s
   uint32_t inject_unpublished = 0;         // test hook: leave each pass's first hand-off unpublished
   uint32_t queue_first_record = 0;         // test hook: number of each pass's first record
+  uint32_t inject_first_leaves = 0;        // test hook: each pass's first waiting warp leaves at once
 };
 
 // Parts of one device block and its image in the staging area, each part at a

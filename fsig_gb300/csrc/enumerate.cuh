@@ -100,7 +100,8 @@ struct EnumArgs {
   TaskRec* out_tasks;
   uint32_t* out_ready;
   uint32_t* ctr;  // counters, kCtrStride apart: [0] input grab, [1] queue tail (records reserved) and,
-                  // in the next word, tickets taken, [2] warps at work + records not taken yet,
+                  // in the next word, tickets taken, [2] warps at work + records not taken yet and,
+                  // in the next word, records whose holders left (not counted in the former),
                   // [3] error bits, [4] fault injection's one-shot, [5] once a waiting warp has left,
                   // the record number from which on no more are reserved
   uint32_t room;  // queue_room of the launch's warps
@@ -126,6 +127,9 @@ struct EnumArgs {
   // written but never published, so the warp that takes it waits out
   // ready_wait_ns and the pass reports a timeout
   uint32_t unpublished;
+  // for tests: number of the pass's first record and ticket; whether the warp
+  // that takes that ticket leaves at once
+  uint32_t first_record, first_leaves;
 };
 
 constexpr uint32_t kErrTimeout = 1u;
@@ -366,7 +370,7 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
       bool late = false;
 #pragma unroll 1
       for (uint32_t k = lane; k < total && !late; k += 32) {
-        while (!late && *(volatile uint32_t*)&A.out_ready[queue_slot(base + k)] != ready_free(base + k))
+        while (!late && !ready_writable(*(volatile uint32_t*)&A.out_ready[queue_slot(base + k)], base + k))
           late = global_ns() - t0 > A.ready_wait_ns;
       }
       if (late) atomicOr(&A.ctr[3 * kCtrStride], kErrTimeout);
@@ -396,10 +400,16 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
     int hold = 0;  // test hook: keep the pass's first handed-off record unpublished
     if (A.unpublished && lane == 0) hold = atomicCAS(&A.ctr[4 * kCtrStride], 0u, 1u) == 0u;
     hold = __shfl_sync(kFull, hold, 0);
+    uint32_t left = 0;  // records whose holders left
 #pragma unroll 1
     for (uint32_t k = lane; k < total; k += 32)
-      if (!(hold && k == 0)) atomicExch(&A.out_ready[queue_slot(base + k)], ready_published(base + k));
+      if (!(hold && k == 0)) left += atomicOr(&A.out_ready[queue_slot(base + k)], 1u) >> 31;
+    left = __reduce_add_sync(kFull, left);
     if (lane == 0) {
+      if (left) {  // the next pass's: nobody here has to wait for them
+        atomicAdd(&A.ctr[2 * kCtrStride + 1], left);
+        atomicSub(&A.ctr[2 * kCtrStride], left);
+      }
       ws.ev[2]++;
       ws.ev[3] += total;
     }
@@ -865,10 +875,16 @@ __global__ void __launch_bounds__(kEnumWarps * 32, kEnumMinBlocks) enumerate_ker
               atomicOr(&A.ctr[3 * kCtrStride], kErrTimeout);
               break;
             }
-          } else if (now - t_idle >= A.idle_wait_ns) {
-            // leave: this ticket's record, if it comes, waits for the next pass
+          } else if (now - t_idle >= (A.first_leaves && mine == A.first_record ? 0ull : A.idle_wait_ns)) {
+            // leave: this ticket's record, if it comes, waits for the next pass.
+            // (Unmarked, such a record kept the counter from zero: every other
+            // waiting warp then waited out its own idle_wait at the pass's end.)
             atomicCAS(&A.ctr[5 * kCtrStride], 0u, max(tail + A.room, 1u));
-            break;
+            const uint32_t was =
+                atomicCAS(const_cast<uint32_t*>(word), ready_free(mine), ready_free(mine) | kHolderLeft);
+            if (was == ready_free(mine)) break;
+            // published meanwhile, or the slot's previous record is still being read
+            if (now - t_idle >= A.idle_wait_ns + A.ready_wait_ns && was != ready_published(mine)) break;
           }
           __nanosleep(sleep_ns);
           if (sleep_ns < 1024) sleep_ns <<= 1;

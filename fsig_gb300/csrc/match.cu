@@ -870,6 +870,8 @@ int enum_prepare(Engine& e, const BatchOptions& opt, const GraphView& gv, const 
   A.ready_wait_ns = e.ready_wait_ns;
   A.idle_wait_ns = e.idle_wait_ns;
   A.unpublished = e.inject_unpublished;
+  A.first_record = e.queue_first_record;
+  A.first_leaves = e.inject_first_leaves;
   R.out = qa;
   R.ready = ra;
   R.other = qb;
@@ -903,7 +905,8 @@ int enum_after(Engine& e, EnumRun& R, bool& more, float& ms_enum, uint64_t& d2h)
   d2h += sizeof(uint32_t) * 4 * kCtrStride;
   const uint32_t* hc = R.h_ctr;
   if (hc[3 * kCtrStride] & kErrTimeout) return fail(FSIG_ETIMEOUT, "a work-queue record was not published in time");
-  more = hc[2 * kCtrStride] != 0;
+  const uint32_t left = hc[2 * kCtrStride] + hc[2 * kCtrStride + 1];
+  more = left != 0;
   if (!more) return FSIG_OK;
   // the records nobody took become the next pass's input
   uint32_t* count = R.ctr + 7 * kCtrStride;
@@ -911,7 +914,7 @@ int enum_after(Engine& e, EnumRun& R, bool& more, float& ms_enum, uint64_t& d2h)
   FSIG_CUDA_TRY(cudaGetLastError());
   FSIG_CUDA_TRY(cudaMemcpyAsync(R.h_ctr, count, sizeof(uint32_t), cudaMemcpyDeviceToHost, e.stream));
   FSIG_CUDA_TRY(cudaStreamSynchronize(e.stream));
-  if (R.h_ctr[0] != hc[2 * kCtrStride]) return fail(FSIG_EOVERFLOW, "task records were lost");
+  if (R.h_ctr[0] != left) return fail(FSIG_EOVERFLOW, "task records were lost");
   R.A.in_tasks = R.out;
   R.A.in_index = R.ready;
   R.A.in_count = R.h_ctr[0];

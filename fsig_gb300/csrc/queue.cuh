@@ -3,7 +3,9 @@
 //
 // The queue is a ring: record number t lies in slot t mod kQueueSlots, use
 // t / kQueueSlots of that slot.  Its ready word says free for that use, then
-// published until its ticket holder has read it, then free for the next use.
+// published until its ticket holder has read it, then free for the next use.  A
+// holder that leaves before its record is reserved marks the word: the record,
+// if it is written, is nobody's in this pass.
 // Numbers wrap from 2^32 - 1 to 0, and uses with them: the slot count divides
 // 2^32.
 #pragma once
@@ -30,6 +32,12 @@ constexpr uint32_t kHandOff = 32 + 128;
 __host__ __device__ constexpr uint32_t queue_room(uint32_t warps) { return kQueueSlots - warps * (kHandOff + 1); }
 // Warps of one launch, at most; a GB300 holds 4,864.
 constexpr uint32_t kQueueWarps = kQueueSlots / 8 * 7 / (kHandOff + 1);
+
+// added to the free word by a holder that left; publishing sets the low bit only
+constexpr uint32_t kHolderLeft = 0x80000000u;
+__host__ __device__ __forceinline__ bool ready_writable(uint32_t word, uint32_t number) {
+  return (word & ~kHolderLeft) == ready_free(number);
+}
 
 // whether number a comes after number b (they are less than 2^31 apart)
 __host__ __device__ __forceinline__ bool queue_after(uint32_t a, uint32_t b) { return int32_t(a - b) > 0; }

@@ -280,9 +280,11 @@ int fsig_last_stats(const fsig_engine* e, fsig_batch_stats* out);
  *      FSIG_ETIMEOUT without faulting the GPU; 0 turns it off.  Waits are
  *      limited to 60 s. ---- */
 int fsig_set_queue_waits(fsig_engine* e, uint64_t ready_wait_ns, uint64_t idle_wait_ns, int unpublished);
-/* For tests of what takes a very long pass: the queue's records are numbered
- * from first_record on in later passes (0: off).  Results do not depend on it. */
-int fsig_set_queue_test(fsig_engine* e, uint32_t first_record);
+/* For tests of what takes a very long pass: in later passes the queue's records
+ * are numbered from first_record on (0: off), and with first_leaves = 1 the first
+ * warp that waits for one leaves at once, whatever idle_wait_ns, so that one
+ * record is left for a later pass.  Results do not depend on either. */
+int fsig_set_queue_test(fsig_engine* e, uint32_t first_record, int first_leaves);
 
 /* ---- transforms with the reference's output layout, built on the device ---- */
 /* UndirectedPlainToCSRTransformer::transform (graph_format_transformer.cc:12-37):

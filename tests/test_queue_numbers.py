@@ -13,6 +13,11 @@ def test_ready_words_across_the_wrap(tmp_path):
       CHECK(ready_published(n) == ready_free(n) + 1 && (ready_free(n) & 1u) == 0);
       CHECK(ready_next(n) == ready_free(n + kQueueSlots));  // what the next writer of the slot waits for
       CHECK(ready_next(n) != ready_free(n) && ready_next(n) != ready_published(n));
+      // a holder that left: the record may still be written, then counts as published, and is never taken
+      const uint32_t gone = ready_free(n) | kHolderLeft;
+      CHECK(ready_writable(ready_free(n), n) && ready_writable(gone, n) && !ready_writable(ready_published(n), n));
+      CHECK(((gone | 1u) & 1u) && (gone | 1u) != ready_published(n) && (ready_free(n) | 1u) == ready_published(n));
+      CHECK(!ready_writable(gone | 1u, n) && (ready_published(n) >> 31) == 0);
     }
     for (uint32_t d : {1u, 160u, kQueueSlots, 0x7fffffffu}) CHECK(queue_after(t + d, t) && !queue_after(t, t + d));
     CHECK(!queue_after(t, t));
