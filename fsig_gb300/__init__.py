@@ -465,6 +465,19 @@ def _results(res, count: int) -> list:
             for c, h, st, n, o, ca, lv, mf, mj, w in zip(*cols)]
 
 
+def _results_of(count: int) -> np.ndarray:
+    """Zeroed words for a call's results, every page of them touched: a copy
+    from the GPU into heap pages that never were faults them in one by one (8 MB
+    in 8 ms instead of 0.4, 19 MB in 17 ms instead of 0.3; touched here in 0.3
+    and 0.7).  The C library gives 32 MB and more a mapping of its own, where a
+    copy of 64 MB into fresh pages takes 3.4 ms, touching them first 2.2 + 1.8."""
+    a = np.zeros(count, np.uint32)
+    if a.nbytes < 32 << 20:
+        a[::1024] = 0
+        a[-1:] = 0
+    return a
+
+
 class Engine:
     """One device arena on one GPU; replaces init_GPU + MemoryManager."""
 
@@ -589,8 +602,8 @@ class Engine:
     def build_csr(self, V: int, edges: np.ndarray):
         e = np.ascontiguousarray(edges, np.uint32).reshape(-1)
         E = e.size // 2
-        off = np.zeros(V + 1, np.uint32)
-        adj = np.zeros(max(2 * E, 1), np.uint32)
+        off = _results_of(V + 1)
+        adj = _results_of(max(2 * E, 1))
         if e.size == 0:
             e = np.zeros(2, np.uint32)
         self._check(self._L.fsig_build_csr(self._h, V, E, _u32p(e), _u32p(off), _u32p(adj)), "build_csr")
@@ -602,7 +615,7 @@ class Engine:
         a = np.ascontiguousarray(adj, np.uint32)
         if a.size == 0:
             a = np.zeros(1, np.uint32)
-        out = np.zeros(16 * len(lab), np.uint32)
+        out = _results_of(16 * len(lab))
         self._check(self._L.fsig_build_signature(self._h, len(lab), _i32p(lab), _u32p(off), _u32p(a),
                                                  1 if column_oriented else 0, _u32p(out)), "build_signature")
         return out
@@ -610,7 +623,8 @@ class Engine:
     def build_pcsr(self, labels, offsets, adj, num_labels: int) -> list:
         """The reference's PCSR units, built on the device: a list of
         (keys, list entries, slot table, lists) per unit, as the oracle's pcsr();
-        the arrays of all units are parts of two arrays of this call."""
+        the arrays of all units are parts of two arrays of this call, which live
+        as long as one of them does (copy a unit to keep it alone)."""
         lab = np.ascontiguousarray(labels, np.int32)
         off = np.ascontiguousarray(offsets, np.uint32)
         a = np.ascontiguousarray(adj, np.uint32)
@@ -621,8 +635,8 @@ class Engine:
         ne = np.zeros(max(U, 1), np.uint32)
         self._check(self._L.fsig_build_pcsr(self._h, len(lab), num_labels, _i32p(lab), _u32p(off), _u32p(a),
                                             _u32p(keys), _u32p(ne), None, None), "build_pcsr")
-        table = np.zeros(max(int(keys[:U].sum()) * 32, 1), np.uint32)
-        edges = np.zeros(max(int(ne[:U].sum()), 1), np.uint32)
+        table = _results_of(max(int(keys[:U].sum()) * 32, 1))
+        edges = _results_of(max(int(ne[:U].sum()), 1))
         self._check(self._L.fsig_build_pcsr(self._h, len(lab), num_labels, _i32p(lab), _u32p(off), _u32p(a),
                                             _u32p(keys), _u32p(ne), _u32p(table), _u32p(edges)), "build_pcsr")
         units, ob, eb = [], 0, 0
