@@ -132,6 +132,7 @@ def engine_library() -> C.CDLL:
     L.fsig_set_queue_test.argtypes = [vp, C.c_uint32, C.c_int]
     L.fsig_set_segment_index.argtypes = [vp, C.c_int]
     L.fsig_graph_layout.argtypes = [vp, C.POINTER(C.c_int), C.POINTER(C.c_uint64)]
+    L.fsig_graph_filter.argtypes = [vp, C.POINTER(C.c_uint64)]
     L.fsig_match_range.argtypes = [vp, C.POINTER(_Query), C.c_int, C.c_uint32, C.c_uint32, C.c_uint32,
                                    C.POINTER(_Result), C.POINTER(C.c_uint32)]
     fp = C.POINTER(C.c_float)
@@ -155,7 +156,7 @@ def engine_library() -> C.CDLL:
     L.fsig_write_embeddings.argtypes = [vp, C.POINTER(_Query), C.c_int, C.c_char_p, C.POINTER(_Result)]
     for name in ("fsig_mpnn_set_params", "fsig_mpnn_get_params", "fsig_mpnn_features", "fsig_mpnn_forward",
                  "fsig_mpnn_train_step", "fsig_read_graph_file", "fsig_read_graph_file_threads", "fsig_save_graph_cache", "fsig_load_graph_cache", "fsig_graph_file_data", "fsig_match_embeddings",
-                 "fsig_write_embeddings", "fsig_build_pcsr", "fsig_filter_noalloc", "fsig_set_queue_waits", "fsig_set_queue_test", "fsig_set_segment_index", "fsig_graph_layout", "fsig_match_range", "fsig_last_stats", "fsig_plan_order", "fsig_create", "fsig_destroy", "fsig_load_graph", "fsig_load_graph_file", "fsig_graph_info",
+                 "fsig_write_embeddings", "fsig_build_pcsr", "fsig_filter_noalloc", "fsig_set_queue_waits", "fsig_set_queue_test", "fsig_set_segment_index", "fsig_graph_layout", "fsig_graph_filter", "fsig_match_range", "fsig_last_stats", "fsig_plan_order", "fsig_create", "fsig_destroy", "fsig_load_graph", "fsig_load_graph_file", "fsig_graph_info",
                  "fsig_match", "fsig_match_batch", "fsig_build_csr", "fsig_build_signature", "fsig_filter",
                  "fsig_filter_classes", "fsig_refine_classes"):
         getattr(L, name).restype = C.c_int
@@ -540,6 +541,14 @@ class Engine:
         mode, nbytes = C.c_int(), C.c_uint64()
         self._check(self._L.fsig_graph_layout(self._h, C.byref(mode), C.byref(nbytes)), "graph_layout")
         return dict(segment_index=mode.value, bytes=nbytes.value)
+
+    def graph_filter(self) -> int:
+        """Device bytes of the membership filter; 0 while there is none: no
+        room at the load, or a call took it back and no matching call since
+        found it free.  Results do not depend on it."""
+        n = C.c_uint64()
+        self._check(self._L.fsig_graph_filter(self._h, C.byref(n)), "graph_filter")
+        return n.value
 
     def graph_info(self) -> dict:
         V, nadj, L, md = C.c_uint32(), C.c_uint64(), C.c_int32(), C.c_uint32()

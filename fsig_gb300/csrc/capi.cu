@@ -244,6 +244,13 @@ int fsig_graph_layout(const fsig_engine* h, int* segment_index, uint64_t* bytes)
   return FSIG_OK;
 }
 
+int fsig_graph_filter(const fsig_engine* h, uint64_t* bytes) {
+  if (!h || !bytes) return FSIG_EINVAL;
+  if (!h->e.has_graph) return FSIG_ENOGRAPH;
+  *bytes = fsig::filter_bytes(h->e);
+  return FSIG_OK;
+}
+
 int fsig_match(fsig_engine* h, const fsig_query* q, int algo, fsig_result* out) {
   int rc = select(h);
   if (rc) return finish(h, rc);

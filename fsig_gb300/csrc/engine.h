@@ -37,7 +37,8 @@ struct DeviceGraph {
   uint32_t* adj_old = nullptr;     // [nadj] caller id of each adj entry (for the result hash); null without lseg
   uint32_t* lseg = nullptr;        // [V*(L+1)]; null: segments are found by binary search in the rows
   uint4* sig = nullptr;            // [V*4] 64-byte signature per vertex
-  uint16_t* filt = nullptr;        // [nadj << filter_shift(nadj)] membership filter, in the arena's tail; valid while that is kept
+  uint16_t* filt = nullptr;        // [nadj << filter_shift(nadj)] membership filter, in the arena's tail; valid while that is
+                                   // kept; null when there was no room for it at the load
   std::vector<uint32_t> h_base;    // host copy of base
   uint64_t arena_mark = 0;         // arena top after the graph store
 };
@@ -101,6 +102,10 @@ int reserve_pinned(Engine& e, size_t bytes);
 int build_device_graph(Engine& e, uint32_t V, const int32_t* labels, uint64_t E, const uint32_t* edges);
 bool use_segment_table(int mode, uint32_t V, int32_t L, uint64_t nadj);
 uint64_t store_bytes(const DeviceGraph& g);
+uint64_t filter_bytes(const Engine& e);  // of the membership filter, 0 while there is none
+// Builds a membership filter again whose room a call took back, if that is free
+// now; for a call that has taken every buffer it needs (stream-ordered).
+int restore_membership_filter(Engine& e, uint32_t* launches);
 int save_graph_cache(Engine& e, const char* path);
 // pcsr.cu
 int build_reference_pcsr(Engine& e, uint32_t V, int32_t L, const int32_t* labels, const uint32_t* off,

@@ -587,14 +587,12 @@ __global__ void max_row_kernel(const uint32_t* __restrict__ off, uint32_t V, uin
 // batch's work queues and room for a batch.
 constexpr uint64_t kFilterSpare = 1ull << 30;
 
-// The membership filter in the arena's tail, when there is room to spare;
-// without it the enumeration searches the segments themselves.
-int build_membership_filter(Engine& e, DeviceGraph& g) {
-  g.filt = nullptr;
-  if (!g.nadj) return FSIG_OK;
+// The membership filter in the arena's tail, when there is room for it and
+// `spare` bytes; without it the enumeration searches the segments themselves.
+int build_membership_filter(Engine& e, DeviceGraph& g, uint64_t spare) {
   const uint32_t shift = filter_shift(g.nadj);
   const uint64_t words32 = ((g.nadj << shift) + 1) / 2;
-  uint32_t* filt = e.arena.take_tail<uint32_t>(words32, kFilterSpare);
+  uint32_t* filt = words32 ? e.arena.take_tail<uint32_t>(words32, spare) : nullptr;
   if (!filt) return FSIG_OK;
   FSIG_CUDA_TRY(cudaMemsetAsync(filt, 0, sizeof(uint32_t) * words32, e.stream));
   membership_filter_kernel<<<grid_for((g.nadj + kFilterRun - 1) / kFilterRun * 32, 256, e.num_sms), 256, 0, e.stream>>>(
@@ -605,6 +603,17 @@ int build_membership_filter(Engine& e, DeviceGraph& g) {
 }
 
 }  // namespace
+
+uint64_t filter_bytes(const Engine& e) {
+  return e.has_graph && e.arena.tail ? (e.g.nadj << filter_shift(e.g.nadj)) * sizeof(uint16_t) : 0;
+}
+
+int restore_membership_filter(Engine& e, uint32_t* launches) {
+  if (!e.g.filt || e.arena.tail) return FSIG_OK;
+  const int rc = build_membership_filter(e, e.g, 0);
+  if (!rc && e.arena.tail) *launches += 1;
+  return rc;
+}
 
 bool use_segment_table(int mode, uint32_t V, int32_t L, uint64_t nadj) {
   if (mode == FSIG_SEGMENTS_TABLE) return true;
@@ -744,7 +753,7 @@ int build_device_graph(Engine& e, uint32_t V, const int32_t* h_labels, uint64_t 
   }
   FSIG_CUDA_TRY(cudaGetLastError());
   g.arena_mark = e.arena.mark();
-  rc = build_membership_filter(e, g);
+  rc = build_membership_filter(e, g, kFilterSpare);
   if (rc) return rc;
   FSIG_CUDA_TRY(cudaStreamSynchronize(s));
   e.g = g;
@@ -871,7 +880,7 @@ int load_graph_cache(Engine& e, const char* path) {
   g.h_base.resize(L1);
   FSIG_CUDA_TRY(cudaMemcpy(g.h_base.data(), g.base, 4 * L1, cudaMemcpyDeviceToHost));
   g.arena_mark = e.arena.mark();
-  const int rc = build_membership_filter(e, g);
+  const int rc = build_membership_filter(e, g, kFilterSpare);
   if (rc) return rc;
   FSIG_CUDA_TRY(cudaStreamSynchronize(e.stream));
   e.g = g;

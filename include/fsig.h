@@ -156,6 +156,11 @@ int fsig_set_segment_index(fsig_engine* e, int mode);
  * bytes (every array kept for matching; not the membership filter, which lies
  * in arena room that calls take back when they need it). */
 int fsig_graph_layout(const fsig_engine* e, int* segment_index, uint64_t* store_bytes);
+/* Device bytes of the resident graph's membership filter: 0 when the arena had
+ * no room for it (and 1 GiB beside it) at the load, and after a call that took
+ * its room, until a matching call finds the room free and builds it again.
+ * Results do not depend on it, times do. */
+int fsig_graph_filter(const fsig_engine* e, uint64_t* bytes);
 
 /* Binary cache of the resident graph store (the device arrays as built: the
  * renumbered CSR, caller ids, label segments and signatures), in place of the
