@@ -1035,7 +1035,9 @@ int run_batch(Engine& e, const std::vector<HostQuery>& qs, const BatchOptions& o
     const uint64_t at_qv = in.add(sizeof(QVert) * b.G), at_qoff = in.add(4 * b.qoff.size()),
                    at_gidx = in.add(4 * b.lab_gidx.size()), at_begin = in.add(4 * b.lab_begin.size()),
                    at_gword = in.add(8 * b.gword.size()), at_given = in.add(4 * given.size()),
-                   at_scores = in.add(4 * scores.size()), at_has = in.add(4 * has_given.size());
+                   at_scores = in.add(4 * scores.size());
+    const bool mixed = opt.learned && any_given;  // learned and given orders in one batch
+    const uint64_t at_has = mixed ? in.add(4 * has_given.size()) : 0;
     in.dev = e.arena.take<uint8_t>(in.bytes);
     if (!in.dev) return fail(FSIG_EADMISSION, "batch does not fit the device arena");
     in.host = st.take<uint8_t>(in.bytes);
@@ -1046,7 +1048,7 @@ int run_batch(Engine& e, const std::vector<HostQuery>& qs, const BatchOptions& o
     fill_part(in, at_gword, b.gword);
     fill_part(in, at_given, given);
     fill_part(in, at_scores, scores);
-    fill_part(in, at_has, has_given);
+    if (mixed) fill_part(in, at_has, has_given);
     FSIG_CUDA_TRY(cudaMemcpyAsync(in.dev, in.host, in.bytes, cudaMemcpyHostToDevice, s));
     e.cur_h2d += in.bytes;
     QVert* d_qv = in.d<QVert>(at_qv);
@@ -1129,7 +1131,7 @@ int run_batch(Engine& e, const std::vector<HostQuery>& qs, const BatchOptions& o
         FSIG_CUDA_TRY(cudaGetLastError());
         launches++;
       }
-      if (any_given) {
+      if (mixed) {
         given_scores_kernel<<<std::max<uint32_t>(1, (Q + 127) / 128), 128, 0, s>>>(d_qoff, Q, in.d<uint32_t>(at_has),
                                                                                  d_given, d_lscores);
         FSIG_CUDA_TRY(cudaGetLastError());
