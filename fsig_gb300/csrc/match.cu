@@ -917,6 +917,7 @@ int enum_after(Engine& e, EnumRun& R, bool& more, float& ms_enum, uint64_t& d2h)
   untaken_kernel<<<1, 256, 0, e.stream>>>(R.ready, kQueueSlots, count);
   FSIG_CUDA_TRY(cudaGetLastError());
   FSIG_CUDA_TRY(cudaMemcpyAsync(R.h_ctr, count, sizeof(uint32_t), cudaMemcpyDeviceToHost, e.stream));
+  d2h += sizeof(uint32_t);
   FSIG_CUDA_TRY(cudaStreamSynchronize(e.stream));
   if (R.h_ctr[0] != left) return fail(FSIG_EOVERFLOW, "task records were lost");
   R.A.in_tasks = R.out;
@@ -1181,6 +1182,7 @@ int run_batch(Engine& e, const std::vector<HostQuery>& qs, const BatchOptions& o
   auto copy_back = [&]() -> int {
     FSIG_CUDA_TRY(record(e.ev[2], s));
     FSIG_CUDA_TRY(cudaMemcpyAsync(res.host, res.dev, res_bytes, cudaMemcpyDeviceToHost, s));
+    d2h += res_bytes;
     return FSIG_OK;
   };
 
@@ -1294,7 +1296,6 @@ int run_batch(Engine& e, const std::vector<HostQuery>& qs, const BatchOptions& o
     out.ms_join = graph ? std::max(elapsed(e.ev_outer[0], e.ev_outer[1]), 0.f) : 0.f;
   }
   if (!R.timed) out.ms_enum = -1.f;
-  d2h += res_bytes * out.passes;
   out.h2d_bytes = e.cur_h2d;
   out.d2h_bytes = d2h;
   out.launches = launches;

@@ -24,3 +24,30 @@ def test_a_batch_uploads_its_descriptors_only():
         # 112-byte descriptor, label group entry, order, score and first bitmap
         # word (8 bytes); a query: its first vertex
         assert sizes[1] - sizes[0] == 576 * (3 * (112 + 4 + 4 + 4 + 8) + 4)
+
+
+def test_copies_back_are_counted_once():
+    """A graph brings its results back with the first pass and after the last
+    one, ordinary launches after every pass; each pass its counters (four lines
+    of 128 bytes), each but the last the number of records it left."""
+    g = F.gen_rmat(256, 2048, 0.57, 0.19, 0.19, seed=3)
+    q = F.Query(np.zeros(5, np.int32), np.array([[0, 1], [1, 2], [2, 3], [3, 4], [4, 0]], np.uint32))
+    kw = dict(algo=F.ALGO_FUSED, split_cycles=1000, split_len=32)
+
+    def copied(e, use_graph):
+        e.match_batch([q], use_graph=use_graph, **kw)
+        st = e.last_stats()
+        return st["enum_passes"], st["d2h_bytes"]
+
+    with F.Engine(0, arena_bytes=2 << 30) as e:
+        e.load_graph(g)
+        for use_graph in (False, True):
+            passes, one = copied(e, use_graph)
+            assert passes == 1
+            results = one - 512
+            e.set_queue_waits(idle_wait_ns=1)  # waiting warps leave: their records are later passes'
+            for _ in range(5):
+                p, b = copied(e, use_graph)
+                assert p > 1
+                assert b == (2 if use_graph else p) * results + 512 * p + 4 * (p - 1)
+            e.set_queue_waits()
