@@ -446,7 +446,8 @@ __global__ void __launch_bounds__(256) signature_from_rows_kernel(const int32_t*
 // Membership filter (common.cuh), a warp per 256 adjacency entries, one entry
 // per lane and step; the lane's row is found from the previous one by
 // galloping (rows average a step or two apart).  Bound by the atomics, all to
-// words near the entry's own position: L2.
+// words near the entry's own position: L2.  The arrays may be a cache file's, as
+// they are in the file, so nothing is read or written outside of them.
 constexpr uint32_t kFilterRun = 256;
 __global__ void __launch_bounds__(256) membership_filter_kernel(
     const uint32_t* __restrict__ off, const uint32_t* __restrict__ adj, const int32_t* __restrict__ label,
@@ -473,7 +474,8 @@ __global__ void __launch_bounds__(256) membership_filter_kernel(
       for (; step; step >>= 1)
         if (v + step < V && off[v + step] <= k) v += step;
       const uint32_t x = adj[k];
-      const int32_t l = label[x];
+      const int32_t l = x < V ? label[x] : -1;
+      if (l < 0 || l >= L) continue;
       uint32_t a, b;
       if (lseg) {
         const uint32_t* s = lseg + uint64_t(v) * (uint64_t(L) + 1) + l;
@@ -481,12 +483,12 @@ __global__ void __launch_bounds__(256) membership_filter_kernel(
         b = s[1];
       } else {
         a = lower_bound_u32(adj, off[v], k, base[l]);
-        b = lower_bound_u32(adj, k, off[v + 1], base[l + 1]);
+        b = lower_bound_u32(adj, k, min(off[v + 1], nadj), base[l + 1]);
       }
       const uint32_t first_id = base[l] & ~31u, rel = x - first_id;
       const bool dense = b - a >= filter_dense_len(base[l + 1] - first_id, shift);
       const uint32_t w = (a << shift) + filter_word(dense, rel, filter_hash(x), (b - a) << shift);
-      atomicOr(&filt[w >> 1], filter_mask(dense, rel, filter_bits(x)) << ((w & 1u) * 16));
+      if (w < uint64_t(nadj) << shift) atomicOr(&filt[w >> 1], filter_mask(dense, rel, filter_bits(x)) << ((w & 1u) * 16));
     }
   }
 }
@@ -835,7 +837,7 @@ int load_graph_cache(Engine& e, const char* path) {
   if (!f) return fail(FSIG_EIO, std::string("cannot open ") + path);
   CacheHeader h{};
   if (std::fread(&h, sizeof h, 1, f) != 1 || std::memcmp(h.magic, kCacheMagic, 8) != 0 || h.V == 0 || h.L < 1 ||
-      h.L > int32_t(kMaxLabels) || (h.flags & ~kCacheRows) != 0) {
+      h.L > int32_t(kMaxLabels) || h.nadj > 0xffffffffull || (h.flags & ~kCacheRows) != 0) {
     std::fclose(f);
     return fail(FSIG_EIO, std::string(path) + " is not a graph cache of this engine");
   }
