@@ -65,8 +65,8 @@ PEAKS = ROOT / "MEASURED_PEAKS.json"
 FALLBACK_HBM_GBS = 6800.0
 
 # DRAM bytes (read + write) of one enumerate_kernel launch on a config-5
-# batch, from an ncu capture (profiles/enumerate_kernel_c5.md: 2872 MB/s over
-# 126.2 ms); its loads are served from L2 at about 98 %.
+# batch, from an ncu capture (2872 MB/s over 126.2 ms); its loads are served
+# from L2 at about 98 %.
 ENUM_TRAFFIC_BYTES_PER_LAUNCH = 362_440_000
 
 

@@ -1,7 +1,7 @@
 """Autotuner of the batched path's launch knobs, by measurement.
 
-The enumeration kernel's behaviour on a workload depends on five knobs of
-``fsig_batch_opts``:
+The enumeration kernel's behaviour on a workload depends on four knobs of
+``fsig_batch_opts``, and a fifth is kept:
 
 * ``warps_per_block`` - block size of the persistent enumeration launch
   (warps that share an SM's blocks);
@@ -10,9 +10,9 @@ The enumeration kernel's behaviour on a workload depends on five knobs of
   hand-offs, and so of load balance);
 * ``split_cycles`` - SM cycles a task runs before its unexplored frontier may
   be handed to idle warps;
-* ``isect`` - the set-intersection strategy of the membership tests, 0..3:
-  the enumeration has one strategy by now, so the values time alike; the
-  knob stays for callers that set it.
+* ``isect`` - the set-intersection strategy, 0..3: the enumeration has one
+  strategy by now, so the values time alike and whichever is picked changes
+  nothing; the knob stays for callers that set it or read it from the result.
 
 When the batch refines candidates (``refine_iters`` > 0) one more joins:
 

@@ -58,10 +58,13 @@ __host__ __device__ __forceinline__ void sig_slot(int32_t label, uint32_t& word,
 // probe of a word settles most candidates that a binary search took 7-8
 // dependent loads to refuse: the 512-query batch on 2^26 edges 377 -> 197 ms,
 // house counting on 700 vertices (dense segments) 93 -> 63 ms.  The filter lies
-// in arena room that the next request takes back, so what fitted an arena still
-// fits.  One word an entry is half the adjacency; graphs of at most
-// kFilterSmall entries get four (32 MB then, well inside the L2), which makes
-// segments from a quarter of that length on exact.
+// in arena room that a request which needs it takes back, so what fitted an arena
+// still fits, and is built again once that room is free.  One word an entry is
+// half the adjacency; graphs of at most kFilterSmall entries get four (32 MB
+// then, well inside the L2), which makes segments from a quarter of that length on
+// exact.  (Four measured better at 2.1 M entries and below; one is for graphs whose
+// filter would outgrow the L2, measured at 2^27.  Where between them the line
+// lies best was not measured.)
 // ---------------------------------------------------------------------------
 constexpr uint64_t kFilterSmall = 1ull << 22;
 __host__ __device__ __forceinline__ uint32_t filter_shift(uint64_t nadj) { return nadj <= kFilterSmall ? 2 : 0; }

@@ -33,39 +33,29 @@
 // candidate and an entry take the lanes (joint, in fill).
 //
 // What bounds it: instructions and L2 latency (the working set is L2
-// resident), so the aim is full lanes.  A warp per entry, as before, ran 11 of
-// 32 lanes at the leaf of the 320k-vertex workloads (one range of 11-12
-// neighbours after another) and paid the set-up of a range, some 300
-// instructions, for each.  200 eight-vertex queries there 115 -> 34 ms of
-// kernel, 512 queries of 4-32 vertices 69 -> 34 ms, 253 instructions a window
-// at 79 % of the issue rate.  With the filter, a leaf loop of its own for
-// leaves of one segment, and buffers of one pool per warp (4 blocks an SM also
-// for 32-vertex queries, 3 with 32 entries for each depth): 27 and 23 ms, 198
-// instructions a window at 70 % of the issue rate; 512 queries of 12-32 vertices
-// on 2^26 edges 305 -> 146 ms, 279 instructions a window at 64 %.  With the first
-// filter tested beside the candidate bit (a third of the windows on 2^26 edges
-// end there), leaves of two segments in the leaf loop, and four earlier vertices
-// a load (a loop of one each took 25 % of the house count): 139 ms there, 21.5 ms
-// for 512 queries of 4-32 vertices, house counting 55 -> 32 ms.  With 96 windows a
-// fill and each depth's plan and cursor in one record: 25.4, 20.5 and 132 ms; of
-// the first the leaf loop took two fifths and the set-up of fills the rest.  With
-// longer last buffers and shared leaf ranges: 19.8, 15.2 and 126 ms.  Loading a
-// window ahead gains nothing.
+// resident), so the aim is full lanes and few instructions a window.  A warp per
+// entry ran 11 of 32 lanes at the leaf of the 320k-vertex workloads (one range of
+// 11-12 neighbours after another) and paid the set-up of a range, some 300
+// instructions, for each: 200 eight-vertex queries there took 115 ms of kernel,
+// 512 queries of 4-32 vertices 69, 512 queries of 12-32 vertices on 2^26 edges 305,
+// house counting on 700 vertices 104.  Now 19.8, 15.2, 126 and 32 ms, 243
+// instructions a window at 69 % of the issue rate on 2^26 edges.  (Buffers of one
+// pool per warp leave room for 4 blocks an SM also for 32-vertex queries; 32
+// entries for each depth, for 3.  Loading a window ahead gains nothing.)
 //
 // Work stealing: a warp that runs out of input takes a ticket, one atomicAdd
 // on the queue's head, and waits for the record of that number, polling the
-// record's own ready word.  A busy warp checks every 64 steps whether more
-// tickets than records are out; if so it hands its shallowest pending depth
+// record's own ready word.  A busy warp checks every 32 windows whether
+// more tickets than records are out; if so it hands its shallowest pending depth
 // (buffered candidates and the remaining driver range) to the queue as task
 // records and carries on with the rest.  One counter holds the warps at work
 // plus the records not taken yet; the pass is over when it reaches zero.
-// (Tickets replaced a compare-and-swap on the head by every idle warp for
-// every record: up to 2048 warps retrying on one word served a record in
-// 0.4-1.0 us whatever the work in it, which bounded every batch but the
-// largest.  One 4-vertex query on a 10k-vertex graph 3.8 -> 0.37 ms, 100 of
-// them 37 -> 2.5 ms, 37 refined queries on 2^26 edges 78 -> 29 ms, a
-// 512-query batch there 390 -> 305 ms.)  Waiting is bounded: a warp that waits too long leaves, which
-// never loses work -- the records nobody took are the next pass's input.
+// (With a compare-and-swap on the head by every idle warp for every record, up
+// to 2048 warps retrying on one word served a record in 0.4-1.0 us whatever the
+// work in it, which bounded every batch but the largest: one 4-vertex query on a
+// 10k-vertex graph 3.8 ms, 0.37 with tickets.)  Waiting is bounded: a warp that
+// waits too long leaves, which never loses work -- its record, if it is written,
+// is the next pass's input.
 // Every value that steers a warp's control flow is read by lane 0 and
 // broadcast.
 #pragma once
