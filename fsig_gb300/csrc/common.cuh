@@ -56,8 +56,9 @@ __host__ __device__ __forceinline__ void sig_slot(int32_t label, uint32_t& word,
 // is a Bloom filter whose element x sets two bits of one word, so that with one
 // word an entry 2-3 % of the ids that are not in it pass.  One
 // probe of a word settles most candidates that a binary search took 7-8
-// dependent loads to refuse: the 512-query batch on 2^26 edges 377 -> 197 ms,
-// house counting on 700 vertices (dense segments) 93 -> 63 ms.  The filter lies
+// dependent loads to refuse: the 512-query batch on 2^26 edges 377 -> 197 ms (247
+// without it and 128 with it by now), house counting on 700 vertices (dense
+// segments) 93 -> 63 ms.  The filter lies
 // in arena room that a request which needs it takes back, so what fitted an arena
 // still fits, and is built again once that room is free.  One word an entry is
 // half the adjacency; graphs of at most kFilterSmall entries get four (32 MB
