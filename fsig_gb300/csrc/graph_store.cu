@@ -613,7 +613,8 @@ uint64_t filter_bytes(const Engine& e) {
 int restore_membership_filter(Engine& e, uint32_t* launches) {
   if (!e.g.filt || e.arena.tail) return FSIG_OK;
   const int rc = build_membership_filter(e, e.g, 0);
-  if (!rc && e.arena.tail) *launches += 1;
+  if (rc) e.arena.tail = 0;
+  if (e.arena.tail) *launches += 1;
   return rc;
 }
 

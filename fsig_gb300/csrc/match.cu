@@ -794,6 +794,18 @@ struct EnumRun {
   uint32_t grid = 0, block = 0, active = 0, first_task = 0, pass = 0;
   size_t smem = 0;
   bool timed = true;  // every pass's kernel time was measured
+  bool restored = false;  // the membership filter is built again by the work enqueued
+};
+
+// A batch captured as a graph that is not launched after all does not build the
+// filter either.
+struct FilterUndo {
+  Arena& arena;
+  const EnumRun& run;
+  bool armed;
+  ~FilterUndo() {
+    if (armed && run.restored) arena.tail = 0;
+  }
 };
 
 // One-time kernel attributes and occupancy (host calls, kept out of captures).
@@ -844,7 +856,9 @@ int enum_prepare(Engine& e, const BatchOptions& opt, const GraphView& gv, const 
   // Every buffer of the call is taken by now: the filter's room is still its
   // own, or free again after a call that needed it (0.8 ms for 2^27 entries, once;
   // a batch of 512 queries there takes 128 ms with the filter, 247 without), or in use.
+  R.restored = e.arena.tail == 0;
   int rc = restore_membership_filter(e, &launches);
+  R.restored = R.restored && e.arena.tail != 0;
   if (rc) return rc;
   A.g.filt = e.arena.tail ? e.g.filt : nullptr;
   A.plans = d_plans;
@@ -1189,6 +1203,7 @@ int run_batch(Engine& e, const std::vector<HostQuery>& qs, const BatchOptions& o
   bool more = false;
   out.passes = 0;
   out.ms_enum = 0;
+  FilterUndo undo{e.arena, R, graph};
   if (graph) {
     rc = enqueue();
     if (!rc) rc = copy_back();
@@ -1217,6 +1232,7 @@ int run_batch(Engine& e, const std::vector<HostQuery>& qs, const BatchOptions& o
     cudaGraphDestroy(cg);
     FSIG_CUDA_TRY(cudaEventRecord(e.ev_outer[0], s));
     FSIG_CUDA_TRY(cudaGraphLaunch(e.gexec, s));
+    undo.armed = false;
     FSIG_CUDA_TRY(cudaEventRecord(e.ev_outer[1], s));
     FSIG_CUDA_TRY(cudaStreamSynchronize(s));
     out.passes = 1;
