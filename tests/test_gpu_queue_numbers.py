@@ -55,11 +55,12 @@ def test_a_warp_that_left_does_not_hold_up_the_others(first):
         e.set_queue_waits(idle_wait_ns=30 * 10**9)
         e.set_queue_test(first_record=first, first_leaves=True)
         passes = []
-        for use_graph in (False, True):
+        for use_graph in (False, True) * 8:
             t = time.perf_counter()
             r, = e.match_batch([q], use_graph=use_graph, **kw)
             assert time.perf_counter() - t < 5.0
             assert (r.status, r.count, r.hash) == (0, *want)
             assert r.level_counts == plain.level_counts
             passes.append(e.last_stats()["enum_passes"])
-    assert max(passes) > 1  # the record of the warp that left
+    # the record of the warp that left (unless it was written before that looked)
+    assert max(passes) > 1
